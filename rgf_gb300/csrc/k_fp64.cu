@@ -22,6 +22,22 @@ __device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
+// Every thread of the cluster arrives and waits; shared-memory writes before
+// it are visible to the cluster's reads after it.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;"
+               ::: "memory");
+}
+// *p of the cluster's CTA `rank` (p: this CTA's shared memory)
+__device__ __forceinline__ double ld_cluster(const double* p, int rank) {
+  unsigned a;
+  double v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+               : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+  return v;
+}
+
 struct GemmTileRange {
   int klo, khi;
 };
@@ -403,119 +419,186 @@ __global__ void __launch_bounds__(128) trsm_rows_kernel(double* X, long long xrs
   trsm_rows_body<MODE>(X, xrs, xcs, rows, Ls, rinv, nbk, (long long)blockIdx.x * 16);
 }
 
-// Thin products (m <= 16, op(B) = B^T): lane = output column, the 4 warps of
-// a CTA split a K chunk, blockIdx.y selects the chunk.  Partial sums go to
-// the split-K workspace in the GEMM kernel's layout.
+// Thin products (m <= 16, op(B) = B^T; the arrowhead rows): lane = output
+// column, M (a template parameter: an absent row's FMA would cost as much as
+// a present one's) accumulators per lane.  K is split over a cluster and the
+// four warps as in gemm_thin_n_kernel below; B is read along its contiguous
+// columns, A's M terms per k are one uniform load each.
+template <int M>
 __global__ void __launch_bounds__(128) gemm_thin_m_kernel(GemmDesc g, int kchunk) {
-  __shared__ double red[4][16][33];
+  __shared__ double part[4][M][32];
+  __shared__ double red[M * 32];
   pdl_wait();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + lane;
-  const int k0 = blockIdx.y * kchunk, k1 = min(g.k, k0 + kchunk);
-  double acc[16];
+  const int c0 = blockIdx.x * 32, c = c0 + lane;
+  int k0 = blockIdx.y * kchunk, k1 = min(g.k, k0 + kchunk);
+  if (g.triB == TRI_LOWER) k0 = max(k0, c0);        // op(B)(k, c) = 0 for k < c
+  if (g.triB == TRI_UPPER) k1 = min(k1, c0 + 32);   // and for k > c
+  const long long ras = g.transA ? g.lda : 1, kas = g.transA ? 1 : g.lda;
+  double acc[M];
 #pragma unroll
-  for (int r = 0; r < 16; ++r) acc[r] = 0.0;
-  if (c < g.n) {
-    for (int k = k0 + w; k < k1; k += 4) {
-      if (g.triB == TRI_LOWER && k < c) continue;   // op(B)(k, c) = 0 above
-      if (g.triB == TRI_UPPER && k > c) continue;
-      const double b = g.B[(long long)c + (long long)k * g.ldb];
-      const double* a = g.transA ? g.A + (long long)k : g.A + (long long)k * g.lda;
+  for (int r = 0; r < M; ++r) acc[r] = 0.0;
+  constexpr int U = 8;  // K terms in flight per warp
+  for (int kt = k0 + w * U; kt < k1; kt += 4 * U) {
+    double b[U];
 #pragma unroll
-      for (int r = 0; r < 16; ++r)
-        if (r < g.m) acc[r] = fma(g.transA ? a[(long long)r * g.lda] : a[r], b, acc[r]);
+    for (int u = 0; u < U; ++u) {
+      const int k = kt + u;
+      bool ok = k < k1 && c < g.n;
+      if (g.triB == TRI_LOWER) ok = ok && k >= c;
+      if (g.triB == TRI_UPPER) ok = ok && k <= c;
+      b[u] = ok ? g.B[c + (long long)k * g.ldb] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (kt + u >= k1) break;
+      const double* a = g.A + (kt + u) * kas;
+#pragma unroll
+      for (int r = 0; r < M; ++r) acc[r] = fma(r < g.m ? a[r * ras] : 0.0, b[u], acc[r]);
     }
   }
   pdl_trigger();
 #pragma unroll
-  for (int r = 0; r < 16; ++r) red[w][r][lane] = acc[r];
+  for (int r = 0; r < M; ++r) part[w][r][lane] = acc[r];
   __syncthreads();
-  if (w == 0 && c < g.n) {
-    double* W = g.ws + (long long)blockIdx.y * g.m * g.n;
-#pragma unroll
-    for (int r = 0; r < 16; ++r)
-      if (r < g.m) W[(long long)r + (long long)c * g.m] =
-          ((red[0][r][lane] + red[1][r][lane]) + red[2][r][lane]) + red[3][r][lane];
+  for (int o = threadIdx.x; o < M * 32; o += 128) {
+    const int r = o >> 5, l = o & 31;
+    red[o] = ((part[0][r][l] + part[1][r][l]) + part[2][r][l]) + part[3][r][l];
   }
+  const int nk = gridDim.y, rank = blockIdx.y;
+  if (nk > 1) cluster_sync();
+  else __syncthreads();
+  for (int o = rank * 128 + threadIdx.x; o < M * 32; o += nk * 128) {
+    const int r = o >> 5, col = c0 + (o & 31);
+    double v = 0.0;
+    if (nk > 1) {
+      for (int q = 0; q < nk; ++q) v += ld_cluster(red + o, q);
+    } else {
+      v = red[o];
+    }
+    if (r < g.m && col < g.n) {
+      v *= g.alpha;
+      const bool hi = g.D2 && r >= g.mD1;
+      const long long ro = hi ? r - g.mD1 : r;
+      if (g.beta != 0.0) v += g.beta * (hi ? g.C2 : g.C)[ro + (long long)col * g.ldc];
+      (hi ? g.D2 : g.D)[ro + (long long)col * g.ldd] = v;
+    }
+  }
+  if (nk > 1) cluster_sync();
 }
 
-// Thin products (n <= 16, op(B) = B): thread = output row; the CTA's 128 rows
-// share 32-term K tiles of op(A) and op(B) staged through shared memory (read
-// along A's contiguous dimension either way), so every FP64 instruction has
-// all lanes busy.  The next tile is loaded into registers while the current
-// one is multiplied.  blockIdx.y selects a K chunk; partial sums go to the
-// split-K workspace in the GEMM kernel's layout.  op(A) may be triangular.
+// Thin products (n <= 16, op(B) = B; the steps of the block substitution):
+// bound by the FP64 units (m k n FMAs at ~0.55 TFMA/s; an FP64 instruction
+// holds its unit ~76 cycles even with every lane predicated off, so the
+// columns are a template parameter and no FMA is issued for absent ones).
+// A CTA owns 32 output rows, lane = row.  A cluster of up to 8 CTAs
+// (blockIdx.y) splits K, and within a CTA the four warps take K tiles of 32
+// terms in turn: many SMs work on even a small product.  The partial sums
+// meet in shared memory, first over the warps, then over the cluster through
+// distributed shared memory, both in a fixed order: one launch per product.
+// op(A) is read along its contiguous dimension; a transposed A goes through a
+// per-warp 32 x 32 shared-memory tile.  Measured over whole solves (four such
+// products per block column), against 128-row tiles with 16 predicated columns
+// and a second launch for the reduction: one right-hand side at ns = 256,
+// nt = 60 10.15 -> 1.08 ms (42 -> 4.5 us a product); eight at ns = 1000,
+// nt = 50, split (two sweeps and the residuals) 20.7 -> 10.8 ms.
+// op(A) may be triangular: K tiles that lie in its other triangle are skipped.
+constexpr int THIN_KT = 32;  // K terms of one warp's tile
+template <int N>
 __global__ void __launch_bounds__(128) gemm_thin_n_kernel(GemmDesc g, int kchunk) {
-  __shared__ double As[32][129];
-  __shared__ double Bs[32][17];
+  // per warp: tile of a transposed A, element (k, row) at [k][row ^ k] (no bank
+  // conflicts either way, within the 48 KiB of N = 16); then the warps' sums
+  __shared__ double At[4][THIN_KT][32];
+  __shared__ double Bs[4][THIN_KT][N];
   pdl_wait();
-  const int tid = threadIdx.x;
-  const int r0 = blockIdx.x * 128, r = r0 + tid;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int r0 = blockIdx.x * 32, r = r0 + lane;
   int k0 = blockIdx.y * kchunk, k1 = min(g.k, k0 + kchunk);
-  if (g.triA == TRI_LOWER) k1 = min(k1, r0 + 128);  // op(A)(r, kk) = 0 for kk > r
-  if (g.triA == TRI_UPPER) k0 = max(k0, r0);        // op(A)(r, kk) = 0 for kk < r
-  double acc[16];
+  if (g.triA == TRI_LOWER) k1 = min(k1, r0 + 32);               // op(A)(r, kk) = 0 for kk > r
+  if (g.triA == TRI_UPPER) k0 = max(k0, r0 / THIN_KT * THIN_KT);  // and for kk < r
+  double acc[N];
 #pragma unroll
-  for (int c = 0; c < 16; ++c) acc[c] = 0.0;
-  double ra[32], rb[4];
-  auto load = [&](int kt) {
+  for (int c = 0; c < N; ++c) acc[c] = 0.0;
+  for (int kt = k0 + w * THIN_KT; kt < k1; kt += 4 * THIN_KT) {
+    const int kn = min(THIN_KT, k1 - kt);
+    double ra[THIN_KT];  // op(A)(r, kt + kk), or (transposed) op(A)(r0 + kk, kt + lane)
+    if (!g.transA) {
+      const double* a = g.A + r + (long long)kt * g.lda;
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const int idx = tid + 128 * j;
-      int i, kk;
-      if (!g.transA) { i = idx & 127; kk = idx >> 7; }
-      else           { kk = idx & 31; i = idx >> 5; }
-      const int row = r0 + i, kg = kt + kk;
-      bool ok = row < g.m && kg < k1;
-      if (g.triA == TRI_LOWER) ok = ok && kg <= row;
-      if (g.triA == TRI_UPPER) ok = ok && kg >= row;
-      double v = 0.0;
-      if (ok) v = g.transA ? g.A[(long long)kg + (long long)row * g.lda]
-                           : g.A[(long long)row + (long long)kg * g.lda];
-      ra[j] = v;
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int idx = tid + 128 * j, kk = idx & 31, c = idx >> 5, kg = kt + kk;
-      rb[j] = (c < g.n && kg < k1) ? g.B[(long long)kg + (long long)c * g.ldb] : 0.0;
-    }
-  };
-  auto store = [&]() {
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const int idx = tid + 128 * j;
-      if (!g.transA) As[idx >> 7][idx & 127] = ra[j];
-      else           As[idx & 31][idx >> 5] = ra[j];
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int idx = tid + 128 * j;
-      Bs[idx & 31][idx >> 5] = rb[j];
-    }
-  };
-  if (k0 < k1) {
-    load(k0);
-    for (int kt = k0; kt < k1; kt += 32) {
-      store();
-      __syncthreads();
-      if (kt + 32 < k1) load(kt + 32);
-#pragma unroll 4
-      for (int kk = 0; kk < 32; ++kk) {
-        const double a = As[kk][tid];
-#pragma unroll
-        for (int c = 0; c < 16; ++c)
-          if (c < g.n) acc[c] = fma(a, Bs[kk][c], acc[c]);
+      for (int kk = 0; kk < THIN_KT; ++kk) {
+        bool ok = kk < kn && r < g.m;
+        if (g.triA == TRI_LOWER) ok = ok && kt + kk <= r;
+        if (g.triA == TRI_UPPER) ok = ok && kt + kk >= r;
+        ra[kk] = ok ? *a : 0.0;
+        a += g.lda;
       }
-      __syncthreads();
+    } else {
+      const int kg = kt + lane;
+      const double* a = g.A + kg + (long long)r0 * g.lda;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        bool ok = lane < kn && r0 + i < g.m;
+        if (g.triA == TRI_LOWER) ok = ok && kg <= r0 + i;
+        if (g.triA == TRI_UPPER) ok = ok && kg >= r0 + i;
+        ra[i] = ok ? *a : 0.0;
+        a += g.lda;
+      }
     }
+#pragma unroll
+    for (int c = 0; c < N; ++c)
+      Bs[w][lane][c] = lane < kn && c < g.n ? g.B[kt + lane + (long long)c * g.ldb] : 0.0;
+    if (g.transA) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) At[w][lane][i ^ lane] = ra[i];
+    }
+    __syncwarp();
+    if (g.transA) {
+      for (int kk = 0; kk < kn; ++kk) {
+        const double a = At[w][kk][lane ^ kk];
+#pragma unroll
+        for (int c = 0; c < N; ++c) acc[c] = fma(a, Bs[w][kk][c], acc[c]);
+      }
+    } else {
+#pragma unroll
+      for (int kk = 0; kk < THIN_KT; ++kk) {
+        if (kk >= kn) break;
+#pragma unroll
+        for (int c = 0; c < N; ++c) acc[c] = fma(ra[kk], Bs[w][kk][c], acc[c]);
+      }
+    }
+    __syncwarp();
   }
   pdl_trigger();
-  if (r < g.m) {
-    double* W = g.ws + (long long)blockIdx.y * g.m * g.n;
+  // this CTA's sums: warp partials in At[w][c][lane], summed in warp order
+  // into red[c][row]
+  __syncthreads();
 #pragma unroll
-    for (int c = 0; c < 16; ++c)
-      if (c < g.n) W[(long long)r + (long long)c * g.m] = acc[c];
+  for (int c = 0; c < N; ++c) At[w][c][lane] = acc[c];
+  __syncthreads();
+  double* red = &Bs[0][0][0];  // N x 32
+  for (int o = threadIdx.x; o < N * 32; o += 128) {
+    const int c = o >> 5, l = o & 31;
+    red[o] = ((At[0][c][l] + At[1][c][l]) + At[2][c][l]) + At[3][c][l];
   }
+  const int nk = gridDim.y, rank = blockIdx.y;  // the cluster spans blockIdx.y
+  if (nk > 1) cluster_sync();
+  else __syncthreads();
+  // the cluster's total in rank order; the outputs are dealt over its CTAs
+  for (int o = rank * 128 + threadIdx.x; o < N * 32; o += nk * 128) {
+    const int c = o >> 5, row = r0 + (o & 31);
+    double v = 0.0;
+    if (nk > 1) {
+      for (int q = 0; q < nk; ++q) v += ld_cluster(red + o, q);
+    } else {
+      v = red[o];
+    }
+    if (row < g.m && c < g.n) {
+      v *= g.alpha;
+      if (g.beta != 0.0) v += g.beta * g.C[row + (long long)c * g.ldc];
+      g.D[row + (long long)c * g.ldd] = v;
+    }
+  }
+  if (nk > 1) cluster_sync();  // a CTA's sums are read until every CTA is here
 }
 
 // D = alpha * sum_s W_s + beta * C over the split-K partials, in slice order.
@@ -534,6 +617,49 @@ __global__ void splitk_reduce_kernel(GemmDesc g) {
   (hi ? g.D2 : g.D)[ro + (long long)c * g.ldd] = v;
 }
 
+// K over 1, 2, 4 or 8 CTAs of a cluster: `least` K terms per CTA are the
+// least worth a CTA of their own (a quarter of them per warp).
+dim3 thin_split(const GemmDesc& g, int least, int* kchunk) {
+  int kc = 1;
+  while (kc < 8 && kc * least < g.k) kc *= 2;
+  *kchunk = ((g.k + kc - 1) / kc + THIN_KT - 1) / THIN_KT * THIN_KT;
+  return dim3(1, kc);
+}
+template <int N>
+void launch_thin_n(const GemmDesc& g, cudaStream_t s) {
+  int kchunk;
+  const dim3 cl = thin_split(g, THIN_KT, &kchunk);
+  launch_k_cluster(gemm_thin_n_kernel<N>, dim3((g.m + 31) / 32, cl.y), dim3(128), cl, 0, s, g,
+                   kchunk);
+}
+template <int M>
+void launch_thin_m(const GemmDesc& g, cudaStream_t s) {
+  int kchunk;
+  const dim3 cl = thin_split(g, THIN_KT, &kchunk);
+  launch_k_cluster(gemm_thin_m_kernel<M>, dim3((g.n + 31) / 32, cl.y), dim3(128), cl, 0, s, g,
+                   kchunk);
+}
+void launch_gemm_thin_n(const GemmDesc& g, cudaStream_t s) {
+  if (g.n <= 1) launch_thin_n<1>(g, s);
+  else if (g.n <= 2) launch_thin_n<2>(g, s);
+  else if (g.n <= 3) launch_thin_n<3>(g, s);
+  else if (g.n <= 4) launch_thin_n<4>(g, s);
+  else if (g.n <= 6) launch_thin_n<6>(g, s);
+  else if (g.n <= 8) launch_thin_n<8>(g, s);
+  else if (g.n <= 12) launch_thin_n<12>(g, s);
+  else launch_thin_n<16>(g, s);
+}
+void launch_gemm_thin_m(const GemmDesc& g, cudaStream_t s) {
+  if (g.m <= 1) launch_thin_m<1>(g, s);
+  else if (g.m <= 2) launch_thin_m<2>(g, s);
+  else if (g.m <= 3) launch_thin_m<3>(g, s);
+  else if (g.m <= 4) launch_thin_m<4>(g, s);
+  else if (g.m <= 6) launch_thin_m<6>(g, s);
+  else if (g.m <= 8) launch_thin_m<8>(g, s);
+  else if (g.m <= 12) launch_thin_m<12>(g, s);
+  else launch_thin_m<16>(g, s);
+}
+
 }  // namespace
 
 double gemm_flops(const GemmDesc& g) {
@@ -550,33 +676,13 @@ int launch_gemm_fp64(const GemmDesc& g0, cudaStream_t s) {
   GemmDesc g = g0;
   if (g.m <= 16 && g.transB && g.triA == TRI_NONE && g.batch == 1 && g.ws && !g.outLower &&
       !g.A2) {
-    const int cx = (g.n + 31) / 32;
-    int kchunks = std::max(1, std::min((2 * 152 + cx - 1) / cx, (g.k + 63) / 64));
-    while (kchunks > 1 && (long long)kchunks * g.m * g.n > g.ws_elems) --kchunks;
-    if ((long long)kchunks * g.m * g.n <= g.ws_elems) {
-      const int kchunk = (g.k + kchunks - 1) / kchunks;
-      g.ksplit = kchunks;
-      launch_k(gemm_thin_m_kernel, dim3(cx, kchunks), dim3(128), 0, s, g, kchunk);
-      dim3 rg((g.m + 31) / 32, (g.n + 7) / 8);
-      launch_k(splitk_reduce_kernel, rg, dim3(32, 8), 0, s, g);
-      return 2;
-    }
+    launch_gemm_thin_m(g, s);
+    return 1;
   }
   if (g.n <= 16 && !g.transB && g.triB == TRI_NONE && g.batch == 1 && g.ws && !g.outLower &&
-      !g.A2) {
-    const int rb = (g.m + 127) / 128;
-    // about two CTAs per SM, each with at least 2 K tiles to pipeline
-    int kchunks = std::max(1, std::min((2 * 152 + rb - 1) / rb, (g.k + 63) / 64));
-    while (kchunks > 1 && (long long)kchunks * g.m * g.n > g.ws_elems) --kchunks;
-    if ((long long)kchunks * g.m * g.n <= g.ws_elems) {
-      const int kchunk = ((g.k + kchunks - 1) / kchunks + 31) / 32 * 32;
-      kchunks = (g.k + kchunk - 1) / kchunk;
-      g.ksplit = kchunks;
-      launch_k(gemm_thin_n_kernel, dim3(rb, kchunks), dim3(128), 0, s, g, kchunk);
-      dim3 rg((g.m + 31) / 32, (g.n + 7) / 8);
-      launch_k(splitk_reduce_kernel, rg, dim3(32, 8), 0, s, g);
-      return 2;
-    }
+      !g.A2 && !g.D2) {
+    launch_gemm_thin_n(g, s);
+    return 1;
   }
   // tiles of 64 when they (with split K) cover the SMs, else tiles of 32
   auto count_tiles = [&](int tm) {

@@ -34,23 +34,39 @@ __device__ __forceinline__ void pdl_trigger() {
 
 bool pdl_enabled();
 
+// launch_k_cluster: the same with thread-block clusters of the given size.
 template <typename... KArgs, typename... Args>
-inline void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                     Args... args) {
+inline void launch_k_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, dim3 cluster,
+                             size_t smem, cudaStream_t s, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute at[2];
   cfg.attrs = at;
+  cfg.numAttrs = 0;
+  if (cluster.x * cluster.y * cluster.z > 1) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    at[cfg.numAttrs].val.clusterDim.x = cluster.x;
+    at[cfg.numAttrs].val.clusterDim.y = cluster.y;
+    at[cfg.numAttrs].val.clusterDim.z = cluster.z;
+    cfg.numAttrs++;
+  }
   // created streams only: not the default streams (the legacy one synchronizes
   // with every stream)
-  cfg.numAttrs =
-      pdl_enabled() && s != nullptr && s != cudaStreamLegacy && s != cudaStreamPerThread ? 1 : 0;
+  if (pdl_enabled() && s != nullptr && s != cudaStreamLegacy && s != cudaStreamPerThread) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs++;
+  }
   cudaLaunchKernelEx(&cfg, kern, args...);  // a failure stays the pending launch error
+}
+
+template <typename... KArgs, typename... Args>
+inline void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                     Args... args) {
+  launch_k_cluster(kern, grid, block, dim3(1, 1, 1), smem, s, args...);
 }
 
 enum Tri { TRI_NONE = 0, TRI_LOWER = 1, TRI_UPPER = 2 };
