@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(128) gemm_fp64_kernel(GemmDesc g) {
   pdl_wait();
   const int m0 = blockIdx.x * TM;
   const int n0 = blockIdx.y * TM;
-  if (g.outLower && m0 + TM <= n0) return;  // tile entirely above the diagonal
+  if (!tile_written(g.outLower, g.outUpper, m0, n0, TM)) return;
   const bool splitk = g.ksplit > 1;              // blockIdx.z is the K slice, batch == 1
   const long long bz = splitk ? 0 : blockIdx.z;
   const double* __restrict__ A = g.A + bz * g.sA;
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(128) gemm_fp64_kernel(GemmDesc g) {
       for (int e = 0; e < 2; ++e) {
         const int c = n0 + wn + j * 8 + (lane & 3) * 2 + e;
         if (c >= g.n) continue;
-        if (g.outLower && r < c) continue;
+        if ((g.outLower && r < c) || (g.outUpper && r > c)) continue;
         double v = g.alpha * acc[i][j][e];
         if (g.beta != 0.0) v += g.beta * Cr[(long long)r + (long long)c * g.ldc];
         Dr[(long long)r + (long long)c * g.ldd] = v;
@@ -606,7 +606,7 @@ __global__ void splitk_reduce_kernel(GemmDesc g) {
   pdl_wait();
   pdl_trigger();
   const int r = blockIdx.x * 32 + threadIdx.x, c = blockIdx.y * 8 + threadIdx.y;
-  if (r >= g.m || c >= g.n || (g.outLower && r < c)) return;
+  if (r >= g.m || c >= g.n || (g.outLower && r < c) || (g.outUpper && r > c)) return;
   const long long mn = (long long)g.m * g.n, o = (long long)r + (long long)c * g.m;
   double v = 0.0;
   for (int s = 0; s < g.ksplit; ++s) v += g.ws[s * mn + o];
@@ -667,6 +667,7 @@ double gemm_flops(const GemmDesc& g) {
   double f = 2.0 * m * n * k;
   if (g.triA != TRI_NONE) f = m * (m + 1.0) * n;
   if (g.triB != TRI_NONE) f = m * n * (n + 1.0);
+  if (g.outUpper && g.m == g.n) f = k * m * (m + 1.0);
   if (g.outLower && g.m >= g.n && g.n > 0) f = 2.0 * k * (n * (n + 1.0) / 2.0 + (m - n) * n);
   return f * g.batch;
 }
@@ -674,30 +675,22 @@ double gemm_flops(const GemmDesc& g) {
 int launch_gemm_fp64(const GemmDesc& g0, cudaStream_t s) {
   if (g0.m <= 0 || g0.n <= 0 || g0.batch <= 0) return 0;
   GemmDesc g = g0;
-  if (g.m <= 16 && g.transB && g.triA == TRI_NONE && g.batch == 1 && g.ws && !g.outLower &&
+  if (g.m <= 16 && g.transB && g.triA == TRI_NONE && g.batch == 1 && g.ws && !g.outLower && !g.outUpper &&
       !g.A2) {
     launch_gemm_thin_m(g, s);
     return 1;
   }
-  if (g.n <= 16 && !g.transB && g.triB == TRI_NONE && g.batch == 1 && g.ws && !g.outLower &&
+  if (g.n <= 16 && !g.transB && g.triB == TRI_NONE && g.batch == 1 && g.ws && !g.outLower && !g.outUpper &&
       !g.A2 && !g.D2) {
     launch_gemm_thin_n(g, s);
     return 1;
   }
   // tiles of 64 when they (with split K) cover the SMs, else tiles of 32
-  auto count_tiles = [&](int tm) {
-    const int tx = (g.m + tm - 1) / tm, ty = (g.n + tm - 1) / tm;
-    long long tiles = 0;
-    for (int bx = 0; bx < tx; ++bx)
-      for (int by = 0; by < ty; ++by)
-        if (!(g.outLower && bx * tm + tm <= by * tm)) ++tiles;
-    return tiles;
-  };
-  const long long t64 = count_tiles(64);
+  const long long t64 = tiles_written(g, 64);
   const bool small = g.tile == 32 || (g.tile != 64 && g.batch == 1 && g.ws &&
                                        t64 * std::min(16, std::max(1, g.k / 16)) < 152);
   const int tm = small ? 32 : 64, tk = small ? 8 : 16;
-  const long long tiles = small ? count_tiles(32) : t64;
+  const long long tiles = small ? tiles_written(g, 32) : t64;
   // too few output tiles for 152 SMs (each SM retires only ~3.5 FP64 flops
   // per cycle, so one 64x64x64 tile is tens of microseconds): split K
   int ksplit = 1;

@@ -75,7 +75,7 @@ struct SplitParams {
   // at a time; level of the first half gl1, of the second gl2 (NO_SLICE: none)
   int ngroups;
   unsigned char g0[MAXGROUPS], gs[MAXGROUPS], gl1[MAXGROUPS], gl2[MAXGROUPS], gchunk[MAXGROUPS];
-  int triA, triB, outLower;
+  int triA, triB, outLower, outUpper;
   const int* exA;
   const int* exB;
   int exA_stride, exB_stride;   // per batch item (padded rows)
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-  if (p.outLower && m0 + BM <= n0) return;  // whole tile above the diagonal (uniform exit)
+  if (!tile_written(p.outLower, p.outUpper, m0, n0, BM)) return;  // nothing to write (uniform exit)
   const int zb = blockIdx.z / p.ksplit;     // batch item: slice planes zb*S .. zb*S+S-1
   const int kz = blockIdx.z - zb * p.ksplit;
   const int zS = zb * p.S;
@@ -544,19 +544,20 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     const int ncols = live ? min(64, p.n - cbase) : 0;          // columns < n
     const int cdiag = p.outLower ? r - cbase : 64;                // columns c <= r only
     const int nlive = max(0, min(ncols, cdiag + 1));
+    const int c_lo = p.outUpper ? r - cbase : 0;                  // columns c >= r only
 #pragma unroll 1
     for (int i0 = 0; i0 < 64; i0 += 8) {
       double cv[8];
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        cv[q] = (Cp && i0 + q < nlive) ? *Cp : 0.0;
+        cv[q] = (Cp && i0 + q < nlive && i0 + q >= c_lo) ? *Cp : 0.0;
         if (Cp) Cp += ldc;
       }
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
         const int i = i0 + q;
         const int ec = __shfl_sync(0xffffffffu, i < 32 ? ex_lo : ex_hi, i & 31);
-        if (i < nlive) {
+        if (i < nlive && i >= c_lo) {
           double v = i64_ldexp(eacc[i * 256 + t], er + ec);
           if (amode == 2) v *= alpha;
           if (use_c) v = fma(betac, cv[q], v);
@@ -1021,10 +1022,7 @@ double SplitEngine::estimate_seconds(const GemmDesc& g, int slices) const {
   const int S = slices > 0 ? std::min(slices, MAX_SLICES) : slices_;
   const int Kp = round_up(g.k, BKE);
   const int tx = round_up(g.m, BM) / BM, ty = round_up(g.n, BN) / BN;
-  long long tiles = 0;
-  for (int bx = 0; bx < tx; ++bx)
-    for (int by = 0; by < ty; ++by)
-      if (!(g.outLower && bx * BM + BM <= by * BN)) ++tiles;
+  long long tiles = tiles_written(g, BM);
   tiles *= g.batch;
   const SlotPlan& plan = slot_plan(S);
   int jobs = 0;
@@ -1123,7 +1121,7 @@ long long SplitEngine::gemm(const GemmDesc& g, cudaStream_t s, DevStatus* st,
     p.gchunk[gi] = (unsigned char)std::max(1, EXACT_TERMS / (SBK * gr.count));
   }
   const int np = S * (S + 1) / 2;  // digit-pair products per output tile and K term
-  p.triA = g.triA; p.triB = g.triB; p.outLower = g.outLower;
+  p.triA = g.triA; p.triB = g.triB; p.outLower = g.outLower; p.outUpper = g.outUpper;
   p.ldc = g.ldc; p.ldd = g.ldd; p.sC = g.sC; p.sD = g.sD;
   p.alpha = g.alpha; p.betac = g.beta;
   p.st = st;
@@ -1206,10 +1204,7 @@ long long SplitEngine::gemm(const GemmDesc& g, cudaStream_t s, DevStatus* st,
     // split K when the output tiles fill at most half of the SMs (and the
     // workspace holds them): up to 16 slices of a tile's jobs, so that the
     // launch covers about one wave
-    int ntiles = 0;
-    for (int bx = 0; bx < RpA / BM; ++bx)
-      for (int by = 0; by < RpB / BN; ++by)
-        if (!(g.outLower && bx * BM + BM <= by * BN)) ++ntiles;
+    const int ntiles = (int)tiles_written(g, BM);
     const long long grid_tiles = (long long)(RpA / BM) * (RpB / BN) * nbat;
     p.ksplit = 1;
     if (wsk_ && (long long)ntiles * nbat * 2 <= num_sms_ && grid_tiles <= wsk_tiles_) {
@@ -1221,10 +1216,7 @@ long long SplitEngine::gemm(const GemmDesc& g, cudaStream_t s, DevStatus* st,
     p.cnt = cnt_;
     dim3 grid(RpA / BM, RpB / BN, nbat * p.ksplit);
     if (tensor_flops) {
-      double tiles = 0.0;  // lower-only outputs skip tiles above the diagonal
-      for (int bx = 0; bx < (int)grid.x; ++bx)
-        for (int by = 0; by < (int)grid.y; ++by)
-          if (!(g.outLower && bx * BM + BM <= by * BN)) tiles += 1.0;
+      const double tiles = ntiles;  // tiles with nothing to write are skipped
       *tensor_flops += tiles * nbat * 2.0 * BM * BN * (double)round_up(Kp, SBK) * np;
     }
     launch_k(split_gemm_kernel, grid, dim3(NUM_THREADS), SMEM_BYTES, s, ma, mb, p);
