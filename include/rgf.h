@@ -292,8 +292,9 @@ int rgf_batch_kernels(rgf_batch* b, long long* kernels);
  * Knobs of one handle's factorize + selected inversion (no counterpart in the
  * reference, whose MAGMA calls pick their own blocking).  None changes the
  * algorithm or the operation count; each changes how it is cut into kernels:
- *   leaf_nb     column width of the FP64 leaf Cholesky / triangular solves
- *               the recursive panel factorization bottoms out in: 16, 32, 64;
+ *   leaf_nb     how wide a diagonal tile of the panel factorization one launch
+ *               factors (32-column FP64 leaves inside): 16 = 64 columns,
+ *               32 or 64 = 128 columns;
  *   lookahead   1 = the rows below each diagonal block are solved and updated
  *               on a second, lower-priority stream; 0 = one stream;
  *   split_bias  split precision: a product runs on the tensor cores when its

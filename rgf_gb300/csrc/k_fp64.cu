@@ -10,6 +10,7 @@
 #include <cstdint>
 #include <cstdlib>
 
+#include "rgf_device.h"
 #include "rgf_internal.h"
 
 namespace rgf {
@@ -20,22 +21,6 @@ __device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
                : "+d"(c[0]), "+d"(c[1])
                : "d"(a), "d"(b));
-}
-
-// Every thread of the cluster arrives and waits; shared-memory writes before
-// it are visible to the cluster's reads after it.
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;"
-               ::: "memory");
-}
-// *p of the cluster's CTA `rank` (p: this CTA's shared memory)
-__device__ __forceinline__ double ld_cluster(const double* p, int rank) {
-  unsigned a;
-  double v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-               : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
-  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
-  return v;
 }
 
 struct GemmTileRange {
@@ -200,123 +185,6 @@ __global__ void __launch_bounds__(128) gemm_fp64_kernel(GemmDesc g) {
   }
 }
 
-// ---------------------------------------------------------------------------
-// Leaf Cholesky of one <= 64 x 64 diagonal tile in shared memory.
-// On GB300 each SM sub-partition has its own FP64 unit; one FP64 warp
-// instruction occupies it ~76 cycles whatever the number of active lanes, and
-// a dependent FP64 op waits ~63 (measured), so the column-to-column pivot
-// chain (the next pivot's update, its reciprocal square root, the column's
-// scaling) is the critical path.  The log-determinant is summed later from
-// the factor's diagonal, off this path.
-// ---------------------------------------------------------------------------
-// float -> double by bit manipulation (no FP64 conversion instruction);
-// zero and subnormal floats give zero
-__device__ __forceinline__ double f2d_bits(float f) {
-  const unsigned int u = __float_as_uint(f);
-  const unsigned int ex = (u >> 23) & 0xffu;
-  if (ex == 0) return 0.0;
-  return __longlong_as_double((long long)((unsigned long long)(u >> 31) << 63 |
-                                          (unsigned long long)(ex - 127 + 1023) << 52 |
-                                          (unsigned long long)(u & 0x7fffffu) << 29));
-}
-
-// Reciprocal square root of a normal positive double with few dependent FP64
-// operations (they are the slow link of the leaf's pivot chain): d = m 4^k
-// with m in [1, 4) by integer ops; an FP32 seed y0 = rsqrt(m_hi) is refined
-// once in double-float arithmetic on the FP32 units (m = m_hi + m_lo split
-// exactly from the bit pattern; e = 1 - m y0^2 with FMA-exact products), which
-// gives ~44 bits; one FP64 Newton step then gives full precision.  FP64 ops on
-// the chain: one add, one multiply, two FMAs; the 4^-k scale is an exponent
-// shift.
-__device__ __forceinline__ double rsqrt_fast(double d) {
-  const long long b = __double_as_longlong(d);
-  const int e = (int)((b >> 52) & 0x7ff) - 1023;
-  if (e == -1023) return 1.0 / sqrt(d);                   // subnormal pivot
-  const int k = e >> 1;                                   // d = m * 4^k, m in [1, 4)
-  const long long mb = b - ((long long)(2 * k) << 52);
-  const double m = __longlong_as_double(mb);
-  const int em = (int)((mb >> 52) & 0x7ff) - 1023;        // 0 or 1
-  // m_hi: the top 24 significant bits as a float; m_lo: the remaining 29 bits
-  const float mh = __uint_as_float((unsigned int)(((mb >> 52) - 1023 + 127) << 23) |
-                                   (unsigned int)((mb >> 29) & 0x7fffff));
-  const float ml = (float)(unsigned int)(mb & ((1ll << 29) - 1)) *
-                   __uint_as_float((unsigned int)(127 + em - 52) << 23);
-  const float y0 = rsqrtf(mh);
-  const float p = y0 * y0;
-  const float pe = fmaf(y0, y0, -p);                      // y0^2 = p + pe exactly
-  float t = fmaf(-mh, p, 1.0f);
-  t = fmaf(-mh, pe, t);
-  t = fmaf(-ml, p, t);                                    // e = 1 - m y0^2
-  const double y1 = f2d_bits(y0) + f2d_bits(0.5f * y0 * t);
-  const double hm = __longlong_as_double(mb - (1ll << 52));  // m / 2, exact
-  const double y2 = fma(y1, fma(-hm, y1 * y1, 0.5), y1);    // y1 (1.5 - m y1^2 / 2)
-  return __longlong_as_double(__double_as_longlong(y2) - ((long long)k << 52));
-}
-
-
-// ---------------------------------------------------------------------------
-// Leaf Cholesky, data-flow form: warps hand columns to each other through
-// release/acquire on a shared-memory counter (no CTA-wide barrier per
-// column); see leaf_chol below.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void st_release_cta(int* p, int v) {
-  asm volatile("st.release.cta.shared::cta.b32 [%0], %1;"
-               :: "r"((unsigned)__cvta_generic_to_shared(p)), "r"(v) : "memory");
-}
-__device__ __forceinline__ int ld_acquire_cta(const int* p) {
-  int v;
-  asm volatile("ld.acquire.cta.shared::cta.b32 %0, [%1];"
-               : "=r"(v) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
-  return v;
-}
-
-// The leaf Cholesky proper, on the tile held in shared memory S (lower part).
-// Column c belongs to warp c % 8.  Step j applies the final column j of L to
-// every later column (one FMA per column and 32 rows: L_cj is a broadcast
-// read); the owner of column j + 1 does that column first, then takes its
-// pivot d from shared memory in every lane (rsqrt on all lanes costs the same
-// warp instruction as on one), scales the column to its final value
-// (L_rc = S_rc d^{-1/2}, L_cc = d d^{-1/2}) and publishes it with a release
-// store.  FP64 ops on the pivot chain per column: FMA, the four of rsqrt_fast,
-// one multiply.  Columns are written only by their owner; column j is
-// read-only once published.  Waits are bounded by wait_polls polls, after
-// which the leaf records a timeout and stops.
-__device__ __forceinline__ void leaf_finalize(double (*S)[65], int nbk, int c, int lane,
-                                              int* ready, int* fail) {
-  __syncwarp();
-  const double d = S[c][c];
-  const bool ok = d > 0.0;
-  const double y = ok ? rsqrt_fast(d) : __longlong_as_double(0x7ff8000000000000LL);
-  for (int r = c + lane; r < nbk; r += 32) S[r][c] = (r == c ? d : S[r][c]) * y;
-  if (!ok && lane == 0) atomicMin(fail, c);
-  __syncwarp();
-  if (lane == 0) st_release_cta(ready, c);
-}
-
-__device__ void leaf_chol(double (*S)[65], int nbk, DevStatus* st, int wait_polls, int* ready,
-                          int* abort_, int* fail) {
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (warp == 0) leaf_finalize(S, nbk, 0, lane, ready, fail);
-  for (int j = 0; j + 1 < nbk; ++j) {
-    if (ld_acquire_cta(ready) < j) {
-      int it = 0;
-      while (ld_acquire_cta(ready) < j && !*(volatile int*)abort_ && ++it < wait_polls) {
-      }
-      if (it >= wait_polls) {
-        *(volatile int*)abort_ = 1;
-        if (lane == 0) atomicExch(&st->timeout, 1);
-      }
-      if (*(volatile int*)abort_) break;
-    }
-    int c = j + 1 + ((warp - (j + 1)) % 8 + 8) % 8;  // first owned column > j
-    for (; c < nbk; c += 8) {
-      const double lcj = S[c][j];
-      for (int r = c + lane; r < nbk; r += 32) S[r][c] = fma(-S[r][j], lcj, S[r][c]);
-      if (c == j + 1) leaf_finalize(S, nbk, c, lane, ready, fail);
-    }
-  }
-}
-
 // Row-parallel solve X := X L^{-T} (MODE 0) or X := X L^{-1} (MODE 1) of the
 // rows [r0, r0 + nthreads/8) of X against the nbk x nbk lower tile in Ls.
 // Eight lanes share one row: lane q of the group keeps the unknowns
@@ -366,33 +234,6 @@ __device__ __forceinline__ void trsm_rows_body(double* X, long long xrs, long lo
       if (l < nbk) X[r * xrs + (long long)l * xcs] = u[t];
     }
   }
-}
-
-// Leaf Cholesky of the nbk x nbk lower tile T in one CTA (leaf_chol).  The
-// rows below the leaf are solved by a separate trsm_rows launch: folding that
-// solve into this launch (CTAs that wait for the leaf) was measured slower at
-// ns=2000, as the waiting CTAs hold SMs that the concurrent side-stream
-// products need.
-__global__ void __launch_bounds__(256) leaf_potrf_kernel(double* T, long long ldt, int nbk,
-                                                         int col0, DevStatus* st, int wait_polls) {
-  __shared__ double S[64][65];
-  __shared__ int ready, abort_, fail;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  pdl_wait();
-  for (int c = warp; c < nbk; c += 8)
-    for (int r = c + lane; r < nbk; r += 32) S[r][c] = T[(long long)r + (long long)c * ldt];
-  if (tid == 0) {
-    fail = 0x7fffffff;
-    abort_ = 0;
-    ready = -1;
-  }
-  __syncthreads();
-  leaf_chol(S, nbk, st, wait_polls, &ready, &abort_, &fail);
-  __syncthreads();
-  pdl_trigger();
-  for (int c = warp; c < nbk; c += 8)
-    for (int r = c + lane; r < nbk; r += 32) T[(long long)r + (long long)c * ldt] = S[r][c];
-  if (tid == 0 && fail != 0x7fffffff) atomicMin(&st->not_spd_col, col0 + fail);
 }
 
 // Row-parallel triangular solve with a <= 64 x 64 lower tile (trsm_rows_body):
@@ -712,13 +553,6 @@ int launch_gemm_fp64(const GemmDesc& g0, cudaStream_t s) {
     return 2;
   }
   return 1;
-}
-
-void launch_leaf_potrf(double* T, long long ldt, int nbk, int col0, DevStatus* st,
-                       cudaStream_t s, int wait_polls) {
-  if (nbk <= 0) return;
-  launch_k(leaf_potrf_kernel, dim3(1), dim3(256), 0, s, T, ldt, nbk, col0, st,
-           wait_polls > 0 ? wait_polls : LEAF_WAIT_POLLS);
 }
 
 void launch_trsm_rows(double* X, long long xrs, long long xcs, int rows, const double* L,

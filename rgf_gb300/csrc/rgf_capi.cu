@@ -30,7 +30,7 @@
 using namespace rgf;
 
 namespace {
-constexpr int NB = 64;  // leaf tile of the FP64 panel Cholesky / triangular solves
+constexpr int NB = 64;  // leaf tile of the batched inverses and the corner's triangular solves
 // FP64 refinement of split-precision solves: at most this many correction
 // steps; refinement stops as soon as every right-hand side's normalized
 // residual ||b - A x|| / ||b|| is at or below RGF_REFINE_TOL (one step
@@ -48,6 +48,7 @@ struct rgf_handle {
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   bool on_side = false;  // launch wrappers issue to `side`
+  bool side_used = false;  // the side stream has work that the main stream has not joined
   bool lookahead = true;
   // complex Hermitian instance held as its real embedding (2ns, nt, 2nd):
   // x, b and diag of the C ABI are then complex (interleaved re, im) of size nc
@@ -80,6 +81,8 @@ struct rgf_handle {
   double* d_ref = nullptr;      // refinement of split solves: x, b, y (3 n nrhs)
   double* d_norms = nullptr;    // refinement: ||r_q||, ||b_q|| per right-hand side (2 x 4096)
   size_t ref_cap = 0;           // doubles
+  double* d_panel_ws = nullptr;  // per tile of a diagonal block: launch_panel_tile's ws
+  double* d_arrow = nullptr;     // partial sums of the corner update (launch_arrow_syrk)
   double* d_gemm_ws = nullptr;  // split-K partial sums of small FP64 GEMMs
   double* d_gemm_ws_side = nullptr;  // the same for the side stream
   long long gemm_ws_elems = 0;
@@ -111,7 +114,7 @@ struct rgf_handle {
   // tuning knobs (rgf_set_tuning / rgf_autotune); knob_gen counts changes so
   // that a batch graph captured with older knobs is captured again
   int leaf_wait_polls = 0;   // poll limit of the leaf's pivot waits (0 = default)
-  int nb = 32;               // leaf width of the panel Cholesky (16, 32 or 64)
+  int nb = 32;               // leaf_nb knob (16, 32 or 64): see panel_width
   double split_bias = 1.0;   // the estimated split-product time is scaled by it
   int splitk_max = 0;        // tile shapes: split-K cap of the tensor-core products (0 = 16)
   int fp64_tile = 0;         // and the FP64 output tile (0 = per product; split: 32)
@@ -403,10 +406,12 @@ cudaStream_t cur_stream(const rgf_handle* h) { return h->on_side ? h->side : h->
 void fork_side(rgf_handle* h) {
   cudaEventRecord(h->ev_fork, h->stream);
   cudaStreamWaitEvent(h->side, h->ev_fork, 0);
+  h->side_used = true;
 }
 void join_side(rgf_handle* h) {
   cudaEventRecord(h->ev_join, h->side);
   cudaStreamWaitEvent(h->stream, h->ev_join, 0);
+  h->side_used = false;
 }
 
 // Launch trace: an event on the current stream after the launch just issued.
@@ -494,10 +499,31 @@ void gemm(rgf_handle* h, const GemmDesc& g, int cls) {
   }
 }
 
-void leaf_potrf(rgf_handle* h, double* T, long long ldt, int nbk, int col0) {
-  launch_leaf_potrf(T, ldt, nbk, col0, h->d_status, cur_stream(h), h->leaf_wait_polls);
+// Widest diagonal tile factored by one launch.
+int panel_width(const rgf_handle* h) { return h->nb == 16 ? PANEL_TILE / 2 : PANEL_TILE; }
+
+double* panel_ws(rgf_handle* h, int off) {
+  return h->d_panel_ws + (long long)(off / panel_width(h)) * PANEL_WS;
+}
+
+// Cholesky of the w x w tile at P, `off` columns into its diagonal block.
+void panel_tile(rgf_handle* h, double* P, long long lda, int w, int off, int col0) {
+  launch_panel_tile(P, lda, w, panel_ws(h, off), col0, h->d_status, cur_stream(h),
+                    h->leaf_wait_polls);
   h->kernels_issued++;
   trace(h, "leaf");
+}
+
+// X := X L^{-T} for rows below that tile.
+void panel_rows(rgf_handle* h, double* X, int rows, const double* P, long long lda, int w, int off) {
+  if (rows <= 0) return;
+  launch_panel_rows(X, rows, P, lda, w, panel_ws(h, off), cur_stream(h));
+  h->kernels_issued++;
+  if (!h->trace_path.empty()) {
+    char lab[64];
+    std::snprintf(lab, sizeof(lab), "rows%d w%d", rows, w);
+    trace(h, lab);
+  }
 }
 
 void trsm_rows(rgf_handle* h, double* X, long long xrs, long long xcs, int rows,
@@ -518,31 +544,34 @@ void trsm_rows(rgf_handle* h, double* X, long long xrs, long long xcs, int rows,
 // TRSM of the rows below folded in (RGF.H:254-260, 284-287, 312-317, 335 as
 // one pass).  Halving the column range makes every trailing update one GEMM
 // with an inner dimension of half the range, so most of the work runs in a
-// few large products; 64-column leaves are factored in FP64 in one CTA and
-// solved against row-parallel.
+// few large products; 128-column tiles are factored in FP64 by one launch
+// (panel_tile_kernel) and the rows below them solved by another.
+// off: first column of P within the diagonal block.
 //
 // Rows [0, dr) belong to the diagonal block being factored (the column-to-
 // column critical path); rows [dr, rows) are the block rows below it, which
 // nothing on that path reads.  With look-ahead on, their solves and updates
-// go to the side stream, ordered after the main-stream work they read, so the
-// critical path only carries the diagonal block.
-void panel_potrf(rgf_handle* h, double* P, long long lda, int rows, int cols, int dr, int col0) {
-  const int nb = h->nb;
-  const bool la = h->lookahead && h->side;
+// go to the side stream, ordered after the main-stream work they read by event
+// edges, so the critical path only carries the diagonal block.  A block of a
+// single tile has nothing to overlap: its rows stay on the main stream.
+void panel_potrf(rgf_handle* h, double* P, long long lda, int rows, int cols, int dr, int off,
+                 int col0) {
+  const int nb = panel_width(h);
+  const bool la = h->lookahead && h->side && !(off == 0 && dr <= nb);
   const int split_row = la ? dr : rows;  // rows at or past this go to the side stream
   if (cols <= nb) {
-    leaf_potrf(h, P, lda, cols, col0);
-    if (split_row > cols) trsm_rows(h, P + cols, 1, lda, split_row - cols, P, lda, cols, 0);
+    panel_tile(h, P, lda, cols, off, col0);
+    panel_rows(h, P + cols, split_row - cols, P, lda, cols, off);
     if (rows > split_row) {
       fork_side(h);
       h->on_side = true;
-      trsm_rows(h, P + split_row, 1, lda, rows - split_row, P, lda, cols, 0);
+      panel_rows(h, P + split_row, rows - split_row, P, lda, cols, off);
       h->on_side = false;
     }
     return;
   }
   const int c1 = ((cols / 2 + nb - 1) / nb) * nb;
-  panel_potrf(h, P, lda, rows, c1, dr, col0);
+  panel_potrf(h, P, lda, rows, c1, dr, off, col0);
   // trailing update: P[c1:rows, c1:cols] -= P[c1:rows, 0:c1] P[c1:cols, 0:c1]^T
   auto upd = [&](int r0, int m, int cls) {
     if (m <= 0) return;
@@ -574,7 +603,7 @@ void panel_potrf(rgf_handle* h, double* P, long long lda, int rows, int cols, in
   } else {
     upd(c1, split_row - c1, BULK);
   }
-  panel_potrf(h, P + c1 + (long long)c1 * lda, lda, rows - c1, cols - c1, dr - c1, col0 + c1);
+  panel_potrf(h, P + c1 + (long long)c1 * lda, lda, rows - c1, cols - c1, dr - c1, off + c1, col0 + c1);
 }
 
 // ---- stage 1: factorize (RGF.H:233-340) ----
@@ -627,35 +656,30 @@ void issue_factor(rgf_handle* h) {
       }
       g.alpha = -1.0; g.beta = 1.0; g.outLower = 1;
       gemm(h, g, BULK);
-      if (nd > 0) {
-        const double* Cm = Pm + mf_dense_row(sh, i - 1);
-        GemmDesc c;  // corner -= C_{i-1} C_{i-1}^T  (RGF.H:280, 308)
-        c.m = c.n = (int)nd; c.k = (int)ns;
-        c.A = Cm; c.lda = ldm; c.B = Cm; c.ldb = ldm; c.transB = 1;
-        c.C = c.D = corner; c.ldc = c.ldd = nd;
-        c.alpha = -1.0; c.beta = 1.0; c.outLower = 1;
-        // With look-ahead, on the side stream, where C_{i-1} was computed
-        // (no fork needed): nothing else touches the corner until the last
-        // block's join, so the update leaves the critical path.
-        h->on_side = h->lookahead && h->side;
-        gemm(h, c, SMALL);
-        h->on_side = false;
-      }
     }
-    panel_potrf(h, P, lda, (int)lda, (int)ns, (int)ns, (int)(i * ns));
-    if (h->lookahead && h->side && lda > ns) join_side(h);
+    panel_potrf(h, P, lda, (int)lda, (int)ns, (int)ns, 0, (int)(i * ns));
+    if (h->side_used) join_side(h);
     trace(h, "block end");
   }
   if (nd > 0) {
-    const double* Pl = h->d_MF + mf_col_offset(sh, nt - 1);
-    const double* Cl = Pl + mf_dense_row(sh, nt - 1);
-    GemmDesc c;  // corner -= C_{nt-1} C_{nt-1}^T  (RGF.H:332)
-    c.m = c.n = (int)nd; c.k = (int)ns;
-    c.A = Cl; c.lda = mf_lda(sh, nt - 1); c.B = Cl; c.ldb = mf_lda(sh, nt - 1); c.transB = 1;
-    c.C = c.D = corner; c.ldc = c.ldd = nd;
-    c.alpha = -1.0; c.beta = 1.0; c.outLower = 1;
-    gemm(h, c, SMALL);
-    panel_potrf(h, corner, nd, (int)nd, (int)nd, (int)nd, (int)(nt * ns));  // RGF.H:335
+    // corner -= sum_i C_i C_i^T (RGF.H:280, 308, 332): nothing reads the corner
+    // before its own factorization, so all block columns go in one pass at the end
+    if (h->d_arrow) {
+      launch_arrow_syrk(sh, h->d_MF, h->d_arrow, s);
+      h->kernels_issued += 2;
+      trace(h, "corner");
+    } else {
+      for (long long i = 0; i < nt; ++i) {
+        const double* Ci = h->d_MF + mf_col_offset(sh, i) + mf_dense_row(sh, i);
+        GemmDesc c;
+        c.m = c.n = (int)nd; c.k = (int)ns;
+        c.A = Ci; c.lda = mf_lda(sh, i); c.B = Ci; c.ldb = mf_lda(sh, i); c.transB = 1;
+        c.C = c.D = corner; c.ldc = c.ldd = nd;
+        c.alpha = -1.0; c.beta = 1.0; c.outLower = 1;
+        gemm(h, c, SMALL);
+      }
+    }
+    panel_potrf(h, corner, nd, (int)nd, (int)nd, (int)nd, 0, (int)(nt * ns));  // RGF.H:335
   }
   launch_logdet(sh, h->d_MF, h->d_logpart, h->d_scalars, s);
   h->kernels_issued += 2;
@@ -1188,7 +1212,7 @@ void release(rgf_handle* h) {
   void* bufs[] = {h->d_ia, h->d_ja, h->d_a, h->d_MF, h->d_MS, h->d_U, h->d_T1, h->d_T2, h->d_T3,
                   h->d_logpart, h->d_scalars, h->d_diag, h->d_status, h->d_rhs, h->d_partial,
                   h->d_res, h->d_gemm_ws, h->d_gemm_ws_side, h->d_ref, h->d_rhs2,
-                  h->d_norms};
+                  h->d_norms, h->d_panel_ws, h->d_arrow};
   for (void* p : bufs) dfree(p);
   if (h->ev_fork) cudaEventDestroy(h->ev_fork);
   if (h->ev_join) cudaEventDestroy(h->ev_join);
@@ -1322,6 +1346,11 @@ int rgf_create(const size_t* ia, const size_t* ja, const double* a, size_t ns, s
     if ((st = dalloc(h, &h->d_scalars, 8))) break;
     if ((st = dalloc(h, &h->d_diag, n))) break;
     if ((st = dalloc(h, &h->d_status, 1))) break;
+    if ((st = dalloc(h, &h->d_panel_ws, (std::max(ns, nd) + PANEL_TILE / 2 - 1) / (PANEL_TILE / 2) *
+                                            PANEL_WS))) break;
+    if (nd > 0 && nd <= ARROW_SYRK_MAX_ND &&
+        (st = dalloc(h, &h->d_arrow, arrow_syrk_elems(h->sh))))
+      break;
     h->gemm_ws_elems = std::min<long long>(20ll << 20, 8ll * (2 * (long long)ns + (long long)nd) *
                                                            std::max<long long>(ns, nd));
     if ((st = dalloc(h, &h->d_gemm_ws, h->gemm_ws_elems))) break;
@@ -1963,7 +1992,7 @@ int rgf_batch_kernels(rgf_batch* b, long long* kernels) {
 
 // ============================================================================
 // Tuning knobs and the autotuner.  The knobs change how the factorization and
-// selected inversion are cut into kernels (leaf width, look-ahead stream,
+// selected inversion are cut into kernels (diagonal tile width, look-ahead stream,
 // split/FP64 routing), never the operation count; the autotuner measures the
 // candidates on the instance itself and caches the choice per class.
 // ============================================================================
@@ -2024,7 +2053,7 @@ int time_factor_selinv(rgf_handle* h, int reps, double* ms) {
   return RGF_OK;
 }
 
-// Coordinate descent from the current knobs: leaf width, then look-ahead,
+// Coordinate descent from the current knobs: tile width, then look-ahead,
 // then (split precision) the routing bias.  A candidate replaces the best so
 // far only when it is at least 2% faster, so timing noise does not move the
 // choice away from the defaults.
@@ -2044,7 +2073,7 @@ int tune_handle(rgf_handle* h, rgf_tuning* out) {
     if (t.ms < 0.98 * best.ms) best = t;
     return RGF_OK;
   };
-  for (int nb : {16, 32, 64}) {
+  for (int nb : {16, 32}) {  // 64 cuts like 32
     rgf_tuning t = best;
     t.leaf_nb = nb;
     if ((st = trial(t))) return st;

@@ -132,14 +132,23 @@ size_t hermitian_real_index(size_t ns, size_t nt, size_t nd, size_t k, int imag)
 // Returns the number of kernels launched (2 with split-K).
 int launch_gemm_fp64(const GemmDesc& g, cudaStream_t s);
 
-// Cholesky of the nbk x nbk (nbk <= 64) lower tile at T (column-major, ldt),
-// in place.  Records the first non-positive pivot (global column col0 + j) in st.
+// ---- panel factorization (k_panel.cu) -------------------------------------------
+// Cholesky of the w x w (w <= PANEL_TILE) lower tile at P (column-major, lda), in
+// place.  Records the first non-positive pivot (global column col0 + j) in st.
 // Each wait of a column for the previous pivot polls at most wait_polls times
 // (0 = LEAF_WAIT_POLLS); a wait that runs out records a timeout in st and the
-// leaf stops updating.
+// tile's leaves stop updating.  ws (PANEL_WS doubles) receives what
+// launch_panel_rows reads: per 32-column leaf its unit columns, then d^{-1/2}.
+constexpr int PANEL_LEAF = 32, PANEL_TILE = 128;
+constexpr int PANEL_LEAF_WS = PANEL_LEAF * PANEL_LEAF + PANEL_LEAF;
+constexpr int PANEL_WS = PANEL_TILE / PANEL_LEAF * PANEL_LEAF_WS;
 constexpr int LEAF_WAIT_POLLS = 1 << 26;
-void launch_leaf_potrf(double* T, long long ldt, int nbk, int col0, DevStatus* st,
+void launch_panel_tile(double* P, long long lda, int w, double* ws, int col0, DevStatus* st,
                        cudaStream_t s, int wait_polls = 0);
+// X := X L^{-T} for `rows` rows of w columns at X (leading dimension lda), L the
+// tile factored by launch_panel_tile at P (same lda) with its ws.
+void launch_panel_rows(double* X, int rows, const double* P, long long lda, int w,
+                       const double* ws, cudaStream_t s);
 
 // Every device allocation of the library goes through here (so that a test
 // can make one fail: rgf_debug_fail_alloc_after).  cudaMalloc semantics.
@@ -223,6 +232,12 @@ void launch_rhs_norms(long long n, int nrhs, const double* R, const double* B, d
 constexpr int SPMV_MAX_RHS = 16;
 // x += d over len entries
 void launch_add(long long len, double* x, const double* d, cudaStream_t s);
+// corner -= sum_i C_i C_i^T (lower part) over all block columns, for
+// 0 < nd <= ARROW_SYRK_MAX_ND: partial sums per 256 columns of every block
+// column into partial (arrow_syrk_elems doubles), then added in a fixed order.
+constexpr int ARROW_SYRK_MAX_ND = 32;
+long long arrow_syrk_elems(const BtaShape& sh);
+void launch_arrow_syrk(const BtaShape& sh, double* MF, double* partial, cudaStream_t s);
 // out[q*ldo + dd] = sum_i sum_j C_i(dd, j) * R_i(j, q) over block columns,
 // computed as per-block partials then an ordered sum: the arrowhead part of
 // the forward solve.  y_d -= that.
