@@ -384,13 +384,13 @@ __global__ void __launch_bounds__(TILE_THREADS, 5)
     if (nl > 1) { cluster_arrive(); cluster_wait(); }
     for (int k = 0; k < nl; ++k) {
       const int nbk = min(LB, w - k * LB);
-      if (k + 1 == nl) pdl_trigger();  // one leaf left: the next kernel's CTAs may come in
       if (!*wait.abort_) {
         if (warp < LEAF_WARPS) leaf_ldl(S, V, Lc, nbk, &sh, wait);
         else leaf_send<NW>(V, Lc, ys, nbk, wait, k + 1 < nl);
       }
       __syncthreads();
       if (k + 1 < nl) cluster_arrive();  // (workers: rows solved)
+      else pdl_trigger();                // the next kernel's CTAs may come in
       // results: L = V d^{-1/2} to P, the unit columns and d^{-1/2} to ws
       double* D = P + (long long)k * LB * (lda + 1);
       double* W = ws + (long long)k * PANEL_LEAF_WS;

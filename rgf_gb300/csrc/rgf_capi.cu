@@ -257,6 +257,11 @@ static bool arena_release(void* p) {
   return false;
 }
 
+bool& pdl_scope() {
+  static thread_local bool on = true;
+  return on;
+}
+
 bool pdl_enabled() {
   static const bool on = [] {
     const char* v = std::getenv("RGF_GB300_PDL");
@@ -442,6 +447,7 @@ void trace_flush(rgf_handle* h) {
 
 void gemm(rgf_handle* h, const GemmDesc& g, int cls) {
   if (g.m <= 0 || g.n <= 0 || g.batch <= 0) return;
+  const NoPdl scope(h->on_side);
   const bool bulk = cls != SMALL;
   // fp64_diag: 0 = diagonal blocks at the bulk slice count, 1 = at 7 slices
   // (56-bit operands: FP64-accurate emulation), 2 = native FP64 DMMA
@@ -484,6 +490,7 @@ void gemm(rgf_handle* h, const GemmDesc& g, int cls) {
     gw.ws = h->on_side ? h->d_gemm_ws_side : h->d_gemm_ws;
     gw.ws_elems = h->gemm_ws_elems;
     gw.tile = h->fp64_tile;
+    const NoPdl beside(h->side_used);
     launched = launch_gemm_fp64(gw, cur_stream(h));
   }
   h->kernels_issued += launched;
@@ -508,6 +515,7 @@ double* panel_ws(rgf_handle* h, int off) {
 
 // Cholesky of the w x w tile at P, `off` columns into its diagonal block.
 void panel_tile(rgf_handle* h, double* P, long long lda, int w, int off, int col0) {
+  const NoPdl beside(h->side_used);
   launch_panel_tile(P, lda, w, panel_ws(h, off), col0, h->d_status, cur_stream(h),
                     h->leaf_wait_polls);
   h->kernels_issued++;
@@ -517,6 +525,7 @@ void panel_tile(rgf_handle* h, double* P, long long lda, int w, int off, int col
 // X := X L^{-T} for rows below that tile.
 void panel_rows(rgf_handle* h, double* X, int rows, const double* P, long long lda, int w, int off) {
   if (rows <= 0) return;
+  const NoPdl scope(h->on_side);
   launch_panel_rows(X, rows, P, lda, w, panel_ws(h, off), cur_stream(h));
   h->kernels_issued++;
   if (!h->trace_path.empty()) {

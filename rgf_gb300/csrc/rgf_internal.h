@@ -27,12 +27,25 @@ struct DevStatus {
 // returns once the previous kernel in the stream has completed and its writes
 // are visible.  Both are no-ops in a kernel launched without the attribute.
 // RGF_GB300_PDL=0 launches without it.
+// Launches inside a NoPdl scope of this thread go without it too: those of the
+// look-ahead side stream (their early CTAs would wait on SMs that the main
+// stream's kernels need), and, while that stream has work, the diagonal tiles
+// and FP64 products of the main one (a tile that comes in early sits on an SM
+// whose FP64 units another product is still using).  Factorization replayed as
+// a graph with / without those attributes: ns = 2000, nt = 10 split 32.1 / 28.8 ms,
+// ns = 515, nt = 20 split 10.7 / 9.1 ms, ns = 333, nt = 20 FP64 7.9 / 7.2 ms.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 bool pdl_enabled();
+bool& pdl_scope();  // this thread launches with the attribute (default true)
+struct NoPdl {
+  bool before;
+  explicit NoPdl(bool off) : before(pdl_scope()) { pdl_scope() = before && !off; }
+  ~NoPdl() { pdl_scope() = before; }
+};
 
 // launch_k_cluster: the same with thread-block clusters of the given size.
 template <typename... KArgs, typename... Args>
@@ -55,7 +68,7 @@ inline void launch_k_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, dim3
   }
   // created streams only: not the default streams (the legacy one synchronizes
   // with every stream)
-  if (pdl_enabled() && s != nullptr && s != cudaStreamLegacy && s != cudaStreamPerThread) {
+  if (pdl_enabled() && pdl_scope() && s != nullptr && s != cudaStreamLegacy && s != cudaStreamPerThread) {
     at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
     cfg.numAttrs++;
