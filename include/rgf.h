@@ -310,7 +310,8 @@ typedef struct rgf_tuning {
   double ms;        /* out: factorize + RGFdiag time measured by the autotuner
                        for this choice (0 when not measured)                 */
   int splitk_max;   /* tile shapes: largest split-K degree of the tensor-core
-                       products (0 = default 16, 1 = no split K; 2, 4, 8)    */
+                       products (0 = default 8, 1 = no split K; 2, 4; 8
+                       and 16 = 8, the largest cluster)    */
   int fp64_tile;    /* output tile of the FP64 products: 0 = chosen per
                        product (32 or 64), 32 or 64 = always that           */
   int reserved[2];

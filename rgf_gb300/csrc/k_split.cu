@@ -41,6 +41,7 @@
 #include <vector>
 
 #include "../../include/rgf.h"
+#include "rgf_device.h"
 #include "rgf_split.h"
 
 namespace rgf {
@@ -89,15 +90,13 @@ struct SplitParams {
   int mD1;
   double alpha, betac;
   DevStatus* st;
-  // Split K over ksplit CTAs per output tile (blockIdx.z = batch item *
-  // ksplit + slice): slice kz runs the jobs j with j % ksplit == kz, adds its
-  // fixed-point partial sums to the tile's int64 workspace with atomics
-  // (integer sums: the result is the same bits whatever the order) and the
-  // CTA that arrives last at the tile's counter converts, writes D and sets
-  // workspace and counter back to zero.
+  // Split K over ksplit CTAs per output tile, one cluster (blockIdx.z = batch
+  // item * ksplit + slice): slice kz runs the jobs j with j % ksplit == kz.
+  // The slices' fixed-point partial sums stay in their shared memory and meet
+  // through distributed shared memory: each CTA adds up and writes its share of
+  // the tile's columns (integer sums: the result is the same bits however K is
+  // cut).
   int ksplit;
-  long long* wsk;  // 128 x 128 int64 per tile (column-major by tile column)
-  int* cnt;        // arrival counter per tile
 };
 
 // ---- PTX wrappers -----------------------------------------------------------
@@ -327,7 +326,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   uint64_t* mma_done = acc_empty + 2;                      // every MMA of this CTA retired
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  volatile int* last_flag = reinterpret_cast<volatile int*>(tmem_slot + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
@@ -496,59 +494,47 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       if (lane == 0) mbar_arrive(&acc_empty[buf]);
     }
     pdl_trigger();  // the products are done: the next kernel may be scheduled
-    if (p.ksplit > 1) {
-      // split K: add this slice's partial sums to the tile's workspace; the
-      // last slice to arrive takes the total (and leaves zeros behind)
-      const long long tile =
-          blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * zb);
-      unsigned long long* W = reinterpret_cast<unsigned long long*>(p.wsk) + tile * (BM * BN);
-      if (!*abort_flag) {
-#pragma unroll
-        for (int i = 0; i < 64; ++i)
-          if (acc[i] != 0) atomicAdd(&W[(half * 64 + i) * BM + row], (unsigned long long)acc[i]);
-      }
-      __threadfence();
-      asm volatile("bar.sync 1, 256;" ::: "memory");  // the eight drain warps
-      if (warp == 2 && lane == 0) *last_flag = atomicAdd(&p.cnt[tile], 1) == p.ksplit - 1;
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (*last_flag) {
-        __threadfence();
-#pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          unsigned long long* w = &W[(half * 64 + i) * BM + row];
-          acc[i] = (long long)__ldcg(w);
-          __stcg(w, 0ull);
-        }
-        if (warp == 2 && lane == 0) p.cnt[tile] = 0;
-      }
-    }
     // epilogue: every output once, v = alpha acc 2^(er + exB[c]) + beta C.
-    // The accumulators go to the (now idle) pipeline shared memory and a
-    // compact loop converts eight columns per pass -- the C reads of the
+    // The accumulators go to the (now idle) pipeline shared memory, entry
+    // (column half, row) of column i of the half at [i][half * 128 + row].  Without
+    // split K a thread converts its own 64 columns; with it the cluster's CTA
+    // kz takes the tile's columns kz * cs .. + cs, every other one a thread, and
+    // adds up the slices' entries on the way.  Before (64-bit atomics to a
+    // workspace, the last CTA to arrive converting the whole tile) this part of a
+    // 518 x 515 x 515 product took 33 K cycles, now SPLITK_FIGURES.
+    // A compact loop converts eight columns per pass -- the C reads of the
     // eight issued before any is used -- instead of a 64-fold unrolled body
     // (large code, slow to issue).  The columns' exponents come from two
-    // coalesced loads per warp, shuffled to the lanes.  The conversion is
-    // integer arithmetic (i64_scaled): the only FP64 instruction per output is
-    // the FMA with beta C, and it stands outside any per-lane condition: an FP64
-    // instruction holds its unit 76 cycles even when it is predicated off (an
-    // untaken multiplication by alpha and FMA were nearly half of this loop).
+    // loads per lane, shuffled.  The conversion is integer arithmetic
+    // (i64_scaled): the only FP64 instruction per output is the FMA with beta C,
+    // and it stands outside any per-lane condition: an FP64 instruction holds
+    // its unit 76 cycles even when it is predicated off (an untaken
+    // multiplication by alpha and FMA were nearly half of this loop).
     // Measured per 128 x 128 tile: 43 K -> 18 K cycles without C, 43 K -> 27 K
     // with; a 2006 x 128 x 128 product 49 -> 39 us, 2006 x 2000 x 2000 354 -> 327 us.
-    const bool last = p.ksplit == 1 || *last_flag;
-    if (!*abort_flag && last) {
-      const int r = m0 + row;
-      const bool live = r < p.m;
-      const int t = threadIdx.x - 64;  // drain thread 0..255
-      long long* eacc = reinterpret_cast<long long*>(smem) + t;  // 64 x 256 int64 = 128 KiB
-      // alpha = -1 is a negation of the integers
-      const int amode = p.alpha == 1.0 ? 0 : (p.alpha == -1.0 ? 1 : 2);
+    const int r = m0 + row;
+    const bool live = r < p.m;
+    long long* eacc = reinterpret_cast<long long*>(smem);  // 64 x 256 int64 = 128 KiB
+    // alpha = -1 is a negation of the integers
+    const int amode = p.alpha == 1.0 ? 0 : (p.alpha == -1.0 ? 1 : 2);
 #pragma unroll
-      for (int i = 0; i < 64; ++i) eacc[i * 256] = amode == 1 ? -acc[i] : acc[i];
-      __syncwarp();
-      const int cbase = n0 + half * 64;
+    for (int i = 0; i < 64; ++i) eacc[i * 256 + half * 128 + row] = amode == 1 ? -acc[i] : acc[i];
+    __syncwarp();
+    if (p.ksplit > 1) {
+      cluster_arrive();
+      cluster_wait();
+    }
+    // this thread's columns of the tile: cfirst + cstep * i, i < count
+    const int cs = (BN + p.ksplit - 1) / p.ksplit;
+    const int cstep = p.ksplit > 1 ? 2 : 1;
+    const int cfirst = p.ksplit > 1 ? kz * cs + half : half * 64;
+    const int cend = p.ksplit > 1 ? min(BN, kz * cs + cs) : half * 64 + 64;
+    if (!*abort_flag) {
+      const int cbase = n0 + cfirst;
       const int* exBz = p.exB + (long long)zb * p.exB_stride;
-      const int ex_lo = cbase + lane < p.n ? exBz[cbase + lane] : 0;
-      const int ex_hi = cbase + 32 + lane < p.n ? exBz[cbase + 32 + lane] : 0;
+      const int ca = cbase + cstep * lane, cb = ca + cstep * 32;
+      const int ex_lo = ca < p.n ? exBz[ca] : 0;
+      const int ex_hi = cb < p.n ? exBz[cb] : 0;
       const bool hi = p.D2 && r >= p.mD1;
       const double* C = hi ? p.C2 + (long long)zb * p.sC - p.mD1
                            : (p.C ? p.C + (long long)zb * p.sC : nullptr);
@@ -556,19 +542,21 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       const int er =
           live ? p.exA[(long long)zb * p.exA_stride + r] + p.cs - p.beta * (p.S + 1) + 2 : 0;
       const double alpha = p.alpha, betac = p.betac;
-      const long long ldc = p.ldc, ldd = p.ldd;
-      const int ncols = live ? min(64, p.n - cbase) : 0;          // columns < n
-      const int cdiag = p.outLower ? r - cbase : 64;                // columns c <= r only
-      const int nlive = max(0, min(ncols, cdiag + 1));
-      const int c_lo = p.outUpper ? r - cbase : 0;                  // columns c >= r only
+      const long long ldc = p.ldc * cstep, ldd = p.ldd * cstep;
+      // columns c with c < n, c <= r (outLower), c >= r (outUpper): i in [c_lo, nlive)
+      int climit = min(n0 + cend, p.n);  // first column not written
+      if (p.outLower) climit = min(climit, r + 1);
+      const int nlive = live && climit > cbase ? (climit - cbase + cstep - 1) / cstep : 0;
+      const int c_lo = p.outUpper && r > cbase ? (r - cbase + cstep - 1) / cstep : 0;
       // the warp's columns: from the first any lane writes to the last
       const int i_end = __reduce_max_sync(0xffffffffu, nlive);
-      const int i_beg = max(0, __reduce_min_sync(0xffffffffu, c_lo)) & ~7;
+      const int i_beg = __reduce_min_sync(0xffffffffu, c_lo) & ~7;
       auto convert = [&](auto with_c) {
         constexpr bool WITH_C = decltype(with_c)::value;
         // column pointers advance by ldc / ldd (no 64-bit multiply per output)
-        const double* Cp = WITH_C && live ? C + r + (long long)(cbase + i_beg) * ldc : nullptr;
-        double* Dp = live ? D + r + (long long)(cbase + i_beg) * ldd : nullptr;
+        const double* Cp =
+            WITH_C && live ? C + r + (cbase + (long long)cstep * i_beg) * p.ldc : nullptr;
+        double* Dp = live ? D + r + (cbase + (long long)cstep * i_beg) * p.ldd : nullptr;
 #pragma unroll 1
         for (int i0 = i_beg; i0 < i_end; i0 += 8) {
           double cv[8];
@@ -579,11 +567,28 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
               Cp += ldc;
             }
           }
+          long long w[8];
+          if (p.ksplit > 1) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) w[q] = 0;
+#pragma unroll 4
+            for (int z = 0; z < p.ksplit; ++z) {  // 32 remote reads in flight
+              const unsigned base = cluster_addr(eacc + row, z);
+#pragma unroll
+              for (int q = 0; q < 8; ++q) {
+                const int c = min(cfirst + cstep * (i0 + q), BN - 1);  // column of the tile
+                w[q] += ld_cluster_i64(base + ((c & 63) * 256 + (c >> 6) * 128) * 8);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) w[q] = eacc[(i0 + q) * 256 + half * 128 + row];
+          }
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             const int i = i0 + q;
             const int ec = __shfl_sync(0xffffffffu, i0 < 32 ? ex_lo : ex_hi, i & 31);
-            double v = i64_scaled(eacc[i * 256], er + ec);
+            double v = i64_scaled(w[q], er + ec);
             if (amode == 2) {
               __syncwarp();  // a real branch, not a predicated multiplication
               v *= alpha;
@@ -597,6 +602,19 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       if (p.betac != 0.0) convert(std::true_type{});
       else convert(std::false_type{});
     }
+    __syncwarp();
+  }
+  if (p.ksplit > 1) {
+    // the cluster's barriers count every thread: the producer and MMA warps
+    // join the one before the sums here; the second keeps a CTA's shared memory
+    // in place until all have read it
+    if (warp < 2) {
+      __syncwarp();
+      cluster_arrive();
+      cluster_wait();
+    }
+    cluster_arrive();
+    cluster_wait();
   }
   tc_fence_before();
   __syncthreads();
@@ -615,13 +633,8 @@ __device__ __forceinline__ bool tri_ok(int tri, int r, int k) {
   return tri == TRI_NONE || (tri == TRI_LOWER ? k <= r : k >= r);
 }
 
-// Balanced base-2^beta digits of x * 2^(beta*S - 1 - e) (truncated to an
-// integer, |.| < 2^(beta*S - 1)): S digits, most significant first, the top
-// one in [-2^(beta-1), 2^(beta-1)] and the others in [-2^(beta-1),
-// 2^(beta-1) - 1], written to S planes `plane` elements apart.  With beta = 8
-// every digit is exact in bf16 and every digit product is at most 2^14.
-__device__ __forceinline__ void write_digits(unsigned long long bits, int e, int S, int beta,
-                                             __nv_bfloat16* o, size_t plane) {
+// x * 2^(beta*S - 1 - e), truncated to an integer (|.| < 2^(beta*S - 1))
+__device__ __forceinline__ long long fixed_point(unsigned long long bits, int e, int S, int beta) {
   const bool neg = (bits >> 63) != 0;
   int E = (int)((bits >> 52) & 0x7ff);
   unsigned long long mant = bits & 0xfffffffffffffull;
@@ -632,15 +645,76 @@ __device__ __forceinline__ void write_digits(unsigned long long bits, int e, int
     if (sh >= 0) xi = sh < 64 ? (mant << sh) : 0ull;
     else xi = -sh < 64 ? (mant >> (-sh)) : 0ull;
   }
-  long long v = neg ? -(long long)xi : (long long)xi;
+  return neg ? -(long long)xi : (long long)xi;
+}
+
+// next balanced digit of v (least significant first): in [-2^(beta-1), 2^(beta-1) - 1]
+__device__ __forceinline__ int next_digit(long long& v, int beta) {
   const int half = 1 << (beta - 1), mask = (1 << beta) - 1;
-  for (int s = S - 1; s > 0; --s) {
-    int d = (int)v & mask;
-    d -= d >= half ? mask + 1 : 0;
-    v = (v - d) >> beta;
-    o[(size_t)s * plane] = __float2bfloat16_rn((float)d);
-  }
+  int d = (int)v & mask;
+  d -= d >= half ? mask + 1 : 0;
+  v = (v - d) >> beta;
+  return d;
+}
+
+// Balanced base-2^beta digits of fixed_point(x): S digits, most significant
+// first, the top one in [-2^(beta-1), 2^(beta-1)] and the others in
+// [-2^(beta-1), 2^(beta-1) - 1], written to S planes `plane` elements apart.
+// With beta = 8 every digit is exact in bf16 and every digit product is at most
+// 2^14.
+__device__ __forceinline__ void write_digits(unsigned long long bits, int e, int S, int beta,
+                                             __nv_bfloat16* o, size_t plane) {
+  long long v = fixed_point(bits, e, S, beta);
+  for (int s = S - 1; s > 0; --s)
+    o[(size_t)s * plane] = __float2bfloat16_rn((float)next_digit(v, beta));
   o[0] = __float2bfloat16_rn((float)(int)v);
+}
+
+// The same (beta = 8) for two neighbouring terms, as one 32-bit store per plane
+// (o is at an even term of rows whose pitch is a multiple of 64 terms: 4-byte
+// aligned).  With 128 added at every lower digit's place, the bytes of the sum
+// are the digits plus 128: no digit waits for another one's borrow.  A byte
+// becomes a float as the mantissa of 2^23 + byte, and its bf16 is the float's
+// upper half (eight significant bits): no conversion instruction.  fixed_point
+// is one 64-bit shift: the mantissa is below bit 63 before it goes right.
+__device__ __forceinline__ long long fixed_point8(unsigned long long bits, int e, int S) {
+  const int E = (int)((bits >> 52) & 0x7ff);
+  const unsigned long long mant =
+      ((bits & 0xfffffffffffffull) | (E ? 1ull << 52 : 0ull)) << 10;
+  // x 2^(8 S - 1 - e) = mant 2^-rs; |x| < 2^e bounds rs below by 0
+  const unsigned rs = (unsigned)(1086 + e - 8 * S - max(E, 1));
+  unsigned long long xi;
+  asm("shr.u64 %0, %1, %2;" : "=l"(xi) : "l"(mant), "r"(rs));  // 0 for rs > 63
+  return (long long)bits < 0 ? -(long long)xi : (long long)xi;
+}
+template <int ST>  // number of digits, 0: S
+__device__ __forceinline__ void write_digit_pair(unsigned long long bits0, unsigned long long bits1,
+                                                 int e, int S, __nv_bfloat16* o, size_t plane) {
+  const int n = ST ? ST : S;
+  const long long v0 = fixed_point8(bits0, e, n), v1 = fixed_point8(bits1, e, n);
+  unsigned* q = reinterpret_cast<unsigned*>(o + (size_t)(n - 1) * plane);
+  const size_t step = plane / 2;
+  // 128 at each of the n - 1 lower digits' places
+  const unsigned long long bias = 0x0080808080808080ull >> (8 * (8 - n));
+  const unsigned long long w0 = (unsigned long long)v0 + bias, w1 = (unsigned long long)v1 + bias;
+  auto pack = [](float f0, float f1) {
+    return __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632);
+  };
+  auto byte_float = [](unsigned long long w, int i) {
+    const unsigned h = i < 4 ? (unsigned)w : (unsigned)(w >> 32);
+    return __uint_as_float(__byte_perm(h, 0x4Bu, 0x4550u | (unsigned)(i & 3))) - 8388736.0f;
+  };
+#pragma unroll
+  for (int i = 0; i < 7; ++i) {
+    if (i >= n - 1) break;
+    *q = pack(byte_float(w0, i), byte_float(w1, i));
+    q -= step;
+  }
+  // the top digit, signed, halved sums so that it cannot overflow at n = 8
+  auto top = [&](long long v) {
+    return (float)(int)(n == 1 ? v : ((v >> 1) + (long long)(bias >> 1)) >> (8 * (n - 1) - 1));
+  };
+  *q = pack(top(v0), top(v1));
 }
 
 __device__ __forceinline__ int exp_of_max(unsigned long long mx) {
@@ -742,13 +816,19 @@ __global__ void slice_kernel(const double* X, long long rs, long long ks, int R,
   }
 }
 
-// Both operands of a product with a short K in one launch: a CTA owns 32 rows
-// of op(A) or op(B) (blockIdx.x below nblkA: A) and SLICE_KC terms of K
-// (blockIdx.y); it finds the rows' maximum magnitudes over all of K, then
-// writes the S digit planes of its K range tile by tile.
-// Replaces the max / exponent / slice kernels (and the memsets) of the long-K
-// path, which dominate small products.
-constexpr int SLICE_KC = 128;  // K terms sliced per CTA of slice_pair_kernel
+// Both operands of a product in one launch (K up to SLICE_MAX_K): a CTA owns 32
+// rows of op(A) or op(B) (blockIdx.x below nblkA: A) and kc terms of K
+// (blockIdx.y); the CTAs of a row block form a cluster.  Each reads its part of
+// the operand once, along the contiguous dimension, into shared memory, finds
+// the rows' maximum magnitudes over it, takes the maxima over the cluster
+// through distributed shared memory, and writes the S digit planes from shared
+// memory, two terms (one 32-bit store) a lane.  Bound by latency on small
+// operands and by the reads and writes (8 + 2 S bytes a term) on large ones.
+// Before, every CTA of a row block read all of K for the maxima (K <= 512), or
+// memset, maximum, exponent and slice kernels ran per operand (longer K):
+// SLICE_FIGURES
+constexpr int SLICE_MAX_KC = 256;                // K terms of one CTA
+constexpr int SLICE_MAX_K = 8 * SLICE_MAX_KC;    // of a cluster
 
 struct SliceOperand {
   const double* X;
@@ -759,10 +839,13 @@ struct SliceOperand {
   __nv_bfloat16* out;
 };
 
-__global__ void __launch_bounds__(256) slice_pair_kernel(SliceOperand a, SliceOperand b, int nblkA,
-                                                          int K, int Kp, int S, int beta) {
-  __shared__ double tile[32][33];
-  __shared__ unsigned long long red[8][33];
+template <int NW, int ST>  // warps of a CTA; digits (0: S)
+__global__ void __launch_bounds__(NW * 32) slice_pair_kernel(SliceOperand a, SliceOperand b, int nblkA,
+                                                          int K, int Kp, int kc, int S) {
+  extern __shared__ double tile[];  // [row][k], pitch kc + 1
+  __shared__ unsigned long long red[NW][32];
+  __shared__ unsigned long long rmax[32];  // this CTA's row maxima, read by the cluster
+  __shared__ int exs[32];
   pdl_wait();
   pdl_trigger();
   const bool isA = (int)blockIdx.x < nblkA;
@@ -771,77 +854,75 @@ __global__ void __launch_bounds__(256) slice_pair_kernel(SliceOperand a, SliceOp
   const long long z = blockIdx.z;
   const double* X = o.X + z * o.sX;
   const double* Xb = o.X2 ? o.X2 - o.R1 + z * o.sX : X;
-  int* ex = o.ex + z * o.Rp;
-  __nv_bfloat16* out = o.out + (size_t)z * S * o.Rp * Kp;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  auto val = [&](int r, int k) -> double {
-    if (r >= o.R || k >= K || !tri_ok(o.tri, r, k)) return 0.0;
-    return (o.X2 && r >= o.R1 ? Xb : X)[(long long)r * o.rs + (long long)k * o.ks];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int k0 = blockIdx.y * kc, kn = min(kc, Kp - k0);  // this CTA's terms (kn a multiple of 64)
+  const int pitch = kc + 1;
+  auto bits = [](double v) {
+    return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
   };
-  // pass 1: row maxima of |x| as bit patterns
-  if (o.rs == 1) {  // rows contiguous: lane = row, warp = k phase
+  if (o.rs == 1) {  // rows contiguous: lane = row, warp = phase of k
+    const int r = r0 + lane;
+    const double* x = (o.X2 && r >= o.R1 ? Xb : X) + r + (long long)(k0 + warp) * o.ks;
+    const long long dx = NW * o.ks;
     unsigned long long m = 0;
 #pragma unroll 8
-    for (int k = ty; k < K; k += 8) {  // independent loads in flight
-      const unsigned long long v =
-          (unsigned long long)__double_as_longlong(val(r0 + tx, k)) & 0x7fffffffffffffffull;
-      m = v > m ? v : m;
+    for (int k = warp; k < kn; k += NW) {  // independent loads in flight
+      double v = 0.0;
+      if (r < o.R && k0 + k < K && tri_ok(o.tri, r, k0 + k)) v = *x;
+      x += dx;
+      tile[lane * pitch + k] = v;
+      m = max(m, bits(v));
     }
-    red[ty][tx] = m;
-  } else {  // k contiguous: warp = 4 rows, lane = k phase
+    red[warp][lane] = m;
+    __syncthreads();
+    if (warp == 0) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int rl = ty + 8 * i;
+      for (int w = 1; w < NW; ++w) m = max(m, red[w][lane]);
+      rmax[lane] = m;
+    }
+  } else {  // k contiguous: a warp takes every NW-th row, lane = phase of k
+#pragma unroll
+    for (int i = 0; i < 32 / NW; ++i) {
+      const int rl = warp + NW * i, r = r0 + rl;
+      const double* x = X + (long long)r * o.rs + k0;
       unsigned long long m = 0;
 #pragma unroll 4
-      for (int k = tx; k < K; k += 32) {
-        const unsigned long long v =
-            (unsigned long long)__double_as_longlong(val(r0 + rl, k)) & 0x7fffffffffffffffull;
-        m = v > m ? v : m;
+      for (int k = lane; k < kn; k += 32) {
+        double v = 0.0;
+        if (r < o.R && k0 + k < K && tri_ok(o.tri, r, k0 + k)) v = x[k];
+        tile[rl * pitch + k] = v;
+        m = max(m, bits(v));
       }
 #pragma unroll
-      for (int d = 16; d > 0; d >>= 1) {
-        const unsigned long long y = __shfl_xor_sync(0xffffffffu, m, d);
-        m = y > m ? y : m;
-      }
-      if (tx == 0) red[0][rl] = m;
+      for (int d = 16; d > 0; d >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
+      if (lane == 0) rmax[rl] = m;
     }
   }
   __syncthreads();
-  __shared__ int exs[32];
-  if (threadIdx.x < 32) {
-    unsigned long long m = red[0][threadIdx.x];
-    if (o.rs == 1)
-      for (int w = 1; w < 8; ++w) m = red[w][threadIdx.x] > m ? red[w][threadIdx.x] : m;
-    const int r = r0 + threadIdx.x;
-    const int e = r < o.R ? exp_of_max(m) : 0;
-    exs[threadIdx.x] = e;
-    if (r < o.Rp && blockIdx.y == 0) ex[r] = e;
+  const int nk = gridDim.y;
+  if (nk > 1) cluster_sync();
+  if (warp == 0) {
+    unsigned long long m = rmax[lane];
+    for (int q = 0; q < nk; ++q)
+      m = max(m, (unsigned long long)ld_cluster_i64(cluster_addr(&rmax[lane], q)));
+    const int r = r0 + lane, e = r < o.R ? exp_of_max(m) : 0;
+    exs[lane] = e;
+    if (blockIdx.y == 0) o.ex[z * o.Rp + r] = e;  // (Rp is a multiple of 32)
   }
   __syncthreads();
-  // pass 2: digits, one 32 x 32 tile at a time (read along the contiguous
-  // dimension, write along k)
+  if (nk > 1) cluster_arrive();  // the maxima have been read here
   const size_t plane = (size_t)o.Rp * Kp;
-  // this CTA's K range: SLICE_KC terms (blockIdx.y); the row maxima above span all of K
-  const int kend = min(Kp, ((int)blockIdx.y + 1) * SLICE_KC);
-  for (int k0 = blockIdx.y * SLICE_KC; k0 < kend; k0 += 32) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      int rl, kl;
-      if (o.rs == 1) { rl = tx; kl = ty + 8 * i; }
-      else           { kl = tx; rl = ty + 8 * i; }
-      tile[rl][kl] = val(r0 + rl, k0 + kl);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int rl = ty + 8 * i, r = r0 + rl, k = k0 + tx;
-      if (r >= o.Rp) continue;
-      write_digits((unsigned long long)__double_as_longlong(tile[rl][tx]), exs[rl], S, beta,
-                   out + (size_t)r * Kp + k, plane);
-    }
-    __syncthreads();
+#pragma unroll 1
+  for (int i = 0; i < 32 / NW; ++i) {
+    const int rl = warp + NW * i, e = exs[rl];
+    const double* t = tile + rl * pitch + 2 * lane;
+    __nv_bfloat16* out = o.out + (size_t)z * S * plane + (size_t)(r0 + rl) * Kp + k0 + 2 * lane;
+#pragma unroll 1
+    for (int k = 0; k < kn; k += 64)
+      write_digit_pair<ST>((unsigned long long)__double_as_longlong(t[k]),
+                           (unsigned long long)__double_as_longlong(t[k + 1]), e, S, out + k, plane);
   }
+  if (nk > 1) cluster_wait();
 }
 
 // ---- host side ------------------------------------------------------------------
@@ -894,7 +975,36 @@ SplitEngine* SplitEngine::create(int slices, int* status) {
     *status = RGF_ENOTSUP;
     return nullptr;
   }
+  for (auto* k : {slice_pair_kernel<16, 0>, slice_pair_kernel<16, 5>, slice_pair_kernel<16, 7>})
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(32 * (SLICE_MAX_KC + 1) * sizeof(double))) != cudaSuccess) {
+      cudaGetLastError();
+      *status = RGF_ENOTSUP;
+      return nullptr;
+    }
   SplitEngine* e = new SplitEngine();
+  // how many clusters of each split-K degree the device holds at once
+  static std::once_flag once;
+  static std::array<int, MAX_SPLITK + 1> clusters{};
+  std::call_once(once, [] {
+    for (int k = 2; k <= MAX_SPLITK; ++k) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(1, 1, k);
+      cfg.blockDim = dim3(NUM_THREADS);
+      cfg.dynamicSmemBytes = SMEM_BYTES;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = k;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&clusters[k], split_gemm_kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        clusters[k] = 0;
+      }
+    }
+  });
+  e->max_clusters_ = clusters;
   e->slices_ = slices > 0 ? slices : 5;
   e->min_k_ = 64;
   return e;
@@ -902,36 +1012,6 @@ SplitEngine* SplitEngine::create(int slices, int* status) {
 
 SplitEngine::~SplitEngine() {
   device_free(ws_);
-  device_free(wsk_);
-}
-
-int SplitEngine::ensure_splitk(long long tiles, cudaStream_t s) {
-  if (tiles <= wsk_tiles_) return RGF_OK;
-  device_free(wsk_);
-  wsk_ = nullptr;
-  cnt_ = nullptr;
-  wsk_tiles_ = 0;
-  const size_t bytes = (size_t)tiles * BM * BN * sizeof(long long) + (size_t)tiles * sizeof(int);
-  void* p = nullptr;
-  if (device_malloc(&p, bytes) != cudaSuccess) {
-    cudaGetLastError();
-    return RGF_ENOMEM;
-  }
-  if (cudaMemsetAsync(p, 0, bytes, s) != cudaSuccess) {  // ordered before this stream's use
-    device_free(p);
-    return RGF_ECUDA;
-  }
-  wsk_ = static_cast<long long*>(p);
-  cnt_ = reinterpret_cast<int*>(wsk_ + (size_t)tiles * BM * BN);
-  wsk_tiles_ = tiles;
-  return RGF_OK;
-}
-
-int SplitEngine::reset_splitk(cudaStream_t s) {
-  if (!wsk_) return RGF_OK;
-  const size_t bytes = (size_t)wsk_tiles_ * BM * BN * sizeof(long long) +
-                       (size_t)wsk_tiles_ * sizeof(int);
-  return cudaMemsetAsync(wsk_, 0, bytes, s) == cudaSuccess ? RGF_OK : RGF_ECUDA;
 }
 
 int SplitEngine::ensure_ws(size_t bytes) {
@@ -949,7 +1029,6 @@ int SplitEngine::ensure_ws(size_t bytes) {
 
 namespace {
 constexpr int MAX_SLICES = 8;
-constexpr int SHORT_K = 512;  // products with K up to this slice both operands in one launch
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 // bytes of workspace one batch item of an (RpA x Kp) by (RpB x Kp) problem needs
 size_t item_bytes(int S, int RpA, int RpB, int Kp) {
@@ -1061,13 +1140,10 @@ double SplitEngine::estimate_seconds(const GemmDesc& g, int slices) const {
     const int chunk = std::max(1, EXACT_TERMS / (SBK * gr.count));
     jobs += (Kp / SBK + chunk - 1) / chunk;
   }
-  long long ksplit = 1;
-  if (wsk_ && tiles * 2 <= num_sms_ && (long long)tx * ty * g.batch <= wsk_tiles_)
-    ksplit = std::max<long long>(
-        1, std::min<long long>({(long long)splitk_max_, jobs, num_sms_ / std::max(1ll, tiles)}));
+  const long long ksplit = split_k(tiles, jobs);
   const double waves = std::ceil((double)(tiles * ksplit) / num_sms_);
   const bool same = g.A == g.B && g.lda == g.ldb && g.transA != g.transB;
-  const double t_slice = (Kp <= SHORT_K ? 8e-6 : 16e-6) +
+  const double t_slice = (Kp <= SLICE_MAX_K ? 8e-6 : 16e-6) +
                          (g.m + (same ? 0.0 : g.n)) * (double)Kp * (8.0 + 2.0 * S) * g.batch / 3e12;
   const double steps = (double)plan.slots.size() * (Kp / 16.0) / ksplit;
   return 20e-6 + t_slice + waves * steps * 120e-9;
@@ -1100,7 +1176,7 @@ bool SplitEngine::supports(const GemmDesc& g) const {
          round_up(g.k, BKE) <= max_k_;
 }
 
-int SplitEngine::prepare(int max_rows, int max_k, int batch_hint, cudaStream_t s) {
+int SplitEngine::prepare(int max_rows, int max_k, int batch_hint) {
   max_rows_ = round_up(std::max(max_rows, 1), BM);
   max_k_ = round_up(std::max(max_k, 1), BKE);
   int dev = 0;
@@ -1109,10 +1185,17 @@ int SplitEngine::prepare(int max_rows, int max_k, int batch_hint, cudaStream_t s
     cudaGetLastError();
     return RGF_ECUDA;
   }
-  int st = reserve(max_rows_, max_k_, batch_hint);
-  if (st) return st;
-  // split K serves launches whose tiles cover at most half of the SMs
-  return ensure_splitk(std::max(1, num_sms_ / 2), s);
+  return reserve(max_rows_, max_k_, batch_hint);
+}
+
+// Split-K degree for `tiles` output tiles of `jobs` jobs each: when the tiles
+// fill at most half of the SMs, the largest cluster (up to 8 CTAs) of which the
+// device holds one per tile at the same time.
+int SplitEngine::split_k(long long tiles, int jobs) const {
+  if (tiles * 2 > num_sms_) return 1;
+  int k = std::min({splitk_max_, jobs, MAX_SPLITK});
+  while (k > 1 && tiles > max_clusters_[k]) --k;
+  return std::max(1, k);
 }
 
 long long SplitEngine::gemm(const GemmDesc& g, cudaStream_t s, DevStatus* st,
@@ -1195,14 +1278,27 @@ long long SplitEngine::gemm(const GemmDesc& g, cudaStream_t s, DevStatus* st,
     const double* A = g.A + (long long)b0 * g.sA;
     const double* A2 = g.A2 ? g.A2 + (long long)b0 * g.sA : nullptr;
     const double* B = g.B + (long long)b0 * g.sB;
-    if (Kp <= SHORT_K) {
+    if (Kp <= SLICE_MAX_K) {
       SliceOperand oa{A, A2, g.transA ? g.lda : 1, g.transA ? 1 : g.lda, g.sA, g.m,
                       A2 ? g.mA1 : g.m, RpA, g.triA, exA, sa};
       SliceOperand ob{B, nullptr, g.transB ? 1 : g.ldb, g.transB ? g.ldb : 1, g.sB, g.n, g.n,
                       RpB, triBt, exB, sb};
       const int nblkA = RpA / 32, nblkB = same ? 0 : RpB / 32;
-      launch_k(slice_pair_kernel, dim3(nblkA + nblkB, (Kp + SLICE_KC - 1) / SLICE_KC, nbat),
-               dim3(256), 0, s, oa, ob, nblkA, (int)g.k, Kp, S, beta);
+      // K over a cluster of up to 8 CTAs of 64, 128, ... or 256 terms each
+      const int parts = std::min(8, Kp / 64);
+      const int kc = round_up((Kp + parts - 1) / parts, 64), nk = (Kp + kc - 1) / kc;
+      // 8 warps up to 128 terms a CTA, 16 above: a CTA of 256 terms holds 66 KB of
+      // shared memory, three to an SM, and needs the threads to move them
+      static_assert(SPLIT_BETA == 8, "write_digit_pair");
+      auto* kern = kc <= 128 ? (S == 5   ? slice_pair_kernel<8, 5>
+                                : S == 7 ? slice_pair_kernel<8, 7>
+                                         : slice_pair_kernel<8, 0>)
+                             : (S == 5   ? slice_pair_kernel<16, 5>
+                                : S == 7 ? slice_pair_kernel<16, 7>
+                                         : slice_pair_kernel<16, 0>);
+      launch_k_cluster(kern, dim3(nblkA + nblkB, nk, nbat), dim3(kc <= 128 ? 256 : 512),
+                       dim3(1, nk, 1), (size_t)32 * (kc + 1) * sizeof(double), s, oa, ob, nblkA,
+                       (int)g.k, Kp, kc, S);
       launched += 1;
     } else {
       if (!g.transA) slice(A, 1, g.lda, g.sA, g.m, g.triA, exA, mxA, sa, RpA, A2, g.mA1);
@@ -1232,25 +1328,17 @@ long long SplitEngine::gemm(const GemmDesc& g, cudaStream_t s, DevStatus* st,
     p.C2 = g.C2 ? g.C2 + (long long)b0 * g.sC : nullptr;
     p.D2 = g.D2 ? g.D2 + (long long)b0 * g.sD : nullptr;
     p.mD1 = g.mD1;
-    // split K when the output tiles fill at most half of the SMs (and the
-    // workspace holds them): up to 16 slices of a tile's jobs, so that the
-    // launch covers about one wave
     const int ntiles = (int)tiles_written(g, BM);
-    const long long grid_tiles = (long long)(RpA / BM) * (RpB / BN) * nbat;
-    p.ksplit = 1;
-    if (wsk_ && (long long)ntiles * nbat * 2 <= num_sms_ && grid_tiles <= wsk_tiles_) {
-      int jobs = 0;  // jobs of a tile with the full K range
-      for (int gi = 0; gi < p.ngroups; ++gi) jobs += (Kp / SBK + p.gchunk[gi] - 1) / p.gchunk[gi];
-      p.ksplit = std::max(1, std::min({splitk_max_, jobs, num_sms_ / (ntiles * nbat)}));
-    }
-    p.wsk = wsk_;
-    p.cnt = cnt_;
+    int jobs = 0;  // jobs of a tile with the full K range
+    for (int gi = 0; gi < p.ngroups; ++gi) jobs += (Kp / SBK + p.gchunk[gi] - 1) / p.gchunk[gi];
+    p.ksplit = split_k((long long)ntiles * nbat, jobs);
     dim3 grid(RpA / BM, RpB / BN, nbat * p.ksplit);
     if (tensor_flops) {
       const double tiles = ntiles;  // tiles with nothing to write are skipped
       *tensor_flops += tiles * nbat * 2.0 * BM * BN * (double)round_up(Kp, SBK) * np;
     }
-    launch_k(split_gemm_kernel, grid, dim3(NUM_THREADS), SMEM_BYTES, s, ma, mb, p);
+    launch_k_cluster(split_gemm_kernel, grid, dim3(NUM_THREADS), dim3(1, 1, p.ksplit), SMEM_BYTES, s,
+                     ma, mb, p);
     launched += 1;
   }
   return launched;

@@ -116,7 +116,7 @@ struct rgf_handle {
   int leaf_wait_polls = 0;   // poll limit of the leaf's pivot waits (0 = default)
   int nb = 32;               // leaf_nb knob (16, 32 or 64): see panel_width
   double split_bias = 1.0;   // the estimated split-product time is scaled by it
-  int splitk_max = 0;        // tile shapes: split-K cap of the tensor-core products (0 = 16)
+  int splitk_max = 0;        // tile shapes: split-K cap of the tensor-core products (0 = 8)
   int fp64_tile = 0;         // and the FP64 output tile (0 = per product; split: 32)
   double tuned_ms = 0.0;     // factorize + RGFdiag time measured by the autotuner
   long long knob_gen = 0;
@@ -1106,10 +1106,6 @@ int sync_and_check(rgf_handle* h) {
   DevStatus st;
   RGF_CK(cudaMemcpy(&st, h->d_status, sizeof(st), cudaMemcpyDeviceToHost));
   if (st.timeout) {
-    // a split product that gave up may have left its split-K workspace dirty
-    for (SplitEngine* e : {h->split, h->split_side})
-      if (e) e->reset_splitk(h->stream);
-    cudaStreamSynchronize(h->stream);
     return RGF_ETIMEOUT;
   }
   if (st.bad_input) return RGF_EINVAL;
@@ -1386,11 +1382,11 @@ int rgf_create(const size_t* ia, const size_t* ja, const double* a, size_t ns, s
       h->split = SplitEngine::create(o.slices, &st);
       if (st) break;
       // operands have at most 2ns+nd rows and ns+nd terms
-      st = h->split->prepare((int)(2 * ns + nd), (int)(ns + nd), (int)nt, h->stream);
+      st = h->split->prepare((int)(2 * ns + nd), (int)(ns + nd), (int)nt);
       if (st) break;
       h->split_side = SplitEngine::create(o.slices, &st);
       if (st) break;
-      st = h->split_side->prepare((int)(ns + nd), (int)ns, 1, h->stream);
+      st = h->split_side->prepare((int)(ns + nd), (int)ns, 1);
       if (st) break;
     }
     if (async) {  // copies and ingests overlap the first factorization
@@ -1744,7 +1740,7 @@ int rgf_dgemm_device(int precision, int slices, char transa, char transb, int m,
   SplitEngine* eng = nullptr;
   if (precision == RGF_PREC_SPLIT) {
     eng = SplitEngine::create(slices, &status);
-    if (!status) status = eng->prepare(std::max(m, n), k, 1, s);
+    if (!status) status = eng->prepare(std::max(m, n), k, 1);
   }
   if (!status) {
     if (eng && eng->supports(g)) eng->gemm(g, s, st);

@@ -35,6 +35,11 @@ __device__ __forceinline__ unsigned cluster_addr(const void* p, int rank) {
       : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
   return a;
 }
+__device__ __forceinline__ long long ld_cluster_i64(unsigned addr) {
+  long long v;
+  asm volatile("ld.shared::cluster.b64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ void st_cluster(unsigned addr, double v) {
   asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
 }

@@ -6,6 +6,7 @@
 
 #include <cuda.h>
 
+#include <array>
 #include <cstddef>
 #include <map>
 #include <tuple>
@@ -23,14 +24,14 @@ class SplitEngine {
   // terms (allocates once, outside any graph capture).
   // batch_hint: largest batch the caller issues (sizes the workspace so that
   // batched problems run in few chunks; capped at 1 GiB).
-  // The split-K workspace is cleared on stream s (before its first use there).
-  int prepare(int max_rows, int max_k, int batch_hint, cudaStream_t s);
+  int prepare(int max_rows, int max_k, int batch_hint);
   // True when g can run on the tensor cores (k >= min_k and within the
   // prepared sizes; batched problems run in chunks that fit the workspace).
   bool supports(const GemmDesc& g) const;
   int slices() const { return slices_; }
-  // Largest split-K degree (1 = none); a tuning knob.
-  void set_splitk_max(int k) { splitk_max_ = k > 0 ? k : 16; }
+  // Largest split-K degree (1 = none, 0 = default); a tuning knob.
+  static constexpr int MAX_SPLITK = 8;
+  void set_splitk_max(int k) { splitk_max_ = k > 0 ? k : MAX_SPLITK; }
   // MMA streams per output tile and K term at S slices (each one N=256 MMA
   // of one A digit against two B digits, or N=128 against one)
   static int slots(int S);
@@ -42,17 +43,13 @@ class SplitEngine {
   // slices > 0 overrides the engine's slice count (up to 8) for this call.
   long long gemm(const GemmDesc& g, cudaStream_t s, DevStatus* st,
                  double* tensor_flops = nullptr, int slices = 0);
-  // Zero the split-K workspace and counters (they clear themselves after
-  // every launch that completes; a launch that gave up on a wait may leave
-  // them dirty).
-  int reset_splitk(cudaStream_t s);
 
  private:
   SplitEngine() = default;
   int ensure_ws(size_t bytes);
   bool map_for(CUtensorMap* out, void* base, int S, int Rp, int Kp);
   std::map<std::tuple<void*, int, int, int>, CUtensorMap> maps_;
-  int ensure_splitk(long long tiles, cudaStream_t s);
+  int split_k(long long tiles, int jobs) const;
   int reserve(int max_rows, int max_k, int batch_hint);
   int slices_ = 0;
   int min_k_ = 1 << 30;
@@ -60,11 +57,8 @@ class SplitEngine {
   void* ws_ = nullptr;
   size_t ws_bytes_ = 0;
   int num_sms_ = 148;
-  int splitk_max_ = 16;
-  // split K: int64 partial sums (128 x 128 per tile) and arrival counters
-  long long* wsk_ = nullptr;
-  int* cnt_ = nullptr;
-  long long wsk_tiles_ = 0;
+  int splitk_max_ = MAX_SPLITK;
+  std::array<int, MAX_SPLITK + 1> max_clusters_{};  // per split-K degree
 };
 
 }  // namespace rgf
