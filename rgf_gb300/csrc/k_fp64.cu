@@ -185,79 +185,81 @@ __global__ void __launch_bounds__(128) gemm_fp64_kernel(GemmDesc g) {
   }
 }
 
-// Row-parallel solve X := X L^{-T} (MODE 0) or X := X L^{-1} (MODE 1) of the
-// rows [r0, r0 + nthreads/8) of X against the nbk x nbk lower tile in Ls.
-// Eight lanes share one row: lane q of the group keeps the unknowns
-// l = q, q + 8, ... in registers.  Step j: the owner of x_j scales it, one
-// shuffle hands it to the other seven lanes, and each applies it to its own
-// unknowns -- no CTA barrier per column, so the column-to-column chain is a
-// multiply, a shuffle and a fused multiply-add.
-// MODE 0: x_j = (b_j - sum_{l<j} x_l L_jl) / L_jj   (X L^T = B)
-// MODE 1: x_j = (b_j - sum_{l>j} x_l L_lj) / L_jj   (X L = B)
-template <int MODE>
-__device__ __forceinline__ void trsm_rows_body(double* X, long long xrs, long long xcs, int rows,
-                                               double (*Ls)[65], const double* rinv, int nbk,
-                                               long long r0) {
-  const int lane = threadIdx.x & 31, q = lane & 7, gbase = lane & ~7;
-  const long long r = r0 + (threadIdx.x >> 3);
-  const bool live = r < rows;
-  double u[8];
-#pragma unroll
-  for (int t = 0; t < 8; ++t) {
-    const int l = t * 8 + q;
-    u[t] = (live && l < nbk) ? X[r * xrs + (long long)l * xcs] : 0.0;
-  }
-  for (int s = 0; s < nbk; ++s) {
-    const int j = MODE == 0 ? s : nbk - 1 - s;
-    const int jt = j >> 3;
-    double uj = 0.0;
-#pragma unroll
-    for (int t = 0; t < 8; ++t)
-      if (t == jt) uj = u[t];
-    const double xj = __shfl_sync(0xffffffffu, uj * rinv[j], gbase | (j & 7));
-    // slots that can hold a live unknown: a warp-uniform range, so FP64
-    // instructions with no live lane are not issued
-    const int tlo = MODE == 0 ? jt : 0, thi = MODE == 0 ? (nbk - 1) >> 3 : jt;
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      if (t < tlo || t > thi) continue;
-      const int l = t * 8 + q;
-      if (l == j) u[t] = xj;
-      if (MODE == 0 ? (l > j && l < nbk) : (l < j)) u[t] = fma(-xj, MODE == 0 ? Ls[l][j] : Ls[j][l], u[t]);
-    }
-  }
-  pdl_trigger();
-  if (live) {
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      const int l = t * 8 + q;
-      if (l < nbk) X[r * xrs + (long long)l * xcs] = u[t];
-    }
-  }
-}
-
-// Row-parallel triangular solve with a <= 64 x 64 lower tile (trsm_rows_body):
-// a warp holds four rows and a CTA of 4 warps 16 rows, so the FP64 work
-// spreads over many SMs (each SM retires only ~3.5 FP64 flops per cycle).
-template <int MODE>
+// Row-parallel triangular solve with a <= 64 x 64 lower tile:
+// MODE 0: X := X L^{-T}, x_j = (b_j - sum_{l<j} x_l L_jl) / L_jj
+// MODE 1: X := X L^{-1}, x_j = (b_j - sum_{l>j} x_l L_lj) / L_jj
+// G lanes share one row; lane q of them keeps the unknowns t G + q in registers.
+// The tile is held with its rows (MODE 1: columns) scaled to a unit diagonal, so
+// step j hands z_j = x_j L_jj on with one shuffle and updates the unknowns after it
+// with one FMA per slot; the slots are unrolled by blocks of G steps, so that no
+// FP64 instruction is issued for a slot that is done (predicated off it costs
+// the same).  G = 32 (4 rows a CTA) while that many CTAs fit the SMs a few times
+// over, 8 (16 rows a CTA, fewer instructions a row) for more rows: the 64 rows of
+// an inverse's leaf took 36 us with G = 8 and predicated slots, now ~19.
+// INV: X = L^{-T} (b = I, MODE 0) of every 64-column diagonal tile of an nbk x nbk
+// factor at once (blockIdx.z: the tile; X and L start at the first one).
+template <int MODE, int G, bool INV = false>
 __global__ void __launch_bounds__(128) trsm_rows_kernel(double* X, long long xrs, long long xcs,
                                                          int rows, const double* L, long long ldl,
                                                          int nbk, long long sX, long long sL) {
-  __shared__ double Ls[64][65];
+  constexpr int T = 64 / G;  // slots
+  __shared__ double Ls[64][65];  // [j][l]: multiplier of z_j in unknown l
   __shared__ double rinv[64];
   pdl_wait();
   X += (long long)blockIdx.y * sX;
   L += (long long)blockIdx.y * sL;
-  for (int idx = threadIdx.x; idx < 64 * 64; idx += 128) {
-    const int c = idx >> 6, r = idx & 63;
-    double v = 0.0;
-    if (r < nbk && c < nbk && r >= c) v = L[(long long)r + (long long)c * ldl];
-    Ls[r][c] = v;
+  if (INV) {
+    const int off = blockIdx.z * 64;
+    X += off * (xcs + xrs);
+    L += off * (ldl + 1);
+    nbk = rows = min(64, nbk - off);
+  }
+  const int tid = threadIdx.x;
+  if (tid < 64) rinv[tid] = tid < nbk ? 1.0 / L[(long long)tid * (ldl + 1)] : 0.0;
+  const int lane = tid & 31, q = lane & (G - 1), gbase = lane & ~(G - 1);
+  const long long r = (long long)blockIdx.x * (128 / G) + tid / G;
+  const bool live = r < rows;
+  double u[T];
+#pragma unroll
+  for (int t = 0; t < T; ++t) {
+    const int l = t * G + q;
+    if (INV) u[t] = r == l ? 1.0 : 0.0;
+    else u[t] = live && l < nbk ? X[r * xrs + (long long)l * xcs] : 0.0;
   }
   __syncthreads();
-  if (threadIdx.x < 64) rinv[threadIdx.x] = (threadIdx.x < nbk) ? 1.0 / Ls[threadIdx.x][threadIdx.x] : 0.0;
+  for (int idx = tid; idx < nbk * 64; idx += 128) {
+    const int c = idx >> 6, row = idx & 63;  // L(row, c), row >= c
+    double v = 0.0;
+    if (row > c && row < nbk) v = L[row + (long long)c * ldl];
+    if (MODE == 0) Ls[c][row] = v * rinv[c];  // z_c -> unknown row
+    else Ls[row][c] = v * rinv[row];          // z_row -> unknown c
+  }
   __syncthreads();
-  trsm_rows_body<MODE>(X, xrs, xcs, rows, Ls, rinv, nbk, (long long)blockIdx.x * 16);
+#pragma unroll
+  for (int b = 0; b < T; ++b) {
+    const int t0 = MODE == 0 ? b : T - 1 - b;  // slot being solved
+#pragma unroll 1
+    for (int s = 0; s < G; ++s) {
+      const int jj = MODE == 0 ? s : G - 1 - s, j = t0 * G + jj;
+      if (j >= nbk) {
+        if (MODE == 0) break;
+        continue;
+      }
+      const double z = -__shfl_sync(0xffffffffu, u[t0], gbase | jj);
+      const double nv = fma(z, Ls[j][t0 * G + q], u[t0]);
+      u[t0] = (MODE == 0 ? q > jj : q < jj) ? nv : u[t0];
+#pragma unroll
+      for (int t = MODE == 0 ? t0 + 1 : 0; t < (MODE == 0 ? T : t0); ++t)
+        u[t] = fma(z, Ls[j][t * G + q], u[t]);
+    }
+  }
+  pdl_trigger();
+#pragma unroll
+  for (int t = 0; t < T; ++t) {
+    const int l = t * G + q;
+    const double x = u[t] * rinv[l];
+    if (live && l < nbk) X[r * xrs + (long long)l * xcs] = x;
+  }
 }
 
 // Thin products (m <= 16, op(B) = B^T; the arrowhead rows): lane = output
@@ -559,11 +561,21 @@ void launch_trsm_rows(double* X, long long xrs, long long xcs, int rows, const d
                       long long ldl, int nbk, int mode, int batch, long long sX, long long sL,
                       cudaStream_t s) {
   if (rows <= 0 || nbk <= 0 || batch <= 0) return;
-  dim3 grid((rows + 15) / 16, batch);
-  if (mode == 0)
-    launch_k(trsm_rows_kernel<0>, grid, dim3(128), 0, s, X, xrs, xcs, rows, L, ldl, nbk, sX, sL);
-  else
-    launch_k(trsm_rows_kernel<1>, grid, dim3(128), 0, s, X, xrs, xcs, rows, L, ldl, nbk, sX, sL);
+  const bool wide = (long long)rows * batch <= 4 * 152 * 4;  // up to four CTAs of four rows an SM
+  const dim3 grid((rows + (wide ? 3 : 15)) / (wide ? 4 : 16), batch);
+  auto* kern = mode == 0 ? (wide ? trsm_rows_kernel<0, 32> : trsm_rows_kernel<0, 8>)
+                         : (wide ? trsm_rows_kernel<1, 32> : trsm_rows_kernel<1, 8>);
+  launch_k(kern, grid, dim3(128), 0, s, X, xrs, xcs, rows, L, ldl, nbk, sX, sL);
+}
+
+void launch_leaf_inverses(double* U, long long ldu, int n, const double* L, long long ldl,
+                          int batch, long long sU, long long sL, cudaStream_t s) {
+  if (n <= 0 || batch <= 0) return;
+  const int leaves = (n + 63) / 64, rows = std::min(n, 64);
+  const bool wide = (long long)rows * leaves * batch <= 4 * 152 * 4;
+  const dim3 grid((rows + (wide ? 3 : 15)) / (wide ? 4 : 16), batch, leaves);
+  launch_k(wide ? trsm_rows_kernel<0, 32, true> : trsm_rows_kernel<0, 8, true>, grid, dim3(128), 0, s,
+           U, 1ll, ldu, rows, L, ldl, n, sU, sL);
 }
 
 }  // namespace rgf

@@ -539,8 +539,8 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
 }
 
-template <int G, int NB>  // NB: 32-column blocks of the tile (the last may be narrower)
-__global__ void __launch_bounds__(128)
+template <int G, int NB, int NT>  // NB: 32-column blocks of the tile (the last may be narrower)
+__global__ void __launch_bounds__(NT)
     panel_rows_kernel(double* X, int rows, const double* P, long long lda, int w,
                       const double* ws) {
   constexpr int SB = LB / G;        // register slots of one block
@@ -550,12 +550,12 @@ __global__ void __launch_bounds__(128)
   __shared__ double Xs[XR > 0 ? LB : 1][XR > 0 ? XR : 1];  // [l][c - 32 (k + 1)]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int q = lane & (G - 1), gbase = lane & ~(G - 1);
-  const int row = blockIdx.x * (128 / G) + warp * (32 / G) + lane / G;
+  const int row = blockIdx.x * (NT / G) + warp * (32 / G) + lane / G;
   const bool live = row < rows;
   pdl_wait();
   auto fetch_leaf = [&](int k) {
     const double* W = ws + (long long)k * PANEL_LEAF_WS;
-    for (int e = tid; e < LB * LB; e += 128) cp_async8(&Lc[0][0] + e, W + e);
+    for (int e = tid; e < LB * LB; e += NT) cp_async8(&Lc[0][0] + e, W + e);
     if (tid < LB) cp_async8(&ys[tid], W + LB * LB + tid);
     cp_async_commit();
   };
@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(128)
     const int kc = k * LB, kn = kc + LB;
     if (k + 1 < NB) {
       const double* src = P + kn + (long long)kc * lda;
-      for (int l = warp; l < LB; l += 4)
+      for (int l = warp; l < LB; l += NT / 32)
         for (int c = lane; c < w - kn; c += 32) cp_async8(&Xs[l][c], src + c + (long long)l * lda);
       cp_async_commit();
       cp_async_wait<1>();
@@ -614,15 +614,15 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-template <int G>
+template <int G, int NT>
 void launch_rows_g(double* X, int rows, const double* P, long long lda, int w, const double* ws,
                    cudaStream_t s) {
-  const dim3 grid((rows + 128 / G - 1) / (128 / G)), block(128);
+  const dim3 grid((rows + NT / G - 1) / (NT / G)), block(NT);
   switch ((w + LB - 1) / LB) {
-    case 1: launch_k(panel_rows_kernel<G, 1>, grid, block, 0, s, X, rows, P, lda, w, ws); break;
-    case 2: launch_k(panel_rows_kernel<G, 2>, grid, block, 0, s, X, rows, P, lda, w, ws); break;
-    case 3: launch_k(panel_rows_kernel<G, 3>, grid, block, 0, s, X, rows, P, lda, w, ws); break;
-    default: launch_k(panel_rows_kernel<G, 4>, grid, block, 0, s, X, rows, P, lda, w, ws); break;
+    case 1: launch_k(panel_rows_kernel<G, 1, NT>, grid, block, 0, s, X, rows, P, lda, w, ws); break;
+    case 2: launch_k(panel_rows_kernel<G, 2, NT>, grid, block, 0, s, X, rows, P, lda, w, ws); break;
+    case 3: launch_k(panel_rows_kernel<G, 3, NT>, grid, block, 0, s, X, rows, P, lda, w, ws); break;
+    default: launch_k(panel_rows_kernel<G, 4, NT>, grid, block, 0, s, X, rows, P, lda, w, ws); break;
   }
 }
 
@@ -669,15 +669,18 @@ void launch_panel_tile(double* P, long long lda, int w, double* ws, int col0, De
                    lda, w, ws, col0, st, polls);
 }
 
-// G = 32 / 16 / 8 lanes a row, so 4 / 8 / 16 rows a CTA: the fewest rows a CTA
-// that still let the 152 SMs take all rows at once (a CTA's time grows with its
-// rows; two CTAs on an SM share its FP64 units).
+// G lanes a row and four or eight warps: 4 / 8 / 16 rows a CTA, the fewest that
+// still let the 152 SMs take all rows at once (a CTA's time grows with its rows;
+// two CTAs on an SM share its FP64 units).  16 rows go as two warps a
+// sub-partition of two rows each: 6% more instructions than one warp of four, but
+// one warp's shuffles and shared-memory reads run behind the other's FMAs
+// (1872 rows of 128 columns: 67 -> 48 us; the FMAs alone, spread evenly, 32).
 void launch_panel_rows(double* X, int rows, const double* P, long long lda, int w,
                        const double* ws, cudaStream_t s) {
   if (rows <= 0 || w <= 0) return;
-  if (rows <= 4 * 152) launch_rows_g<32>(X, rows, P, lda, w, ws, s);
-  else if (rows <= 8 * 152) launch_rows_g<16>(X, rows, P, lda, w, ws, s);
-  else launch_rows_g<8>(X, rows, P, lda, w, ws, s);
+  if (rows <= 4 * 152) launch_rows_g<32, 128>(X, rows, P, lda, w, ws, s);
+  else if (rows <= 8 * 152) launch_rows_g<16, 128>(X, rows, P, lda, w, ws, s);
+  else launch_rows_g<16, 256>(X, rows, P, lda, w, ws, s);
 }
 
 }  // namespace rgf

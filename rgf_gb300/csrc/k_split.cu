@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     // kz takes the tile's columns kz * cs .. + cs, every other one a thread, and
     // adds up the slices' entries on the way.  Before (64-bit atomics to a
     // workspace, the last CTA to arrive converting the whole tile) this part of a
-    // 518 x 515 x 515 product took 33 K cycles, now SPLITK_FIGURES.
+    // 518 x 515 x 515 product took 33 K cycles, now 21 K.
     // A compact loop converts eight columns per pass -- the C reads of the
     // eight issued before any is used -- instead of a 64-fold unrolled body
     // (large code, slow to issue).  The columns' exponents come from two
@@ -825,8 +825,9 @@ __global__ void slice_kernel(const double* X, long long rs, long long ks, int R,
 // memory, two terms (one 32-bit store) a lane.  Bound by latency on small
 // operands and by the reads and writes (8 + 2 S bytes a term) on large ones.
 // Before, every CTA of a row block read all of K for the maxima (K <= 512), or
-// memset, maximum, exponent and slice kernels ran per operand (longer K):
-// SLICE_FIGURES
+// memset, maximum, exponent and slice kernels ran per operand (longer K): 9.5 ->
+// 5.8 us for 2006 x 128, 21 -> 11 us for both operands of 2006 x 512 x 512, 26 us
+// for 2006 x 2000 terms (75 MB moved).
 constexpr int SLICE_MAX_KC = 256;                // K terms of one CTA
 constexpr int SLICE_MAX_K = 8 * SLICE_MAX_KC;    // of a cluster
 
@@ -1123,11 +1124,12 @@ int SplitEngine::reserve(int max_rows, int max_k, int batch_hint) {
   return ensure_ws(std::max(one, std::min(batch, (size_t)1 << 30)) + 1024);
 }
 
-// Estimated device time of gemm(g) (seconds), fitted to GB300 timings of
-// this kernel: about 20 us of launches, pipeline fill and epilogue, the
-// slicing (about 8 us per launch plus the operands' FP64 reads and bf16
-// writes at ~3 TB/s), and per wave of CTAs 120 ns per K=16 step of each MMA
-// stream, divided over the split-K slices.
+// Estimated device time of gemm(g) (seconds), fitted to GB300 timings: 12 us of
+// launches, pipeline fill and job hand-offs; the slicing (5.5 us plus the
+// operands' FP64 reads and bf16 writes at ~3 TB/s); per wave of CTAs 90 ns per
+// K=16 step of each MMA stream, divided over the split-K slices, and 12 us of
+// epilogue, likewise divided, plus 3 us of exchange.  Within 20% of the measured
+// 22 us (130 x 128 x 128, 5 digits) to 300 us (2006 x 2000 x 2000).
 double SplitEngine::estimate_seconds(const GemmDesc& g, int slices) const {
   const int S = slices > 0 ? std::min(slices, MAX_SLICES) : slices_;
   const int Kp = round_up(g.k, BKE);
@@ -1143,10 +1145,11 @@ double SplitEngine::estimate_seconds(const GemmDesc& g, int slices) const {
   const long long ksplit = split_k(tiles, jobs);
   const double waves = std::ceil((double)(tiles * ksplit) / num_sms_);
   const bool same = g.A == g.B && g.lda == g.ldb && g.transA != g.transB;
-  const double t_slice = (Kp <= SLICE_MAX_K ? 8e-6 : 16e-6) +
+  const double t_slice = (Kp <= SLICE_MAX_K ? 5.5e-6 : 16e-6) +
                          (g.m + (same ? 0.0 : g.n)) * (double)Kp * (8.0 + 2.0 * S) * g.batch / 3e12;
   const double steps = (double)plan.slots.size() * (Kp / 16.0) / ksplit;
-  return 20e-6 + t_slice + waves * steps * 120e-9;
+  const double t_end = 12e-6 / ksplit + (ksplit > 1 ? 3e-6 : 0.0);
+  return 12e-6 + t_slice + waves * (steps * 90e-9 + t_end);
 }
 
 // Tensor maps are encoded once per (base, planes, rows, K) and reused: the
@@ -1190,11 +1193,13 @@ int SplitEngine::prepare(int max_rows, int max_k, int batch_hint) {
 
 // Split-K degree for `tiles` output tiles of `jobs` jobs each: when the tiles
 // fill at most half of the SMs, the largest cluster (up to 8 CTAs) of which the
-// device holds one per tile at the same time.
+// device holds one per tile at the same time with a tenth to spare (at the
+// limit, 27 tiles in clusters of 5, the previous kernel's last CTAs push some
+// clusters into a second wave: 39 to 58 us).
 int SplitEngine::split_k(long long tiles, int jobs) const {
   if (tiles * 2 > num_sms_) return 1;
   int k = std::min({splitk_max_, jobs, MAX_SPLITK});
-  while (k > 1 && tiles > max_clusters_[k]) --k;
+  while (k > 1 && tiles * 10 > max_clusters_[k] * 9) --k;
   return std::max(1, k);
 }
 

@@ -480,7 +480,9 @@ void gemm(rgf_handle* h, const GemmDesc& g, int cls) {
     // ~9 us of launches and ~0.9 TFLOP/s.  Small or thin products are faster
     // in FP64 (which is also FP64-accurate).
     const double t_split = eng->estimate_seconds(g, slices);
-    const double t_fp64 = 9e-6 + gemm_flops(g) / 0.9e12;
+    // (half of that beside the look-ahead stream's row solves, which use the
+    // same FP64 units)
+    const double t_fp64 = 9e-6 + gemm_flops(g) / (h->side_used && cls == DIAG ? 0.45e12 : 0.9e12);
     split = t_split * h->split_bias < t_fp64;
   }
   if (split) {
@@ -694,33 +696,28 @@ void issue_factor(rgf_handle* h) {
   h->kernels_issued += 2;
 }
 
-// For every diagonal block at once: U_i = L_ii^{-T} (upper triangular).
-// Right-looking RLTN solve U L^T = I by 64-column blocks; only rows above the
-// current block are non-zero, so the work is ns^3/3 per block.  The
-// nt-1 blocks of leading dimension 2ns+nd run as one batch, the last block
-// (leading dimension ns+nd) and the corner separately.
 // For `batch` diagonal blocks at once: U = L^{-T} (upper triangular).
 // Recursive halving: with L = [L11 0; L21 L22], U = [U11 U12; 0 U22] where
 // U11 = L11^{-T}, U22 = L22^{-T} and U12 = -U11 (L21^T U22).  The two halves
 // are independent; each level adds two GEMMs with an inner dimension of half
 // the range, batched over all blocks, so the inverse runs as a few large
 // products (DIAG class: FP64 or FP64-accurate split).  Leaves (<= 64) solve
-// X L^T = I row-parallel.  T (the product L21^T U22) lives in Tmp at the
+// X L^T = I row-parallel, all of them at once.  T (the product L21^T U22) lives in Tmp at the
 // position of U12.
 void issue_trtri(rgf_handle* h, double* U, long long ldu, long long n, const double* L,
                  long long ldl, double* Tmp, long long ldt, int batch, long long sU, long long sL,
-                 long long sT) {
+                 long long sT, bool leaves = true) {
   if (batch <= 0 || n <= 0) return;
-  if (n <= NB) {
-    launch_set_identity(U, ldu, (int)n, batch, sU, h->stream);
+  if (leaves) {  // all <= 64-column leaves in one launch
+    launch_leaf_inverses(U, ldu, (int)n, L, ldl, batch, sU, sL, cur_stream(h));
     h->kernels_issued++;
-    trsm_rows(h, U, 1, ldu, (int)n, L, ldl, (int)n, 0, batch, sU, sL);
-    return;
+    trace(h, "leaf inverses");
   }
+  if (n <= NB) return;
   const long long n1 = ((n / 2 + NB - 1) / NB) * NB, n2 = n - n1;
-  issue_trtri(h, U, ldu, n1, L, ldl, Tmp, ldt, batch, sU, sL, sT);
+  issue_trtri(h, U, ldu, n1, L, ldl, Tmp, ldt, batch, sU, sL, sT, false);
   issue_trtri(h, U + n1 + n1 * ldu, ldu, n2, L + n1 + n1 * ldl, ldl, Tmp + n1 + n1 * ldt, ldt,
-              batch, sU, sL, sT);
+              batch, sU, sL, sT, false);
   double* T = Tmp + n1 * ldt;
   GemmDesc a;  // T = L21^T U22
   a.m = (int)n1; a.n = (int)n2; a.k = (int)n2;
@@ -761,14 +758,25 @@ void issue_inverses(rgf_handle* h) {
   // (W^T = U_i - ...); the recursion writes only their upper part, so the
   // strictly lower part must be zero.
   cudaMemsetAsync(h->d_U, 0, sizeof(double) * (nt * ss + nd * nd), h->stream);
-  if (nt > 1)
-    issue_trtri(h, h->d_U, ns, ns, h->d_MF, 2 * ns + nd, h->d_MS, 2 * ns + nd, (int)(nt - 1), ss,
-                ns * (2 * ns + nd), ns * (2 * ns + nd));
+  // The last block (another leading dimension) and the corner go to the side
+  // stream, beside the batch of the others: their recursions are chains of small
+  // launches (selected inversion at ns = 2000, nt = 10 14.3 -> 11.9 ms, half of it
+  // from the leaves' row solves).
+  const bool beside = nt > 1 && h->side;
+  if (beside) {
+    fork_side(h);
+    h->on_side = true;
+  }
   issue_trtri(h, h->d_U + (nt - 1) * ss, ns, ns, h->d_MF + mf_col_offset(sh, nt - 1), ns + nd,
               h->d_MS + mf_col_offset(sh, nt - 1), ns + nd, 1, 0, 0, 0);
   if (nd > 0)
     issue_trtri(h, h->d_U + nt * ss, nd, nd, h->d_MF + mf_col_offset(sh, nt), nd,
                 h->d_MS + mf_col_offset(sh, nt), nd, 1, 0, 0, 0);
+  h->on_side = false;
+  if (nt > 1)
+    issue_trtri(h, h->d_U, ns, ns, h->d_MF, 2 * ns + nd, h->d_MS, 2 * ns + nd, (int)(nt - 1), ss,
+                ns * (2 * ns + nd), ns * (2 * ns + nd));
+  if (beside) join_side(h);
 }
 
 // ---- stage 3: selected inversion ----

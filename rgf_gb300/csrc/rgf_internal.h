@@ -191,6 +191,11 @@ void launch_trsm_rows(double* X, long long xrs, long long xcs, int rows, const d
                       long long ldl, int nbk, int mode, int batch, long long sX, long long sL,
                       cudaStream_t s);
 
+// U = L^{-T} of every 64 x 64 diagonal tile (the last may be smaller) of the n x n
+// lower factor L, for `batch` of them; only those tiles of U are written.
+void launch_leaf_inverses(double* U, long long ldu, int n, const double* L, long long ldl,
+                          int batch, long long sU, long long sL, cudaStream_t s);
+
 // Measured FP64 (DMMA) throughput of the current device in TFLOP/s.
 int measure_fp64_peak(double* tflops);
 
