@@ -312,8 +312,8 @@ typedef struct rgf_tuning {
   int splitk_max;   /* tile shapes: largest split-K degree of the tensor-core
                        products (0 = default 8, 1 = no split K; 2, 4; 8
                        and 16 = 8, the largest cluster)    */
-  int fp64_tile;    /* output tile of the FP64 products: 0 = chosen per
-                       product (32 or 64), 32 or 64 = always that           */
+  int fp64_tile;    /* output tile of the FP64 products: 0 = default (32), 32
+                       or 64 = always that                                  */
   int reserved[2];
 } rgf_tuning;
 

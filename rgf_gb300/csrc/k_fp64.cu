@@ -52,8 +52,10 @@ __global__ void __launch_bounds__(128) gemm_fp64_kernel(GemmDesc g) {
   const int m0 = blockIdx.x * TM;
   const int n0 = blockIdx.y * TM;
   if (!tile_written(g.outLower, g.outUpper, m0, n0, TM)) return;
-  const bool splitk = g.ksplit > 1;              // blockIdx.z is the K slice, batch == 1
-  const long long bz = splitk ? 0 : blockIdx.z;
+  // blockIdx.z = batch item * ksplit + K slice; the slices of a tile are a cluster
+  const bool splitk = g.ksplit > 1;
+  const long long bz = blockIdx.z / g.ksplit;
+  const int kz = (int)blockIdx.z - (int)bz * g.ksplit;
   const double* __restrict__ A = g.A + bz * g.sA;
   const double* A2 = g.A2 ? g.A2 + bz * g.sA - g.mA1 : nullptr;
   const int mA1 = g.A2 ? g.mA1 : g.m;
@@ -64,8 +66,11 @@ __global__ void __launch_bounds__(128) gemm_fp64_kernel(GemmDesc g) {
   double* D2 = g.D2 ? g.D2 + bz * g.sD - g.mD1 : nullptr;
   const int mD1 = g.D2 ? g.mD1 : g.m;
 
-  __shared__ double As[TK][PAD];
-  __shared__ double Bs[TK][PAD];
+  // operand tiles, then (split K) this slice's sums, element (r, c) at [c * TM + r]
+  constexpr int SMEM = 2 * TK * PAD > TM * TM ? 2 * TK * PAD : TM * TM;
+  __shared__ double smem[SMEM];
+  double(*As)[PAD] = reinterpret_cast<double(*)[PAD]>(smem);
+  double(*Bs)[PAD] = reinterpret_cast<double(*)[PAD]>(smem + TK * PAD);
 
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
@@ -74,7 +79,7 @@ __global__ void __launch_bounds__(128) gemm_fp64_kernel(GemmDesc g) {
   if (splitk) {
     const int len = max(0, kr.khi - kr.klo);
     const int chunk = ((len + g.ksplit - 1) / g.ksplit + TK - 1) / TK * TK;
-    const int lo = kr.klo + (int)blockIdx.z * chunk;
+    const int lo = kr.klo + kz * chunk;
     kr.khi = min(kr.khi, lo + chunk);
     kr.klo = lo;
   }
@@ -149,19 +154,44 @@ __global__ void __launch_bounds__(128) gemm_fp64_kernel(GemmDesc g) {
   }
   pdl_trigger();
 
-  if (splitk) {  // raw partial sums of this K slice; reduced in fixed order later
-    double* W = g.ws + (long long)blockIdx.z * g.m * g.n;
+  if (splitk) {
+    // the slices' sums meet through distributed shared memory, in slice order;
+    // each CTA writes its share of the tile
 #pragma unroll
-    for (int i = 0; i < F; ++i) {
-      const int r = m0 + wm + i * 8 + (lane >> 2);
+    for (int i = 0; i < F; ++i)
 #pragma unroll
       for (int j = 0; j < F; ++j)
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int c = n0 + wn + j * 8 + (lane & 3) * 2 + e;
-          if (r < g.m && c < g.n) W[(long long)r + (long long)c * g.m] = acc[i][j][e];
-        }
+        for (int e = 0; e < 2; ++e)
+          smem[(wn + j * 8 + (lane & 3) * 2 + e) * TM + wm + i * 8 + (lane >> 2)] = acc[i][j][e];
+    cluster_sync();
+    const int share = (TM * TM / 128 + g.ksplit - 1) / g.ksplit;  // passes of 128 elements
+    constexpr int U = 4;                                          // passes in flight
+#pragma unroll 1
+    for (int q0 = 0; q0 < share; q0 += U) {
+      double v[U] = {};
+#pragma unroll 4
+      for (int z = 0; z < g.ksplit; ++z) {
+        double w[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          w[u] = ld_cluster(smem + min((kz * share + q0 + u) * 128 + tid, TM * TM - 1), z);
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] += w[u];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int idx = (kz * share + q0 + u) * 128 + tid;
+        const int r = m0 + idx % TM, c = n0 + idx / TM;
+        if (q0 + u >= share || idx >= TM * TM || r >= g.m || c >= g.n || (g.outLower && r < c) ||
+            (g.outUpper && r > c))
+          continue;
+        double x = g.alpha * v[u];
+        if (g.beta != 0.0) x += g.beta * (r < mD1 ? C : C2)[(long long)r + (long long)c * g.ldc];
+        (r < mD1 ? D : D2)[(long long)r + (long long)c * g.ldd] = x;
+      }
     }
+    cluster_sync();  // a CTA's sums are read until every CTA is here
     return;
   }
 #pragma unroll
@@ -444,20 +474,37 @@ __global__ void __launch_bounds__(128) gemm_thin_n_kernel(GemmDesc g, int kchunk
   if (nk > 1) cluster_sync();  // a CTA's sums are read until every CTA is here
 }
 
-// D = alpha * sum_s W_s + beta * C over the split-K partials, in slice order.
-__global__ void splitk_reduce_kernel(GemmDesc g) {
-  pdl_wait();
-  pdl_trigger();
-  const int r = blockIdx.x * 32 + threadIdx.x, c = blockIdx.y * 8 + threadIdx.y;
-  if (r >= g.m || c >= g.n || (g.outLower && r < c) || (g.outUpper && r > c)) return;
-  const long long mn = (long long)g.m * g.n, o = (long long)r + (long long)c * g.m;
-  double v = 0.0;
-  for (int s = 0; s < g.ksplit; ++s) v += g.ws[s * mn + o];
-  v *= g.alpha;
-  const bool hi = g.D2 && r >= g.mD1;
-  const long long ro = hi ? r - g.mD1 : r;
-  if (g.beta != 0.0) v += g.beta * (hi ? g.C2 : g.C)[ro + (long long)c * g.ldc];
-  (hi ? g.D2 : g.D)[ro + (long long)c * g.ldd] = v;
+// How many clusters of k CTAs the device holds with one CTA to an SM (asked of the
+// runtime once, for a CTA that takes most of an SM's shared memory).
+struct ClusterRoom {
+  int clusters[9];
+};
+const ClusterRoom& cluster_room() {
+  static const ClusterRoom room = [] {
+    ClusterRoom r{};
+    r.clusters[1] = 152;
+    auto* k = gemm_fp64_kernel<32, 8>;
+    constexpr int FILL = 160 << 10;
+    const bool ok =
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, FILL) == cudaSuccess;
+    for (int n = 2; n <= 8; ++n) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(1, 1, n);
+      cfg.blockDim = dim3(128);
+      cfg.dynamicSmemBytes = FILL;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = n;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      if (!ok || cudaOccupancyMaxActiveClusters(&r.clusters[n], k, &cfg) != cudaSuccess)
+        r.clusters[n] = 128 / n;
+    }
+    cudaGetLastError();
+    return r;
+  }();
+  return room;
 }
 
 // K over 1, 2, 4 or 8 CTAs of a cluster: `least` K terms per CTA are the
@@ -518,42 +565,52 @@ double gemm_flops(const GemmDesc& g) {
 int launch_gemm_fp64(const GemmDesc& g0, cudaStream_t s) {
   if (g0.m <= 0 || g0.n <= 0 || g0.batch <= 0) return 0;
   GemmDesc g = g0;
-  if (g.m <= 16 && g.transB && g.triA == TRI_NONE && g.batch == 1 && g.ws && !g.outLower && !g.outUpper &&
+  if (g.m <= 16 && g.transB && g.triA == TRI_NONE && g.batch == 1 && !g.outLower && !g.outUpper &&
       !g.A2) {
     launch_gemm_thin_m(g, s);
     return 1;
   }
-  if (g.n <= 16 && !g.transB && g.triB == TRI_NONE && g.batch == 1 && g.ws && !g.outLower && !g.outUpper &&
+  if (g.n <= 16 && !g.transB && g.triB == TRI_NONE && g.batch == 1 && !g.outLower && !g.outUpper &&
       !g.A2 && !g.D2) {
     launch_gemm_thin_n(g, s);
     return 1;
   }
-  // tiles of 64 when they (with split K) cover the SMs, else tiles of 32
-  const long long t64 = tiles_written(g, 64);
-  const bool small = g.tile == 32 || (g.tile != 64 && g.batch == 1 && g.ws &&
-                                       t64 * std::min(16, std::max(1, g.k / 16)) < 152);
-  const int tm = small ? 32 : 64, tk = small ? 8 : 16;
-  const long long tiles = small ? tiles_written(g, 32) : t64;
-  // too few output tiles for 152 SMs (each SM retires only ~3.5 FP64 flops
-  // per cycle, so one 64x64x64 tile is tens of microseconds): split K
+  // Output tile and split K (a cluster of up to 8 CTAs): the kernel is bound by
+  // the FP64 units, so a launch lasts as long as the SM with the most work:
+  // ceil(CTAs / 152) shares of tile^2 K / ksplit FMAs at 3200 a microsecond and
+  // SM, at least two where the tiles' clusters do not fit the chip one CTA to an
+  // SM; split K costs ~2 us.  32-wide tiles leave less of a last share empty than
+  // 64-wide ones and were never slower (FP64 factorize + RGFdiag at ns = 1000,
+  // nt = 10 81 against 115 ms, ns = 333, nt = 17 12.2 against 16.8).  Against the
+  // previous rule (up to 16 K slices of 64-wide tiles through a workspace and a
+  // second launch) the selected inversion at ns = 1000, nt = 10 went from 58.8 to
+  // 49.2 ms, at ns = 333, nt = 17 from 9.0 to 6.3.
+  const int tm = g.tile == 64 ? 64 : 32, tk = tm == 64 ? 16 : 8;
+  const double tiles = (double)tiles_written(g, tm) * g.batch;
+  const ClusterRoom& room = cluster_room();
   int ksplit = 1;
-  if (g.batch == 1 && g.ws && g.k >= 2 * tk) {
-    if (tiles > 0 && tiles < 2 * 152) {
-      ksplit = (int)std::min<long long>(16, (3 * 152 + tiles - 1) / tiles);
-      ksplit = std::min(ksplit, g.k / tk);
-      while (ksplit > 1 && (long long)ksplit * g.m * g.n > g.ws_elems) --ksplit;
+  double best = 1e300;
+  // beside the look-ahead stream's work the wide clusters of a product of many
+  // tiles wait for room (factorization at ns = 1000, nt = 10 31.9 ms with up to 8,
+  // 30.2 with up to 2); for few tiles the shorter launch still wins (ns = 333,
+  // nt = 17 6.0 against 6.4)
+  const int ks_max = g.beside && tiles > 76 ? 2 : 8;
+  for (int ks = 1; ks <= ks_max; ++ks) {
+    // a K step of the kernel a slice at least; nothing to gain past a few waves
+    if (ks > 1 && (g.k < tk * ks || tiles > 8 * 152 || (long long)ks * g.batch > 65535)) break;
+    double shares = std::ceil(tiles * ks / 152.0);
+    if (tiles > room.clusters[ks]) shares = std::max(shares, 2.0);
+    const double us = shares * tm * tm * ((double)g.k / ks) / 3200.0 + (ks > 1 ? 2.0 : 0.0);
+    if (us < best) {
+      best = us;
+      ksplit = ks;
     }
   }
   g.ksplit = ksplit;
   const int tx = (g.m + tm - 1) / tm, ty = (g.n + tm - 1) / tm;
-  dim3 grid(tx, ty, ksplit > 1 ? ksplit : g.batch);
-  if (small) launch_k(gemm_fp64_kernel<32, 8>, grid, dim3(128), 0, s, g);
-  else launch_k(gemm_fp64_kernel<64, 16>, grid, dim3(128), 0, s, g);
-  if (ksplit > 1) {
-    dim3 rg((g.m + 31) / 32, (g.n + 7) / 8);
-    launch_k(splitk_reduce_kernel, rg, dim3(32, 8), 0, s, g);
-    return 2;
-  }
+  const dim3 grid(tx, ty, ksplit * g.batch), cluster(1, 1, ksplit);
+  if (tm == 32) launch_k_cluster(gemm_fp64_kernel<32, 8>, grid, dim3(128), cluster, 0, s, g);
+  else launch_k_cluster(gemm_fp64_kernel<64, 16>, grid, dim3(128), cluster, 0, s, g);
   return 1;
 }
 

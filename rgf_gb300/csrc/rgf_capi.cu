@@ -83,9 +83,6 @@ struct rgf_handle {
   size_t ref_cap = 0;           // doubles
   double* d_panel_ws = nullptr;  // per tile of a diagonal block: launch_panel_tile's ws
   double* d_arrow = nullptr;     // partial sums of the corner update (launch_arrow_syrk)
-  double* d_gemm_ws = nullptr;  // split-K partial sums of small FP64 GEMMs
-  double* d_gemm_ws_side = nullptr;  // the same for the side stream
-  long long gemm_ws_elems = 0;
 
   bool factored = false;
   bool selinv_done = false;
@@ -117,7 +114,7 @@ struct rgf_handle {
   int nb = 32;               // leaf_nb knob (16, 32 or 64): see panel_width
   double split_bias = 1.0;   // the estimated split-product time is scaled by it
   int splitk_max = 0;        // tile shapes: split-K cap of the tensor-core products (0 = 8)
-  int fp64_tile = 0;         // and the FP64 output tile (0 = per product; split: 32)
+  int fp64_tile = 0;         // and the FP64 output tile (0 = 32)
   double tuned_ms = 0.0;     // factorize + RGFdiag time measured by the autotuner
   long long knob_gen = 0;
 
@@ -489,9 +486,8 @@ void gemm(rgf_handle* h, const GemmDesc& g, int cls) {
     launched = eng->gemm(g, cur_stream(h), h->d_status, &tflops, slices);
   } else {
     GemmDesc gw = g;
-    gw.ws = h->on_side ? h->d_gemm_ws_side : h->d_gemm_ws;
-    gw.ws_elems = h->gemm_ws_elems;
     gw.tile = h->fp64_tile;
+    gw.beside = h->side_used;
     const NoPdl beside(h->side_used);
     launched = launch_gemm_fp64(gw, cur_stream(h));
   }
@@ -1224,7 +1220,7 @@ void release(rgf_handle* h) {
   delete h->split_side;
   void* bufs[] = {h->d_ia, h->d_ja, h->d_a, h->d_MF, h->d_MS, h->d_U, h->d_T1, h->d_T2, h->d_T3,
                   h->d_logpart, h->d_scalars, h->d_diag, h->d_status, h->d_rhs, h->d_partial,
-                  h->d_res, h->d_gemm_ws, h->d_gemm_ws_side, h->d_ref, h->d_rhs2,
+                  h->d_res, h->d_ref, h->d_rhs2,
                   h->d_norms, h->d_panel_ws, h->d_arrow};
   for (void* p : bufs) dfree(p);
   if (h->ev_fork) cudaEventDestroy(h->ev_fork);
@@ -1324,11 +1320,7 @@ int rgf_create(const size_t* ia, const size_t* ja, const double* a, size_t ns, s
   if (!h) return RGF_ENOMEM;
   h->device = dev;
   h->opts = o;
-  // Split precision leaves the FP64 kernel the small, latency-bound products of
-  // the diagonal-block chain and the batched inverses, which run faster cut
-  // into 32 x 32 tiles (more CTAs) whatever their size: measured 3.5% on
-  // factorize + RGFdiag at ns = 2000.
-  if (o.precision == RGF_PREC_SPLIT) h->fp64_tile = 32;
+  if (o.precision == RGF_PREC_SPLIT) h->fp64_tile = 32;  // (the default tile, named)
   h->sh = {(long long)ns, (long long)nt, (long long)nd, n};
   h->nnz = (long long)ia[n];
   h->mf_size = 2 * (long long)(nt - 1) * ns * ns + (long long)ns * ns + n * (long long)nd;
@@ -1364,10 +1356,6 @@ int rgf_create(const size_t* ia, const size_t* ja, const double* a, size_t ns, s
     if (nd > 0 && nd <= ARROW_SYRK_MAX_ND &&
         (st = dalloc(h, &h->d_arrow, arrow_syrk_elems(h->sh))))
       break;
-    h->gemm_ws_elems = std::min<long long>(20ll << 20, 8ll * (2 * (long long)ns + (long long)nd) *
-                                                           std::max<long long>(ns, nd));
-    if ((st = dalloc(h, &h->d_gemm_ws, h->gemm_ws_elems))) break;
-    if ((st = dalloc(h, &h->d_gemm_ws_side, h->gemm_ws_elems))) break;
     // the CSC goes up in two halves on the two streams, so that two copy
     // engines move it at once; the main stream joins before anything reads it
     // (asynchronous upload: below, in block-column chunks)
@@ -2108,7 +2096,7 @@ int tune_handle(rgf_handle* h, rgf_tuning* out) {
       if ((st = trial(t))) return st;
     }
   }
-  for (int tile : {0, 32, 64}) {  // and the FP64 products' output tile
+  for (int tile : {32, 64}) {  // and the FP64 products' output tile (0 cuts like 32)
     rgf_tuning t = best;
     t.fp64_tile = tile;
     if ((st = trial(t))) return st;

@@ -106,12 +106,8 @@ struct GemmDesc {
   int triA = TRI_NONE, triB = TRI_NONE, outLower = 0, outUpper = 0;
   int batch = 1;
   long long sA = 0, sB = 0, sC = 0, sD = 0;
-  // FP64 kernel only: workspace for split-K partial sums (used when a single
-  // problem has too few output tiles to fill the GPU); ksplit is set by the
-  // launcher.
-  double* ws = nullptr;
-  long long ws_elems = 0;
-  int ksplit = 1;
+  int ksplit = 1;       // FP64 kernel: set by the launcher
+  bool beside = false;  // FP64 kernel: other work shares the GPU
   int tile = 0;  // FP64 kernel: output tile 32 or 64; 0 = chosen by the launcher
 };
 
@@ -142,7 +138,7 @@ int hermitian_embed(const size_t* ia, const size_t* ja, const double* a, size_t 
 size_t hermitian_real_index(size_t ns, size_t nt, size_t nd, size_t k, int imag);
 
 // ---- FP64 kernels (k_fp64.cu) ---------------------------------------------
-// Returns the number of kernels launched (2 with split-K).
+// Returns the number of kernels launched.
 int launch_gemm_fp64(const GemmDesc& g, cudaStream_t s);
 
 // ---- panel factorization (k_panel.cu) -------------------------------------------
