@@ -141,36 +141,41 @@ __global__ void set_identity_kernel(double* X, long long ld, int m, long long st
   if (r < m && c < m) X[r + (long long)c * ld] = (r == c) ? 1.0 : 0.0;
 }
 
-__global__ void copy_kernel(const double* X, long long ldx, double* Y, long long ldy, int m,
-                            int n, long long sX, long long sY) {
-  pdl_wait();
-  pdl_trigger();
-  X += (long long)blockIdx.z * sX;
-  Y += (long long)blockIdx.z * sY;
-  const int r = blockIdx.x * 32 + threadIdx.x, c = blockIdx.y * 8 + threadIdx.y;
-  if (r < m && c < n) Y[r + (long long)c * ldy] = X[r + (long long)c * ldx];
-}
-
-// X(r, c) = X(c, r) for r < c: the strictly upper triangle of the n x n
-// matrix X (column-major, ld) from its lower one.  The CTA of source tile
-// (bi, bj), bi >= bj, reads that 32 x 32 lower tile along its columns into
-// shared memory and writes it transposed along the columns of tile (bj, bi);
-// no CTA reads a tile another one writes.
-__global__ void mirror_lower_kernel(double* X, long long ld, int n) {
+// X(r, c) = X(c, r) for r < c: the strictly upper triangle of the n x n matrix X
+// (column-major, ld) from its lower one, and with S the full symmetric
+// [X, Xd^T; Xd, Sdd] into S (packed; nd = 0: X alone).  Tiles of 32: nb of the rows
+// of X, then those of the nd arrowhead rows.  The CTA of source tile (bi, bj),
+// bi >= bj, reads it along its columns into shared memory and writes it transposed
+// along the columns of tile (bj, bi); no CTA reads a tile another one writes.
+__global__ void mirror_sigma_kernel(double* X, long long ld, int n, const double* Xd,
+                                    const double* Sdd, int nd, double* S, int nb) {
   __shared__ double t[32][33];  // t[column offset][row offset] of the source tile
   pdl_wait();
   pdl_trigger();
   const int bi = blockIdx.x, bj = blockIdx.y;
   if (bi < bj) return;
   const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
+  const bool dr = bi >= nb, dc = bj >= nb;       // arrowhead rows, columns
+  const int r0 = (dr ? bi - nb : bi) * 32, c0 = (dc ? bj - nb : bj) * 32;
+  const int nr = dr ? nd : n, nc = dc ? nd : n;
+  const double* src = dc ? Sdd : dr ? Xd : X;
+  const long long lds = dc ? nd : ld;
+  const long long m2 = n + nd;
+  const int fr = dr ? n : 0, fc = dc ? n : 0;  // where the tile's rows, columns start in S
   for (int k = ty; k < 32; k += 8) {
-    const int r = bi * 32 + tx, c = bj * 32 + k;
-    if (r < n && c < n) t[k][tx] = X[r + (long long)c * ld];
+    const int r = r0 + tx, c = c0 + k;
+    if (r < nr && c < nc && (dr != dc || r >= c)) {
+      const double v = src[r + (long long)c * lds];
+      t[k][tx] = v;
+      if (S) S[fr + r + (fc + c) * m2] = v;
+    }
   }
   __syncthreads();
   for (int k = ty; k < 32; k += 8) {
-    const int r = bj * 32 + tx, c = bi * 32 + k;  // X(r, c) = X(c, r) = t[tx][k]
-    if (r < c && c < n) X[r + (long long)c * ld] = t[tx][k];
+    const int r = c0 + tx, c = r0 + k;  // the transposed element (r, c) = t[tx][k]
+    if (r >= nc || c >= nr || (dr == dc && r >= c)) continue;
+    if (!dr) X[r + (long long)c * ld] = t[tx][k];
+    if (S) S[fc + r + (fr + c) * m2] = t[tx][k];
   }
 }
 
@@ -411,6 +416,11 @@ void launch_logdet(const BtaShape& sh, const double* MF, double* parts, double* 
   launch_k(logdet_reduce_kernel, dim3(1), dim3(32), 0, s, parts, np, out);
 }
 
+long long selinv_chunk(const BtaShape& sh) {
+  const long long one = (long long)sizeof(double) * (sh.ns + sh.nd) * sh.ns;
+  return std::max(1LL, std::min(sh.nt - 1, (long long)K_CHUNK_BYTES / one));
+}
+
 void launch_extract_diag(const BtaShape& sh, const double* MS, double* diag, cudaStream_t s) {
   launch_k(extract_diag_kernel, dim3((unsigned)((sh.n + 255) / 256)), dim3(256), 0, s, sh, MS,
            diag);
@@ -423,17 +433,14 @@ void launch_set_identity(double* X, long long ld, int m, int batch, long long st
   launch_k(set_identity_kernel, grid, dim3(32, 8), 0, s, X, ld, m, stride);
 }
 
-void launch_mirror_lower(double* X, long long ld, int n, cudaStream_t s) {
-  if (n <= 1) return;
-  const unsigned nb = (unsigned)((n + 31) / 32);
-  launch_k(mirror_lower_kernel, dim3(nb, nb), dim3(32, 8), 0, s, X, ld, n);
-}
-
-void launch_copy(const double* X, long long ldx, double* Y, long long ldy, int m, int n,
-                 int batch, long long sX, long long sY, cudaStream_t s) {
-  if (m <= 0 || n <= 0 || batch <= 0) return;
-  dim3 grid((m + 31) / 32, (n + 7) / 8, batch);
-  launch_k(copy_kernel, grid, dim3(32, 8), 0, s, X, ldx, Y, ldy, m, n, sX, sY);
+void launch_mirror_sigma(double* X, long long ld, int n, const double* Xd, const double* Sdd,
+                         int nd, double* S, cudaStream_t s) {
+  if (!S) {
+    nd = 0;
+    if (n <= 1) return;
+  }
+  const unsigned nb = (unsigned)((n + 31) / 32), all = nb + (unsigned)((nd + 31) / 32);
+  launch_k(mirror_sigma_kernel, dim3(all, all), dim3(32, 8), 0, s, X, ld, n, Xd, Sdd, nd, S, (int)nb);
 }
 
 // r = b - y; x += d (element-wise over len entries)

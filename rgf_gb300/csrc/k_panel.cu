@@ -201,7 +201,9 @@ __device__ __forceinline__ void bar_sync_leaf() {
 }
 
 // S(r, c) -= sum_{j < 16} V_rj l_cj over the lower elements 16 <= c <= r < 32 of the
-// second half (136 of them): two neighbouring threads share an element's 16
+// second half (136 of them; the terms are summed before they meet S, here and in
+// all updates between leaves, so that S's size rounds once a leaf and not once a
+// column: at ns = 128 that is 1.4 times less error in the factor): two neighbouring threads share an element's 16
 // terms, and the last eight elements go to one warp, four threads each
 __device__ __forceinline__ void leaf_trailing(double (*S)[LB], const double (*V)[LB],
                                               const double (*Lc)[LB]) {
@@ -215,20 +217,20 @@ __device__ __forceinline__ void leaf_trailing(double (*S)[LB], const double (*V)
   int r, c;
   element(t >> 1, r, c);
   int j0 = (t & 1) * (H / 2);
-  double s = (t & 1) == 0 ? S[c][r] : 0.0;
+  double s = 0.0;
 #pragma unroll
-  for (int j = 0; j < H / 2; ++j) s = fma(-V[j0 + j][r], Lc[j0 + j][c], s);
+  for (int j = 0; j < H / 2; ++j) s = fma(V[j0 + j][r], Lc[j0 + j][c], s);
   s += __shfl_xor_sync(0xffffffffu, s, 1);
-  if ((t & 1) == 0) S[c][r] = s;
+  if ((t & 1) == 0) S[c][r] -= s;
   if (t >= LEAF_WARPS * 32 - 32) {
     element(LEAF_WARPS * 16 + ((t & 31) >> 2), r, c);
     j0 = (t & 3) * (H / 4);
-    s = (t & 3) == 0 ? S[c][r] : 0.0;
+    s = 0.0;
 #pragma unroll
-    for (int j = 0; j < H / 4; ++j) s = fma(-V[j0 + j][r], Lc[j0 + j][c], s);
+    for (int j = 0; j < H / 4; ++j) s = fma(V[j0 + j][r], Lc[j0 + j][c], s);
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     s += __shfl_xor_sync(0xffffffffu, s, 2);
-    if ((t & 3) == 0) S[c][r] = s;
+    if ((t & 3) == 0) S[c][r] -= s;
   }
 }
 
@@ -476,14 +478,15 @@ __global__ void __launch_bounds__(TILE_THREADS, 5)
       const bool live = i < nown && r < kn + LB;  // element (r, kn + e)
       if (__any_sync(0xffffffffu, live)) {
         const int l0 = (tid % KS) * (LB / KS);
-        double s = live && l0 == 0 ? own(i)[kn + e] : 0.0;
+        double s = 0.0;
         const double* xr = Xn[live ? r - kn : 0] + l0;
         const double* xc = Xn[live ? e : 0] + l0;
 #pragma unroll
-        for (int l = 0; l < LB / KS; ++l) s = fma(-xr[l], xc[l], s);
+        for (int l = 0; l < LB / KS; ++l) s = fma(xr[l], xc[l], s);
 #pragma unroll
         for (int o = 1; o < KS; o *= 2) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (live && l0 == 0) st_cluster(cluster_addr(bufA + e * LB + (r - kn), 0), s);
+        if (live && l0 == 0)
+          st_cluster(cluster_addr(bufA + e * LB + (r - kn), 0), own(i)[kn + e] - s);
       }
     }
     __syncthreads();
@@ -499,7 +502,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 5)
           const bool live = c <= r;
           const double* xc = P + (live ? c : r) + (long long)kc * lda;
           const double* xr = own(i) + kc;
-          double s = live ? own(i)[c] : 0.0;
+          double s = 0.0;
 #pragma unroll 1
           for (int l0 = 0; l0 < LB; l0 += 8) {
             double b[8];
@@ -509,9 +512,9 @@ __global__ void __launch_bounds__(TILE_THREADS, 5)
               xc += lda;
             }
 #pragma unroll
-            for (int l = 0; l < 8; ++l) s = fma(-xr[l0 + l], b[l], s);
+            for (int l = 0; l < 8; ++l) s = fma(xr[l0 + l], b[l], s);
           }
-          if (live) own(i)[c] = s;
+          if (live) own(i)[c] -= s;
         }
       }
     }
@@ -590,17 +593,22 @@ __global__ void __launch_bounds__(NT)
       cp_async_wait<0>();
       __syncthreads();
       fetch_leaf(k + 1);
+      double sum[NB * SB];  // of this block's terms, before they meet u
+#pragma unroll
+      for (int s = (k + 1) * SB; s < NB * SB; ++s) sum[s] = 0.0;
 #pragma unroll
       for (int t = 0; t < SB; ++t) {
 #pragma unroll 1
         for (int jj = 0; jj < G; ++jj) {
-          const double x = -__shfl_sync(0xffffffffu, u[k * SB + t], gbase | jj);
+          const double x = __shfl_sync(0xffffffffu, u[k * SB + t], gbase | jj);
           const double* xr = &Xs[t * G + jj][q];
 #pragma unroll
           for (int s = (k + 1) * SB; s < NB * SB; ++s)
-            u[s] = fma(x, xr[s * G - kn], u[s]);
+            sum[s] = fma(x, xr[s * G - kn], sum[s]);
         }
       }
+#pragma unroll
+      for (int s = (k + 1) * SB; s < NB * SB; ++s) u[s] -= sum[s];
       __syncthreads();  // Xs is overwritten next
     }
   }

@@ -962,6 +962,10 @@ constexpr size_t SMEM_BYTES = 1024 + 3 * NSTAGE * TILE_BYTES + 256;
 
 int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
+int transposed(int tri) {
+  return tri == TRI_LOWER ? TRI_UPPER : tri == TRI_UPPER ? TRI_LOWER : TRI_NONE;
+}
+
 }  // namespace
 
 SplitEngine* SplitEngine::create(int slices, int* status) {
@@ -976,7 +980,8 @@ SplitEngine* SplitEngine::create(int slices, int* status) {
     *status = RGF_ENOTSUP;
     return nullptr;
   }
-  for (auto* k : {slice_pair_kernel<16, 0>, slice_pair_kernel<16, 5>, slice_pair_kernel<16, 7>})
+  for (auto* k : {slice_pair_kernel<16, 0>, slice_pair_kernel<16, 5>, slice_pair_kernel<16, 6>,
+                  slice_pair_kernel<16, 7>})
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(32 * (SLICE_MAX_KC + 1) * sizeof(double))) != cudaSuccess) {
       cudaGetLastError();
@@ -1144,12 +1149,40 @@ double SplitEngine::estimate_seconds(const GemmDesc& g, int slices) const {
   }
   const long long ksplit = split_k(tiles, jobs);
   const double waves = std::ceil((double)(tiles * ksplit) / num_sms_);
-  const bool same = g.A == g.B && g.lda == g.ldb && g.transA != g.transB;
+  const bool same = g.A == g.B && g.lda == g.ldb && g.transA != g.transB &&
+                    g.triA == transposed(g.triB);
   const double t_slice = (Kp <= SLICE_MAX_K ? 5.5e-6 : 16e-6) +
                          (g.m + (same ? 0.0 : g.n)) * (double)Kp * (8.0 + 2.0 * S) * g.batch / 3e12;
   const double steps = (double)plan.slots.size() * (Kp / 16.0) / ksplit;
   const double t_end = 12e-6 / ksplit + (ksplit > 1 ? 3e-6 : 0.0);
   return 12e-6 + t_slice + waves * (steps * 90e-9 + t_end);
+}
+
+// Which bulk products may run at the engine's slice count is part of the results'
+// accuracy (5 slices keep ~40 bits of an operand), so the line stays where it has
+// always been, at this estimate of the time of one product (not of a batch) with split
+// K over a workspace, and does not follow the kernels' speed.
+bool SplitEngine::may_slice(const GemmDesc& g, double bias) const {
+  const int tx = round_up(g.m, BM) / BM, ty = round_up(g.n, BN) / BN;
+  const int Kp = round_up(g.k, BKE);
+  long long tiles = 0;
+  for (int x = 0; x < tx; ++x)
+    for (int y = 0; y < ty; ++y) tiles += !(g.outLower && x * BM + BM <= y * BN);
+  const SlotPlan& plan = slot_plan(slices_);
+  long long jobs = 0;
+  for (const SlotGroup& gr : plan.groups) {
+    const int chunk = std::max(1, EXACT_TERMS / (SBK * gr.count));
+    jobs += (Kp / SBK + chunk - 1) / chunk;
+  }
+  long long ksplit = 1;
+  if (tiles * 2 <= num_sms_ && tx * ty <= 80)
+    ksplit = std::max(1LL, std::min({16LL, jobs, num_sms_ / std::max(1LL, tiles)}));
+  const bool same = g.A == g.B && g.lda == g.ldb && g.transA != g.transB && g.triA == TRI_NONE;
+  const double t_slice = (Kp <= 512 ? 8e-6 : 16e-6) +
+                         (g.m + (same ? 0.0 : g.n)) * (double)Kp * (8.0 + 2.0 * slices_) / 3e12;
+  const double steps = (double)plan.slots.size() * (Kp / 16.0) / ksplit;
+  const double t = 20e-6 + t_slice + std::ceil((double)(tiles * ksplit) / num_sms_) * steps * 120e-9;
+  return t * bias < 9e-6 + gemm_flops(g) / g.batch / 0.9e12;
 }
 
 // Tensor maps are encoded once per (base, planes, rows, K) and reused: the
@@ -1209,10 +1242,10 @@ long long SplitEngine::gemm(const GemmDesc& g, cudaStream_t s, DevStatus* st,
   const int S = slices > 0 ? std::min(slices, MAX_SLICES) : slices_, beta = SPLIT_BETA;
   const int Kp = round_up(g.k, BKE);
   const int RpA = round_up(g.m, BM), RpB = round_up(g.n, BM);
-  // op(B)^T is op(A) or its first n rows: the slices (and exponents) of A serve both
+  // op(B)^T is op(A) or its first n rows (and triangular alike): the slices (and
+  // exponents) of A serve both
   const bool same = g.A == g.B && g.lda == g.ldb && g.sA == g.sB && g.transA != g.transB &&
-                    g.n <= g.m && (!g.A2 || g.n <= g.mA1) && g.triA == TRI_NONE &&
-                    g.triB == TRI_NONE;
+                    g.n <= g.m && (!g.A2 || g.n <= g.mA1) && g.triA == transposed(g.triB);
   const size_t per_item = item_bytes(S, RpA, same ? 0 : RpB, Kp);
   const int chunk = (int)std::max<size_t>(1, std::min<size_t>(g.batch, ws_bytes_ / per_item));
   SplitParams p;
@@ -1245,7 +1278,7 @@ long long SplitEngine::gemm(const GemmDesc& g, cudaStream_t s, DevStatus* st,
   p.alpha = g.alpha; p.betac = g.beta;
   p.st = st;
   p.exA_stride = RpA; p.exB_stride = same ? RpA : RpB;
-  const int triBt = g.triB == TRI_LOWER ? TRI_UPPER : g.triB == TRI_UPPER ? TRI_LOWER : TRI_NONE;
+  const int triBt = transposed(g.triB);
   long long launched = 0;
   uint8_t* base = static_cast<uint8_t*>(ws_);
   for (int b0 = 0; b0 < g.batch; b0 += chunk) {
@@ -1296,9 +1329,11 @@ long long SplitEngine::gemm(const GemmDesc& g, cudaStream_t s, DevStatus* st,
       // shared memory, three to an SM, and needs the threads to move them
       static_assert(SPLIT_BETA == 8, "write_digit_pair");
       auto* kern = kc <= 128 ? (S == 5   ? slice_pair_kernel<8, 5>
+                                : S == 6 ? slice_pair_kernel<8, 6>
                                 : S == 7 ? slice_pair_kernel<8, 7>
                                          : slice_pair_kernel<8, 0>)
                              : (S == 5   ? slice_pair_kernel<16, 5>
+                                : S == 6 ? slice_pair_kernel<16, 6>
                                 : S == 7 ? slice_pair_kernel<16, 7>
                                          : slice_pair_kernel<16, 0>);
       launch_k_cluster(kern, dim3(nblkA + nblkB, nk, nbat), dim3(kc <= 128 ? 256 : 512),

@@ -64,8 +64,11 @@ struct rgf_handle {
   double* d_MF = nullptr;
   double* d_MS = nullptr;
   double* d_U = nullptr;     // Linv^T of every diagonal block (ns x ns each), then the corner
-  double* d_T1 = nullptr;    // (ns + nd) x ns
-  double* d_T2 = nullptr;    // ns x ns
+  double* d_T1 = nullptr;    // ns x ns (compat recursion)
+  double* d_T2 = nullptr;    // ns x ns (compat recursion)
+  double* d_K = nullptr;     // k_chunk blocks of (ns + nd) x ns
+  double* d_S = nullptr;     // (ns + nd) x (ns + nd)
+  long long k_chunk = 0;     // blocks whose K_i is formed at once
   double* d_T3 = nullptr;    // nd x ns
   double* d_logpart = nullptr;
   int nparts = 0;
@@ -398,7 +401,10 @@ void dfree(void* p) { device_free(p); }
 // GEMM classes: SMALL always runs in FP64; BULK may run as split products;
 // DIAG (updates inside a diagonal block's Cholesky or inverse) runs split
 // only when the handle does not keep diagonal blocks in FP64.
-enum GemmClass { SMALL = 0, BULK = 1, DIAG = 2 };
+// BULK1: as BULK, one slice more (U U^T, whose operands' truncations are the same and
+// so add up instead of averaging out: 1.4 times the error of a product of two
+// different operands at equal slices).
+enum GemmClass { SMALL = 0, BULK = 1, DIAG = 2, BULK1 = 3 };
 
 cudaStream_t cur_stream(const rgf_handle* h) { return h->on_side ? h->side : h->stream; }
 
@@ -442,15 +448,46 @@ void trace_flush(rgf_handle* h) {
   h->trace_stage++;
 }
 
+// Digit slices for g on the split engine, 0 = FP64 only.  Where the engine's own slice
+// count is not allowed for a triangular or lower-only product but would be for a full one
+// of its size (SplitEngine::may_slice), blocks of that size already carry sliced
+// products, and it may take 7: 56-bit operands, FP64-accurate emulation (ns = 256,
+// nt = 30: selected inversion 3.6 -> 2.1 ms).  Below that line everything is FP64.
+// fp64_diag: 0 = diagonal blocks at the bulk slice count, 1 = at 7 slices, 2 = native
+// FP64 DMMA.
+int class_slices(const rgf_handle* h, const SplitEngine* eng, const GemmDesc& g, int cls) {
+  constexpr int EXACT = 7;
+  const int fd = h->opts.fp64_diag, S = eng->slices();
+  if (cls == SMALL || (cls == DIAG && fd == 2)) return 0;
+  if (cls == DIAG && fd == 1) return EXACT;
+  const int own = cls == BULK1 ? std::min(S + 1, 8) : S;
+  if (eng->may_slice(g, h->split_bias)) return own;
+  GemmDesc full = g;
+  full.triA = full.triB = TRI_NONE;
+  full.outLower = full.outUpper = 0;
+  return fd == 1 && S <= EXACT && eng->may_slice(full, h->split_bias) ? EXACT : 0;
+}
+
+// Whether g runs on the split engine: by estimated time, the engine's estimate (its
+// launches, slicing, MMA streams and split K) against the FP64 DMMA kernel at
+// ~9 us of launches and ~0.9 TFLOP/s.  Small or thin products are faster in FP64
+// (which is also FP64-accurate).
+// Returns the slice count, 0 = FP64.
+int routed_slices(const rgf_handle* h, const GemmDesc& g, int cls) {
+  const SplitEngine* eng = h->on_side ? h->split_side : h->split;
+  if (!eng || !eng->supports(g)) return 0;
+  const int slices = class_slices(h, eng, g, cls);
+  if (!slices) return 0;
+  // (half of that beside the look-ahead stream's row solves, which use the
+  // same FP64 units)
+  const double t_fp64 = 9e-6 + gemm_flops(g) / (h->side_used && cls == DIAG ? 0.45e12 : 0.9e12);
+  return eng->estimate_seconds(g, slices) * h->split_bias < t_fp64 ? slices : 0;
+}
+
 void gemm(rgf_handle* h, const GemmDesc& g, int cls) {
   if (g.m <= 0 || g.n <= 0 || g.batch <= 0) return;
   const NoPdl scope(h->on_side);
   const bool bulk = cls != SMALL;
-  // fp64_diag: 0 = diagonal blocks at the bulk slice count, 1 = at 7 slices
-  // (56-bit operands: FP64-accurate emulation), 2 = native FP64 DMMA
-  const int fd = h->opts.fp64_diag;
-  const bool may_split = cls == BULK || (cls == DIAG && fd != 2);
-  const int slices = (cls == DIAG && fd == 1) ? 7 : 0;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (h->timer_on && bulk) {
     if (h->ev_pool.empty()) {
@@ -470,18 +507,8 @@ void gemm(rgf_handle* h, const GemmDesc& g, int cls) {
   long long launched = 1;
   double tflops = 0.0;
   SplitEngine* eng = h->on_side ? h->split_side : h->split;
-  bool split = eng && may_split && eng->supports(g);
-  if (split) {
-    // Route by estimated time: the split engine's estimate (its launches,
-    // slicing, MMA streams and split K) against the FP64 DMMA kernel at
-    // ~9 us of launches and ~0.9 TFLOP/s.  Small or thin products are faster
-    // in FP64 (which is also FP64-accurate).
-    const double t_split = eng->estimate_seconds(g, slices);
-    // (half of that beside the look-ahead stream's row solves, which use the
-    // same FP64 units)
-    const double t_fp64 = 9e-6 + gemm_flops(g) / (h->side_used && cls == DIAG ? 0.45e12 : 0.9e12);
-    split = t_split * h->split_bias < t_fp64;
-  }
+  const int slices = routed_slices(h, g, cls);
+  const bool split = slices > 0;
   if (split) {
     launched = eng->gemm(g, cur_stream(h), h->d_status, &tflops, slices);
   } else {
@@ -745,15 +772,12 @@ GemmDesc mk(int m, int n, int k, const double* A, long long lda, int tA, const d
 
 // U_i = L_ii^{-T} of every diagonal block and of the corner, as one batched
 // recursive TRTRI (the blocks are independent once the factor exists); MS is
-// the recursion's scratch.
+// the recursion's scratch.  Only the upper triangles are written: every product
+// declares U triangular.
 void issue_inverses(rgf_handle* h) {
   const BtaShape& sh = h->sh;
   const long long ns = sh.ns, nt = sh.nt, nd = sh.nd;
   const long long ss = ns * ns;
-  // The inverses are upper triangular and are read as full blocks
-  // (W^T = U_i - ...); the recursion writes only their upper part, so the
-  // strictly lower part must be zero.
-  cudaMemsetAsync(h->d_U, 0, sizeof(double) * (nt * ss + nd * nd), h->stream);
   // The last block (another leading dimension) and the corner go to the side
   // stream, beside the batch of the others: their recursions are chains of small
   // launches (selected inversion at ns = 2000, nt = 10 14.3 -> 11.9 ms, half of it
@@ -790,6 +814,39 @@ void issue_selinv(rgf_handle* h) {
     gemm(h, mk(ind, ind, ind, Ud, nd, 0, Ud, nd, 1, nullptr, 0, Sdd, nd, 1.0, 0.0), SMALL);
   }
   const bool compat = h->opts.selinv_mode == RGF_SELINV_COMPAT;
+  const int m2 = ins + ind;
+  const long long sP = ns * (2 * ns + nd);  // one block column of MF and MS
+  long long k_lo = nt - 1;                  // blocks [k_lo, ...) have their K in d_K
+  // G_i = -[Sigma_{i+1,i+1}; Sigma_{d,i+1}] K_B (+ what G_i holds)
+  auto g_split = [&](long long i, const double* K, double beta) {
+    double* G = h->d_MS + mf_col_offset(sh, i) + ns;
+    const double* Sn = h->d_MS + mf_col_offset(sh, i + 1);
+    const long long ldn = mf_lda(sh, i + 1), ldg = 2 * ns + nd;
+    GemmDesc g = mk(m2, ins, ins, Sn, ldn, 0, K, m2, 0, G, ldg, G, ldg, -1.0, beta);
+    if (nd > 0) {
+      g.A2 = Sn + mf_dense_row(sh, i + 1);
+      g.mA1 = ins;
+    }
+    return g;
+  };
+  // G's route: an FP64 product reads the full symmetric S; a sliced one reads
+  // Sigma_{i+1,i+1} and Sigma_{d,i+1} where they are
+  const bool dense = nt < 2 || !routed_slices(h, g_split(0, h->d_K, 0.0), BULK);
+  if (!compat) {
+    // Q_ii = U_i U_i^T of every block (lower part), the constant term of Sigma_ii
+    GemmDesc u = mk(ins, ins, ins, h->d_U, ns, 0, h->d_U, ns, 1, nullptr, 0, h->d_MS, 2 * ns + nd,
+                    1.0, 0.0);
+    u.triA = TRI_UPPER;
+    u.triB = TRI_LOWER;
+    u.outLower = 1;
+    u.batch = (int)(nt - 1); u.sA = u.sB = ss; u.sD = sP;
+    gemm(h, u, BULK1);
+    u.batch = 1;
+    u.A = u.B = h->d_U + (nt - 1) * ss;
+    u.D = h->d_MS + mf_col_offset(sh, nt - 1);
+    u.ldd = ns + nd;
+    gemm(h, u, BULK1);
+  }
   for (long long i = nt - 1; i >= 0; --i) {
     const double* P = h->d_MF + mf_col_offset(sh, i);
     double* Q = h->d_MS + mf_col_offset(sh, i);
@@ -800,70 +857,69 @@ void issue_selinv(rgf_handle* h) {
     const bool has_next = i < nt - 1;
     const double* Sn = has_next ? h->d_MS + mf_col_offset(sh, i + 1) : nullptr;  // Sigma_{i+1,i+1}
     const long long ldn = has_next ? mf_lda(sh, i + 1) : 0;
-    const double* Sdn = has_next ? Sn + mf_dense_row(sh, i + 1) : nullptr;       // Sigma_{d,i+1}
     if (!compat) {
-      // Rows below the diagonal block are [L_{i+1,i}; C_i] = P + ns and
-      // [Sigma_{i+1,i}; Sigma_{d,i}] = Q + ns (adjacent), so the products that
-      // produce or consume them run once over ns + nd rows instead of as a
-      // square product plus a thin nd-row one.
-      if (has_next) {
-        const int m2 = ins + ind;
-        const long long ldt = m2;
-        // [X; Y] = [Sigma_{i+1,i+1}; Sigma_{d,i+1}] L_{i+1,i}
-        //          + [Sigma_{d,i+1}^T C_i; Sigma_dd C_i]
-        GemmDesc x = mk(m2, ins, ins, Sn, ldn, 0, Bi, lda, 0, nullptr, 0, h->d_T1, ldt, 1.0, 0.0);
+      // With K_i = [L_{i+1,i}; C_i] L_ii^{-1} and S the symmetric
+      // [Sigma_{i+1,i+1}, .; Sigma_{d,i+1}, Sigma_dd]:
+      //   G_i = [Sigma_{i+1,i}; Sigma_{d,i}] = -S K_i
+      //   Sigma_ii = U_i U_i^T - K_i^T G_i
+      // Only these two products wait for the block before them; K_i and U_i U_i^T
+      // depend on the factor alone, so they run as batches over many blocks, which
+      // fill the GPU where a single block's product does not.
+      const double* K = h->d_T3;
+      if (!has_next) {
         if (nd > 0) {
-          x.A2 = Sdn;
-          x.mA1 = ins;
+          GemmDesc k = mk(ind, ins, ins, Ci, lda, 0, Ui, ns, 1, nullptr, 0, h->d_T3, nd, 1.0, 0.0);
+          k.triB = TRI_LOWER;
+          gemm(h, k, BULK);
+          gemm(h, mk(ind, ins, ind, Sdd, nd, 0, h->d_T3, nd, 0, nullptr, 0,
+                     Q + mf_dense_row(sh, i), lda, -1.0, 0.0), SMALL);
         }
-        gemm(h, x, BULK);
-        if (nd > 0) {
-          gemm(h, mk(ins, ins, ind, Sdn, ldn, 1, Ci, lda, 0, h->d_T1, ldt, h->d_T1, ldt, 1.0, 1.0),
-               SMALL);
-          gemm(h, mk(ind, ins, ind, Sdd, nd, 0, Ci, lda, 0, h->d_T1 + ns, ldt, h->d_T1 + ns, ldt,
-                     1.0, 1.0), SMALL);
-        }
-        // [Sigma_{i+1,i}; Sigma_{d,i}] = -[X; Y] L_ii^{-1} = -[X; Y] U_i^T
-        GemmDesc g = mk(m2, ins, ins, h->d_T1, ldt, 0, Ui, ns, 1, nullptr, 0, Q + ns, lda, -1.0, 0.0);
-        g.triB = TRI_LOWER;
-        gemm(h, g, BULK);
-        // W^T = U_i - [Sigma_{i+1,i}; Sigma_{d,i}]^T [L_{i+1,i}; C_i], upper triangle
-        // (see Sigma_ii below)
-        GemmDesc w = mk(ins, ins, m2, Q + ns, lda, 1, Bi, lda, 0, Ui, ns, h->d_T2, ns, -1.0, 1.0);
-        w.outUpper = 1;
-        gemm(h, w, BULK);
       } else {
-        if (nd > 0) {
-          // Y = Sigma_dd C_i;  Sigma_{d,i} = -Y U_i^T
-          gemm(h, mk(ind, ins, ind, Sdd, nd, 0, Ci, lda, 0, nullptr, 0, h->d_T3, nd, 1.0, 0.0),
-               SMALL);
-          GemmDesc g = mk(ind, ins, ins, h->d_T3, nd, 0, Ui, ns, 1, nullptr, 0,
-                          Q + mf_dense_row(sh, i), lda, -1.0, 0.0);
-          g.triB = TRI_LOWER;
-          gemm(h, g, BULK);
-          // W^T = U_i - Sigma_{d,i}^T C_i, upper triangle
-          GemmDesc w = mk(ins, ins, ind, Q + mf_dense_row(sh, i), lda, 1, Ci, lda, 0, Ui, ns,
-                          h->d_T2, ns, -1.0, 1.0);
-          w.outUpper = 1;
-          gemm(h, w, SMALL);
+        K = h->d_K + (i - k_lo) * ns * m2;
+        if (dense) {
+          gemm(h, mk(m2, ins, m2, h->d_S, m2, 0, K, m2, 0, nullptr, 0, Q + ns, lda, -1.0, 0.0),
+               BULK);
         } else {
-          launch_copy(Ui, ns, h->d_T2, ns, ins, ins, 1, 0, 0, s);
-          h->kernels_issued++;
+          if (nd > 0) join_side(h);  // -[Sigma_{d,i+1}^T; Sigma_dd] K_C is in place
+          gemm(h, g_split(i, K, nd > 0 ? 1.0 : 0.0), BULK);
         }
       }
-      // Sigma_ii = L_ii^{-T} W = U_i (W^T)^T, symmetric: only its lower
-      // triangle is computed (the output tiles above the diagonal, nearly
-      // half, are skipped), then mirrored.  For r >= c its terms U(r, k) W(k, c)
-      // are non-zero for k >= r >= c only (U is upper triangular), so of W only
-      // the lower triangle is ever read, and the product above forms only that
-      // (factorize + RGFdiag at
-      // ns = 1000, nt = 50 in FP64 550 -> 494 ms; ns = 2000, nt = 100 split 591 -> 577 ms)
-      GemmDesc g = mk(ins, ins, ins, Ui, ns, 0, h->d_T2, ns, 1, nullptr, 0, Q, lda, 1.0, 0.0);
-      g.triA = TRI_UPPER;
-      g.triB = TRI_LOWER;
-      g.outLower = 1;
-      gemm(h, g, BULK);
-      launch_mirror_lower(Q, lda, ins, s);
+      auto sigma = [&] {
+        if (!has_next && nd == 0) return;
+        const int kk = has_next ? m2 : ind;
+        GemmDesc g = mk(ins, ins, kk, K, kk, 1, Q + ns, lda, 0, Q, lda, Q, lda, -1.0, 1.0);
+        g.outLower = 1;
+        gemm(h, g, BULK);
+      };
+      // K of the next blocks, once the last K of the previous batch has been used
+      const bool refill = i > 0 && i - 1 < k_lo;
+      if (refill) {
+        sigma();
+        const long long lo = std::max(0LL, i - h->k_chunk);
+        GemmDesc k = mk(m2, ins, ins, h->d_MF + mf_col_offset(sh, lo) + ns, 2 * ns + nd, 0,
+                        h->d_U + lo * ss, ns, 1, nullptr, 0, h->d_K, m2, 1.0, 0.0);
+        k.triB = TRI_LOWER;
+        k.batch = (int)(i - lo); k.sA = sP; k.sB = ss; k.sD = ns * m2;
+        gemm(h, k, BULK);
+        k_lo = lo;
+      }
+      if (i > 0 && nd > 0 && !dense) {
+        // the arrowhead's part of the next block's G, in FP64 (in the same sliced
+        // product its larger terms would set the scale of the others); it needs
+        // nothing of Sigma_ii and runs beside it
+        const double* Kc = h->d_K + (i - 1 - k_lo) * ns * m2 + ns;
+        double* Gn = h->d_MS + mf_col_offset(sh, i - 1) + ns;
+        const double* Sd = Q + mf_dense_row(sh, i);
+        const long long ldg = 2 * ns + nd;
+        fork_side(h);
+        h->on_side = true;
+        gemm(h, mk(ins, ins, ind, Sd, lda, 1, Kc, m2, 0, nullptr, 0, Gn, ldg, -1.0, 0.0), SMALL);
+        gemm(h, mk(ind, ins, ind, Sdd, nd, 0, Kc, m2, 0, nullptr, 0, Gn + ns, ldg, -1.0, 0.0), SMALL);
+        h->on_side = false;
+      }
+      if (!refill) sigma();
+      // Sigma_ii is symmetric: its upper triangle, and S for the next block
+      launch_mirror_sigma(Q, lda, ins, Q + mf_dense_row(sh, i), Sdd, ind, i > 0 && dense ? h->d_S : nullptr, s);
       h->kernels_issued++;
     } else {
       // the reference's recursion (RGF.H:444-502):
@@ -1141,12 +1197,26 @@ int ensure_factored(rgf_handle* h) {
 int alloc_selinv(rgf_handle* h) {
   if (h->d_MS) return RGF_OK;
   const long long ns = h->sh.ns, nt = h->sh.nt, nd = h->sh.nd;
+  const bool compat = h->opts.selinv_mode == RGF_SELINV_COMPAT;
   int st;
+  auto once = [&](double** p, long long n) { return *p ? RGF_OK : dalloc(h, p, (size_t)n); };
+  if ((st = once(&h->d_U, nt * ns * ns + nd * nd))) return st;
+  if ((st = once(&h->d_T3, std::max<long long>(1, nd * ns)))) return st;
+  if (compat) {
+    if ((st = once(&h->d_T1, ns * ns))) return st;
+    if ((st = once(&h->d_T2, ns * ns))) return st;
+  } else {
+    if ((st = once(&h->d_S, (ns + nd) * (ns + nd)))) return st;
+    if (!h->d_K) {  // as many blocks as K_CHUNK_BYTES holds; one when memory is short
+      h->k_chunk = selinv_chunk(h->sh);
+      if ((st = dalloc(h, &h->d_K, (size_t)(h->k_chunk * (ns + nd) * ns))) && h->k_chunk > 1) {
+        h->k_chunk = 1;
+        st = dalloc(h, &h->d_K, (size_t)((ns + nd) * ns));
+      }
+      if (st) return st;
+    }
+  }
   if ((st = dalloc(h, &h->d_MS, h->mf_size))) return st;
-  if ((st = dalloc(h, &h->d_U, nt * ns * ns + nd * nd))) return st;
-  if ((st = dalloc(h, &h->d_T1, (ns + nd) * ns))) return st;
-  if ((st = dalloc(h, &h->d_T2, ns * ns))) return st;
-  if ((st = dalloc(h, &h->d_T3, std::max<long long>(1, nd * ns)))) return st;
   RGF_CK(cudaMemsetAsync(h->d_MS, 0, sizeof(double) * h->mf_size, h->stream));
   return RGF_OK;
 }
@@ -1218,7 +1288,7 @@ void release(rgf_handle* h) {
   if (h->trace_t0) cudaEventDestroy(h->trace_t0);
   delete h->split;
   delete h->split_side;
-  void* bufs[] = {h->d_ia, h->d_ja, h->d_a, h->d_MF, h->d_MS, h->d_U, h->d_T1, h->d_T2, h->d_T3,
+  void* bufs[] = {h->d_ia, h->d_ja, h->d_a, h->d_MF, h->d_MS, h->d_U, h->d_T1, h->d_T2, h->d_T3, h->d_K, h->d_S,
                   h->d_logpart, h->d_scalars, h->d_diag, h->d_status, h->d_rhs, h->d_partial,
                   h->d_res, h->d_ref, h->d_rhs2,
                   h->d_norms, h->d_panel_ws, h->d_arrow};

@@ -202,6 +202,10 @@ struct BtaShape {
 long long mf_col_offset(const BtaShape& sh, long long i);
 long long mf_lda(const BtaShape& sh, long long i);
 long long mf_dense_row(const BtaShape& sh, long long i);
+// Blocks whose K_i = [L_{i+1,i}; C_i] L_ii^{-1} the selected inversion forms in one
+// batch: as many as fit K_CHUNK_BYTES (four blocks of ns = 2000), at least one.
+constexpr size_t K_CHUNK_BYTES = (size_t)128 << 20;
+long long selinv_chunk(const BtaShape& sh);
 
 // Scatter the device CSC into the (pre-zeroed) MF layout; one warp per column.
 // Columns [c_lo, c_hi) only (c_hi < 0: to the last column): every entry of a
@@ -220,11 +224,12 @@ void launch_extract_diag(const BtaShape& sh, const double* MS, double* diag, cud
 // batch of identity matrices (m x m, ld) at X + b*stride
 void launch_set_identity(double* X, long long ld, int m, int batch, long long stride,
                          cudaStream_t s);
-// Y (m x n, ldy) = X (m x n, ldx); batched
-// Upper triangle of the symmetric n x n matrix X from its lower triangle.
-void launch_mirror_lower(double* X, long long ld, int n, cudaStream_t s);
-void launch_copy(const double* X, long long ldx, double* Y, long long ldy, int m, int n,
-                 int batch, long long sX, long long sY, cudaStream_t s);
+// Upper triangle of the symmetric n x n matrix X from its lower triangle; with S
+// (may be null) also the full symmetric
+// [X, Xd^T; Xd, Sdd] into S ((n + nd) x (n + nd), packed), Xd (nd x n, ld) its
+// arrowhead rows and Sdd nd x nd.
+void launch_mirror_sigma(double* X, long long ld, int n, const double* Xd, const double* Sdd,
+                         int nd, double* S, cudaStream_t s);
 // r = b - A x (symmetric, from the lower CSC) for the first column; then
 // out[0] = ||r||_2, out[1] = ||b||_2 (scaled sums of squares, as dnrm2).
 // scratch: n doubles.  CSC entries outside the lower triangle or past row n-1

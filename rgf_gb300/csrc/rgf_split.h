@@ -37,6 +37,8 @@ class SplitEngine {
   static int slots(int S);
   // Estimated device time of gemm(g, ..., slices), in seconds.
   double estimate_seconds(const GemmDesc& g, int slices = 0) const;
+  // Whether g's accuracy class allows the engine's slice count (see there).
+  bool may_slice(const GemmDesc& g, double bias) const;
   int min_k() const { return min_k_; }
   // Issue D = alpha op(A) op(B) + beta C on stream s; returns kernels launched
   // and, in *tensor_flops (if given), the bf16 slice-product flops it runs.

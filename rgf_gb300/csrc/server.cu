@@ -46,16 +46,16 @@ size_t estimate_bytes(const rgf_opts& o, size_t ns, size_t nt, size_t nd, size_t
   const size_t n = ns * nt + nd;
   const size_t mf = 2 * (nt - 1) * ns * ns + ns * ns + n * nd;
   size_t b = 16 * nnz + 8 * (n + 1) + 8 * mf;       // CSC + factor
-  b += 8 * mf + 8 * (nt * ns * ns + nd * nd) + 8 * (2 * ns * ns + nd * ns);  // selected inverse
-  // split-K workspaces of the main and side streams
-  b += 2 * 8 * std::min<size_t>(20u << 20, 8 * (2 * ns + nd) * std::max(ns, nd));
+  b += 8 * mf + 8 * (nt * ns * ns + nd * nd) + 8 * (nd * ns + 1);  // selected inverse
+  const rgf::BtaShape sh{(long long)ns, (long long)nt, (long long)nd, (long long)n};
+  if (o.selinv_mode == RGF_SELINV_COMPAT) b += 8 * 2 * ns * ns;
+  else b += 8 * (ns + nd) * (ns * (size_t)rgf::selinv_chunk(sh) + ns + nd);  // its workspaces
   if (o.precision == RGF_PREC_SPLIT) {  // slice workspaces of the main and side streams
     const size_t r = (2 * ns + nd + 127) / 128 * 128, k = (ns + nd + 63) / 64 * 64;
     const size_t one = 2 * 8 * r * k * 2;
     b += std::max(one, std::min<size_t>((size_t)1 << 30, nt * one / 4)) + (1 << 20);
     const size_t r2 = (ns + nd + 127) / 128 * 128;
     b += 2 * 8 * r2 * k * 2 + (1 << 20);
-    b += 2 * (80 * 128 * 128 * 8 + 4096);  // split-K partial sums of both engines
   }
   return b + (8u << 20);
 }
