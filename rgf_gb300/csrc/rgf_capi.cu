@@ -832,6 +832,8 @@ void issue_selinv(rgf_handle* h) {
   // G's route: an FP64 product reads the full symmetric S; a sliced one reads
   // Sigma_{i+1,i+1} and Sigma_{d,i+1} where they are
   const bool dense = nt < 2 || !routed_slices(h, g_split(0, h->d_K, 0.0), BULK);
+  // small blocks: the whole chain in one launch
+  const int chain = compat || h->k_chunk < nt - 1 ? 0 : selinv_chain_ctas(sh);
   if (!compat) {
     // Q_ii = U_i U_i^T of every block (lower part), the constant term of Sigma_ii
     GemmDesc u = mk(ins, ins, ins, h->d_U, ns, 0, h->d_U, ns, 1, nullptr, 0, h->d_MS, 2 * ns + nd,
@@ -847,7 +849,29 @@ void issue_selinv(rgf_handle* h) {
     u.ldd = ns + nd;
     gemm(h, u, BULK1);
   }
-  for (long long i = nt - 1; i >= 0; --i) {
+  // K_i of blocks [lo, hi) as one batch into d_K
+  auto batch_k = [&](long long lo, long long hi) {
+    GemmDesc k = mk(m2, ins, ins, h->d_MF + mf_col_offset(sh, lo) + ns, 2 * ns + nd, 0,
+                    h->d_U + lo * ss, ns, 1, nullptr, 0, h->d_K, m2, 1.0, 0.0);
+    k.triB = TRI_LOWER;
+    k.batch = (int)(hi - lo); k.sA = sP; k.sB = ss; k.sD = ns * m2;
+    gemm(h, k, BULK);
+    k_lo = lo;
+  };
+  auto last_k = [&] {  // C_i L_ii^{-1} of the last block
+    GemmDesc k = mk(ind, ins, ins, h->d_MF + mf_col_offset(sh, nt - 1) + ns, m2, 0,
+                    h->d_U + (nt - 1) * ss, ns, 1, nullptr, 0, h->d_T3, nd, 1.0, 0.0);
+    k.triB = TRI_LOWER;
+    gemm(h, k, BULK);
+  };
+  if (chain) {
+    batch_k(0, nt - 1);
+    last_k();
+    launch_selinv_chain(sh, chain, h->d_K, h->d_T3, h->d_MS, s);
+    h->kernels_issued++;
+    trace(h, "selinv chain");
+  }
+  for (long long i = chain ? -1 : nt - 1; i >= 0; --i) {
     const double* P = h->d_MF + mf_col_offset(sh, i);
     double* Q = h->d_MS + mf_col_offset(sh, i);
     const long long lda = mf_lda(sh, i);
@@ -868,9 +892,7 @@ void issue_selinv(rgf_handle* h) {
       const double* K = h->d_T3;
       if (!has_next) {
         if (nd > 0) {
-          GemmDesc k = mk(ind, ins, ins, Ci, lda, 0, Ui, ns, 1, nullptr, 0, h->d_T3, nd, 1.0, 0.0);
-          k.triB = TRI_LOWER;
-          gemm(h, k, BULK);
+          last_k();
           gemm(h, mk(ind, ins, ind, Sdd, nd, 0, h->d_T3, nd, 0, nullptr, 0,
                      Q + mf_dense_row(sh, i), lda, -1.0, 0.0), SMALL);
         }
@@ -895,13 +917,7 @@ void issue_selinv(rgf_handle* h) {
       const bool refill = i > 0 && i - 1 < k_lo;
       if (refill) {
         sigma();
-        const long long lo = std::max(0LL, i - h->k_chunk);
-        GemmDesc k = mk(m2, ins, ins, h->d_MF + mf_col_offset(sh, lo) + ns, 2 * ns + nd, 0,
-                        h->d_U + lo * ss, ns, 1, nullptr, 0, h->d_K, m2, 1.0, 0.0);
-        k.triB = TRI_LOWER;
-        k.batch = (int)(i - lo); k.sA = sP; k.sB = ss; k.sD = ns * m2;
-        gemm(h, k, BULK);
-        k_lo = lo;
+        batch_k(std::max(0LL, i - h->k_chunk), i);
       }
       if (i > 0 && nd > 0 && !dense) {
         // the arrowhead's part of the next block's G, in FP64 (in the same sliced

@@ -159,6 +159,19 @@ void launch_panel_tile(double* P, long long lda, int w, double* ws, int col0, De
 void launch_panel_rows(double* X, int rows, const double* P, long long lda, int w,
                        const double* ws, cudaStream_t s);
 
+// ---- chains of small blocks (k_chain.cu) -----------------------------------------
+struct BtaShape {
+  long long ns, nt, nd, n;
+};
+// Selected inversion of all blocks in one launch, for ns + nd <= SELINV_CHAIN_MAX: on
+// entry MS holds Q_i = U_i U_i^T (lower) in its diagonal blocks and Sigma_dd in the corner;
+// K the K_i of blocks 0 .. nt-2, Klast that of the last one (nd x ns).
+constexpr int SELINV_CHAIN_MAX = 72;
+// CTAs of that launch's cluster, 0 where the blocks are too large for it.
+int selinv_chain_ctas(const BtaShape& sh);
+void launch_selinv_chain(const BtaShape& sh, int nc, const double* K, const double* Klast,
+                         double* MS, cudaStream_t s);
+
 // Every device allocation of the library goes through here (so that a test
 // can make one fail: rgf_debug_fail_alloc_after).  cudaMalloc semantics.
 // On a thread that has a device arena set (set_thread_arena), memory comes
@@ -196,9 +209,6 @@ void launch_leaf_inverses(double* U, long long ldu, int n, const double* L, long
 int measure_fp64_peak(double* tflops);
 
 // ---- small kernels (k_misc.cu) ------------------------------------------------
-struct BtaShape {
-  long long ns, nt, nd, n;
-};
 long long mf_col_offset(const BtaShape& sh, long long i);
 long long mf_lda(const BtaShape& sh, long long i);
 long long mf_dense_row(const BtaShape& sh, long long i);

@@ -38,7 +38,8 @@ def _check(rgf, ns, nt, nd, precision="fp64", repeat=1):
             assert np.max(np.abs(got - want)) <= tol * np.max(np.abs(want))
 
 
-@pytest.mark.parametrize("ns", [1, 2, 5, 16, 17, 31, 32, 33, 42, 48, 63, 64, 65, 100, 129])
+@pytest.mark.parametrize("ns", [1, 2, 5, 11, 12, 13, 16, 17, 28, 29, 31, 32, 33, 42, 48, 56, 63, 64, 65, 72, 73,
+                                100, 129])
 @pytest.mark.parametrize("nt,nd", [(1, 0), (2, 1), (5, 0), (4, 6), (3, 17), (3, 33)])
 def test_blocks(rgf, ns, nt, nd):
     _check(rgf, ns, nt, nd, repeat=3)
