@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(CHAIN_THREADS) selinv_chain_kernel(const Selin
       (e < nd * nd ? S : S0 + (p.nt & 1) * m2 * sp)[(ns + x / nd) * sp + ns + x % nd] = Sdd[x];
     }
   }
+  __syncwarp();
   cluster_sync();  // every CTA is here before the first remote store
   for (long long i = p.nt - 1; i >= 0; --i) {
     const bool last = i == p.nt - 1;
@@ -178,45 +179,12 @@ __global__ void __launch_bounds__(CHAIN_THREADS) selinv_chain_kernel(const Selin
           }
       }
     }
+    __syncwarp();
     cluster_sync();
   }
   pdl_trigger();
 }
 
-}  // namespace
-
-namespace {
-// `bytes` of shared memory and clusters of 16 for the kernel on the current device
-template <typename K>
-bool allow_wide(K* kern, size_t bytes) {
-  if (!cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) &&
-      !cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))
-    return true;
-  cudaGetLastError();
-  return false;
-}
-// How many CTAs of the kernel a cluster can have with `bytes` of shared memory each: 16
-// (more than the portable size), else 8, or 0.
-template <typename K>
-int widest_cluster(K* kern, size_t bytes, int threads) {
-  if (!allow_wide(kern, bytes)) return 0;
-  for (int nc = 16; nc >= 8; nc /= 2) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nc);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = bytes;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = nc;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) cudaGetLastError();
-    else if (n >= 4) return nc;  // not only a corner of the chip
-  }
-  return 0;
-}
 }  // namespace
 
 // One CTA does blocks of up to 12 rows as fast as eight (the FP64 work of a block is
@@ -237,7 +205,7 @@ void launch_selinv_chain(const BtaShape& sh, int nc, const double* K, const doub
                          double* MS, cudaStream_t s) {
   const int ns = (int)sh.ns, m2 = (int)(sh.ns + sh.nd);
   const size_t bytes = selinv_chain_elems(ns, m2, nc) * sizeof(double);
-  allow_wide(selinv_chain_kernel, 227 * 1024);  // an attribute of the current device
+  allow_wide_clusters(selinv_chain_kernel, SELINV_CHAIN_SMEM);  // an attribute of the current device
   launch_k_cluster(selinv_chain_kernel, dim3(nc), dim3(CHAIN_THREADS), dim3(nc), bytes, s,
                    SelinvChain{ns, (int)sh.nd, sh.nt, K, Klast, MS});
 }

@@ -622,6 +622,252 @@ __global__ void __launch_bounds__(NT)
   }
 }
 
+// ---- chain: all block columns of a matrix of small blocks in one launch ----------
+// For ns <= 64 (one or two leaves a block) the launches of a block (tile, rows, update of
+// the next block) cost more than their work.  One cluster walks the block columns.
+// Every CTA holds the current diagonal leaf and factors it itself (its ~11 us a 32
+// columns are a serial chain: doing it NC times over costs nothing and saves sending
+// it); the other rows of the block column (rows 32.. of the diagonal block, then the nd
+// arrowhead rows, then the rows of the block below: row t at CTA t % NC) are solved
+// behind the leaf by the CTA that owns them, in shared memory, and go to all CTAs.
+// Then each CTA computes its share of the next leaf (or, after the last leaf, of the
+// next block: its leaf by elements, its rows by owner) and sends the leaf's elements to
+// all.  Two cluster barriers a leaf; the next block column's entries come by
+// asynchronous copies meanwhile.
+// The leaf's pivot chain bounds it (~0.35 us a column, of ~0.45 in all).  Factorization
+// of 40 blocks, launches per block -> this: ns = 3 0.35 -> 0.21 ms, ns = 16 0.64 -> 0.37,
+// ns = 32 0.90 -> 0.59, ns = 42 1.34 -> 0.87, ns = 64 1.61 -> 1.28 (0.13 ms of each the
+// ingest, the corner and the log-determinant).
+constexpr int CHAIN_ROW_WARPS = 8;
+constexpr int CHAIN_THREADS = TILE_THREADS + CHAIN_ROW_WARPS * 32;  // leaf, d^{-1/2}, rows
+
+struct ChainShape {  // of one CTA's shared memory
+  int nD, rows, pitch;
+  __host__ __device__ ChainShape(int ns, int nd, int nc)
+      : nD(ns > LB ? ns - LB : 0), rows((nD + nd + ns + nc - 1) / nc), pitch(ns | 1) {}
+  // own rows twice | rows of the block below | rows 32.. of the diagonal block | own
+  // elements of the next block's leaf
+  __host__ __device__ size_t elems(int ns, int nc) const {
+    return 2 * (size_t)rows * pitch + (size_t)ns * pitch + (size_t)nD * XPITCH +
+           (LB * (LB + 1) / 2 + nc - 1) / nc;
+  }
+};
+
+__global__ void __launch_bounds__(CHAIN_THREADS)
+    chain_factor_kernel(double* MF, int ns, int nd, long long nt, DevStatus* st, int wait_polls) {
+  extern __shared__ double dyn[];
+  __shared__ __align__(16) double Lc[LB][LB];
+  __shared__ double S[LB][LB], V[LB][LB], ys[LB];
+  __shared__ LeafShared sh;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nc = gridDim.x, rank = blockIdx.x;
+  const ChainShape z(ns, nd, nc);
+  const int nD = z.nD, nl = nD ? 2 : 1, xp = z.pitch, n0 = min(ns, LB);
+  double* X0 = dyn;                                  // own row j: t = rank + nc j
+  double* XB = X0 + 2 * z.rows * xp;                 // solved rows of the block below
+  double(*XD)[XPITCH] = reinterpret_cast<double(*)[XPITCH]>(XB + ns * xp);
+  double* E = XB + ns * xp + nD * XPITCH;            // element rank + nc e of the next leaf
+  const int leaf_elems = n0 * (n0 + 1) / 2;
+  const int ne = leaf_elems > rank ? (leaf_elems - rank + nc - 1) / nc : 0;
+  const double unset = __hiloint2double(UNSET_HI, 0);
+  const Wait wait{&sh.abort_, st, wait_polls};
+  auto clear_slots = [&]() {
+    for (int e = tid; e < LB * LB; e += CHAIN_THREADS) (&Lc[0][0])[e] = (&V[0][0])[e] = unset;
+    if (tid < LB) ys[tid] = unset;
+  };
+  auto element = [](int x, int& r, int& c) {         // x = r (r + 1) / 2 + c
+    r = (int)((sqrtf((float)(8 * x + 1)) - 1.0f) * 0.5f);  // exact for x < 528
+    c = x - r * (r + 1) / 2;
+  };
+  const long long sP = (long long)ns * (2 * ns + nd);
+  auto rows_of = [&](long long i) {                  // own rows in block column i
+    const int all = nD + nd + (i < nt - 1 ? ns : 0);
+    return all > rank ? (all - rank + nc - 1) / nc : 0;
+  };
+  // row t of block column i within its panel
+  auto row_at = [&](int t, bool last) {
+    return t < nD ? LB + t : t < nD + nd ? (last ? ns : 2 * ns) + t - nD : ns + t - nD - nd;
+  };
+  auto fetch_rows = [&](long long i) {
+    const bool last = i == nt - 1;
+    const double* P = MF + i * sP;
+    const long long lda = (last ? ns : 2 * ns) + nd;
+    double* X = X0 + (i & 1) * z.rows * xp;
+    const int n = rows_of(i);
+    for (int j = warp; j < n; j += CHAIN_THREADS / 32) {
+      const int t = rank + nc * j, r = row_at(t, last), len = t < nD ? LB + t + 1 : ns;
+      for (int c = lane; c < len; c += 32) cp_async8(X + j * xp + c, P + r + c * lda);
+    }
+  };
+  clear_slots();
+  if (tid == 0) {
+    sh.abort_ = 0;
+    sh.fail = 0x7fffffff;
+  }
+  pdl_wait();
+  fetch_rows(0);
+  cp_async_commit();
+  {
+    const long long lda = (nt == 1 ? ns : 2 * ns) + nd;
+    for (int c = warp; c < n0; c += CHAIN_THREADS / 32)
+      if (lane >= c && lane < n0) S[c][lane] = MF[lane + c * lda];
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  cluster_sync();  // every CTA is here before the first remote store
+
+  for (long long i = 0; i < nt; ++i) {
+    const bool last = i == nt - 1;
+    double* P = MF + i * sP;
+    const long long lda = (last ? ns : 2 * ns) + nd;
+    double* X = X0 + (i & 1) * z.rows * xp;
+    double* Xn = X0 + ((i + 1) & 1) * z.rows * xp;
+    const int nown = rows_of(i);
+    if (!last) {  // the next block column: own rows, own elements of its leaf
+      fetch_rows(i + 1);
+      const double* Pn = P + sP;
+      const long long ldn = (i + 1 == nt - 1 ? ns : 2 * ns) + nd;
+      for (int e = tid; e < ne; e += CHAIN_THREADS) {
+        int r, c;
+        element(rank + nc * e, r, c);
+        cp_async8(E + e, Pn + r + c * ldn);
+      }
+    }
+    cp_async_commit();
+#pragma unroll 1
+    for (int k = 0; k < nl; ++k) {
+      const int kc = k * LB, nbk = min(LB, ns - kc);
+      if (!*wait.abort_) {
+        if (warp < LEAF_WARPS) {
+          leaf_ldl(S, V, Lc, nbk, &sh, wait);
+        } else if (warp == LEAF_WARPS) {
+          leaf_send<1>(V, Lc, ys, nbk, wait, false);
+        } else {
+          constexpr int WG = 16, SL = LB / WG;       // two rows a warp
+          const int q = lane & (WG - 1);
+#pragma unroll 1
+          for (int j0 = (warp - LEAF_WARPS - 1) * 2; j0 < nown; j0 += CHAIN_ROW_WARPS * 2) {
+            const int j = j0 + lane / WG, t = rank + nc * j;
+            const bool live = j < nown && (k == 0 || t >= nD);
+            if (!__any_sync(0xffffffffu, live)) continue;
+            bool over = false;
+            double u[SL];
+#pragma unroll
+            for (int s = 0; s < SL; ++s) {
+              const int c = s * WG + q;
+              u[s] = live && c < nbk ? X[j * xp + kc + c] : 0.0;
+            }
+            leaf_row_solve<WG, true>(u, Lc, nbk, lane, wait, over);
+            const int r = row_at(t, last);
+#pragma unroll
+            for (int s = 0; s < SL; ++s) {
+              const int c = s * WG + q;
+              const double x =
+                  u[s] * lds_wait((unsigned)__cvta_generic_to_shared(&ys[c]), wait, over);
+              if (live && c < nbk) {
+                X[j * xp + kc + c] = x;
+                P[r + (kc + c) * lda] = x;
+                double* all = t < nD ? &XD[t][c]
+                              : t >= nD + nd ? XB + (t - nD - nd) * xp + kc + c : nullptr;
+                if (all)
+                  for (int w = 0; w < nc; ++w) st_cluster(cluster_addr(all, w), x);
+              }
+            }
+            if (__any_sync(0xffffffffu, over)) {
+              if (lane == 0) wait_gave_up(wait);
+              break;
+            }
+          }
+        }
+      }
+      __syncthreads();
+      cluster_arrive();
+      // L = V d^{-1/2}: each CTA writes its share of the leaf's columns
+      for (int c = rank + nc * warp; c < nbk; c += nc * (CHAIN_THREADS / 32))
+        if (lane >= c && lane < nbk)
+          P[kc + lane + (kc + c) * lda] = V[c][lane] * ys[c];
+      if (tid == 0) {
+        if (rank == 0 && sh.fail != 0x7fffffff)
+          atomicMin(&st->not_spd_col, (int)(i * ns) + kc + sh.fail);
+        sh.fail = 0x7fffffff;
+      }
+      cp_async_wait<0>();
+      __syncthreads();
+      clear_slots();
+      __syncwarp();
+      cluster_wait();                                // every row is solved
+      if (k + 1 == nl && last) break;
+      // updates: element e of this CTA is init - a . b over `terms` terms
+      const bool schur = k + 1 == nl;
+      const int terms = schur ? ns : LB;
+      int n = schur ? ne : 0;
+      auto row_len = [&](int j) {                    // elements of own row j
+        const int t = rank + nc * j;
+        if (schur) return t < nD ? LB + t + 1 : t < nD + nd ? ns : 0;
+        return t < nD ? t + 1 : nD;
+      };
+      for (int j = 0; j < nown; ++j) n += row_len(j);
+      int ks = 1;
+      {
+        int cost = 1 << 30;
+        for (int w = 1, lg = 1; w <= 8; w *= 2, ++lg) {
+          const int rounds = (n * w + CHAIN_THREADS - 1) / CHAIN_THREADS;
+          const int x = rounds * ((terms + w - 1) / w + lg);
+          if (x < cost) {
+            cost = x;
+            ks = w;
+          }
+        }
+      }
+      const int t8 = tid & (ks - 1);
+#pragma unroll 1
+      for (int e0 = 0; e0 < n; e0 += CHAIN_THREADS / ks) {
+        int e = e0 + tid / ks;
+        const bool live = e < n;
+        if (!__any_sync(0xffffffffu, live)) continue;
+        if (!live) e = 0;
+        double *dst, init;
+        const double *a, *b;
+        bool all;
+        if (schur && e < ne) {
+          int r, c;
+          element(rank + nc * e, r, c);
+          a = XB + r * xp;
+          b = XB + c * xp;
+          init = E[e];
+          dst = &S[c][r];
+          all = true;
+        } else {
+          if (schur) e -= ne;
+          int j = 0;
+          while (e >= row_len(j)) e -= row_len(j++);
+          const int t = rank + nc * j;
+          all = !schur && t < nD;
+          a = schur && t < nD ? XB + (LB + t) * xp : X + j * xp;
+          b = schur ? XB + e * xp : XD[e];
+          double* own = schur ? Xn + j * xp + e : X + j * xp + LB + e;
+          init = *own;
+          dst = all ? &S[e][t] : own;
+        }
+        double s = 0.0;
+        for (int l = t8; l < terms; l += ks) s = fma(a[l], b[l], s);
+        for (int o = 1; o < ks; o *= 2) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (live) {
+          const double v = init - s;
+          if (all) {
+            for (int w = t8; w < nc; w += ks) st_cluster(cluster_addr(dst, w), v);
+          } else if (t8 == 0) {
+            *dst = v;
+          }
+        }
+      }
+      __syncwarp();
+      cluster_sync();                                // the next leaf is in S, the rows are up to date
+    }
+  }
+  pdl_trigger();
+}
+
 template <int G, int NT>
 void launch_rows_g(double* X, int rows, const double* P, long long lda, int w, const double* ws,
                    cudaStream_t s) {
@@ -689,6 +935,25 @@ void launch_panel_rows(double* X, int rows, const double* P, long long lda, int 
   if (rows <= 4 * 152) launch_rows_g<32, 128>(X, rows, P, lda, w, ws, s);
   else if (rows <= 8 * 152) launch_rows_g<16, 128>(X, rows, P, lda, w, ws, s);
   else launch_rows_g<16, 256>(X, rows, P, lda, w, ws, s);
+}
+
+// One CTA does blocks of up to 12 rows as fast as eight; sixteen beat eight from ~32
+// columns (42: 19 against 20 us a block, 64: 29 against 35).  The line at 64 is the
+// kernel's two leaves; there it is still ahead of the separate launches (37 us).
+int chain_factor_ctas(const BtaShape& sh) {
+  if (sh.ns > CHAIN_MAX_NS || sh.ns + sh.nd > CHAIN_MAX_ROWS) return 0;
+  static const int widest = widest_cluster(chain_factor_kernel, CHAIN_FACTOR_SMEM, CHAIN_THREADS);
+  if (!widest) return 0;
+  return sh.ns + sh.nd <= 12 ? 1 : sh.ns + sh.nd <= 28 ? 8 : widest;
+}
+
+void launch_chain_factor(const BtaShape& sh, int nc, double* MF, DevStatus* st, cudaStream_t s,
+                         int wait_polls) {
+  const ChainShape z((int)sh.ns, (int)sh.nd, nc);
+  allow_wide_clusters(chain_factor_kernel, CHAIN_FACTOR_SMEM);  // an attribute of the current device
+  launch_k_cluster(chain_factor_kernel, dim3(nc), dim3(CHAIN_THREADS), dim3(nc),
+                   z.elems((int)sh.ns, nc) * sizeof(double), s, MF, (int)sh.ns, (int)sh.nd, sh.nt, st,
+                   wait_polls > 0 ? wait_polls : LEAF_WAIT_POLLS);
 }
 
 }  // namespace rgf

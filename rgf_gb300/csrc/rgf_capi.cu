@@ -670,7 +670,16 @@ void issue_factor(rgf_handle* h) {
   }
   h->mf_holds_a = false;
   double* corner = h->d_MF + mf_col_offset(sh, nt);
-  for (long long i = 0; i < nt; ++i) {
+  // small blocks: all block columns in one launch
+  const int chain = chain_factor_ctas(sh);
+  if (chain) {
+    if (streamed)
+      for (long long i = 0; i < nt; ++i) cudaStreamWaitEvent(s, h->ev_chunk[i], 0);
+    launch_chain_factor(sh, chain, h->d_MF, h->d_status, s, h->leaf_wait_polls);
+    h->kernels_issued++;
+    trace(h, "factor chain");
+  }
+  for (long long i = chain ? nt : 0; i < nt; ++i) {
     double* P = h->d_MF + mf_col_offset(sh, i);
     const long long lda = mf_lda(sh, i);
     if (streamed) cudaStreamWaitEvent(s, h->ev_chunk[i], 0);

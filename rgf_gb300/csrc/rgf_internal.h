@@ -82,6 +82,38 @@ inline void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
   launch_k_cluster(kern, grid, block, dim3(1, 1, 1), smem, s, args...);
 }
 
+// `bytes` of shared memory and clusters of 16 for the kernel on the current device
+template <typename K>
+bool allow_wide_clusters(K* kern, size_t bytes) {
+  if (!cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) &&
+      !cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))
+    return true;
+  cudaGetLastError();
+  return false;
+}
+// How many CTAs of the kernel a cluster can have with `bytes` of shared memory each: 16
+// (more than the portable size), else 8, or 0.
+template <typename K>
+int widest_cluster(K* kern, size_t bytes, int threads) {
+  if (!allow_wide_clusters(kern, bytes)) return 0;
+  for (int nc = 16; nc >= 8; nc /= 2) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nc);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = bytes;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = nc;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) cudaGetLastError();
+    else if (n >= 4) return nc;  // not only a corner of the chip
+  }
+  return 0;
+}
+
 enum Tri { TRI_NONE = 0, TRI_LOWER = 1, TRI_UPPER = 2 };
 
 // D = alpha * op(A) * op(B) + beta * C, column-major, op(A) m x k, op(B) k x n.
@@ -163,10 +195,19 @@ void launch_panel_rows(double* X, int rows, const double* P, long long lda, int 
 struct BtaShape {
   long long ns, nt, nd, n;
 };
+// Factorization of all block columns (not the corner) in one launch, for
+// ns <= CHAIN_MAX_NS and ns + nd <= CHAIN_MAX_ROWS (k_panel.cu); MF holds A on entry.
+// Status and waits as launch_panel_tile.
+constexpr int CHAIN_MAX_NS = 64, CHAIN_MAX_ROWS = 72;
+// CTAs of that launch's cluster, 0 where the blocks are too large for it.
+int chain_factor_ctas(const BtaShape& sh);
+void launch_chain_factor(const BtaShape& sh, int nc, double* MF, DevStatus* st, cudaStream_t s,
+                         int wait_polls = 0);
 // Selected inversion of all blocks in one launch, for ns + nd <= SELINV_CHAIN_MAX: on
 // entry MS holds Q_i = U_i U_i^T (lower) in its diagonal blocks and Sigma_dd in the corner;
 // K the K_i of blocks 0 .. nt-2, Klast that of the last one (nd x ns).
 constexpr int SELINV_CHAIN_MAX = 72;
+constexpr int SELINV_CHAIN_SMEM = 180 * 1024, CHAIN_FACTOR_SMEM = 64 * 1024;  // at most
 // CTAs of that launch's cluster, 0 where the blocks are too large for it.
 int selinv_chain_ctas(const BtaShape& sh);
 void launch_selinv_chain(const BtaShape& sh, int nc, const double* K, const double* Klast,
