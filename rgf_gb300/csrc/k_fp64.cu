@@ -374,34 +374,46 @@ __global__ void __launch_bounds__(128) gemm_thin_m_kernel(GemmDesc g, int kchunk
 // holds its unit ~76 cycles even with every lane predicated off, so the
 // columns are a template parameter and no FMA is issued for absent ones).
 // A CTA owns 32 output rows, lane = row.  A cluster of up to 8 CTAs
-// (blockIdx.y) splits K, and within a CTA the four warps take K tiles of 32
-// terms in turn: many SMs work on even a small product.  The partial sums
+// (blockIdx.y) splits the rows' K range evenly, and the four warps a CTA's share (K
+// tiles of 32 dealt to the warps left three of four FP64 units idle at K = 256): many SMs
+// work on even a small product.  The partial sums
 // meet in shared memory, first over the warps, then over the cluster through
 // distributed shared memory, both in a fixed order: one launch per product.
 // op(A) is read along its contiguous dimension; a transposed A goes through a
 // per-warp 32 x 32 shared-memory tile.  Measured over whole solves (four such
 // products per block column), against 128-row tiles with 16 predicated columns
 // and a second launch for the reduction: one right-hand side at ns = 256,
-// nt = 60 10.15 -> 1.08 ms (42 -> 4.5 us a product); eight at ns = 1000,
-// nt = 50, split (two sweeps and the residuals) 20.7 -> 10.8 ms.
+// nt = 60 10.15 -> 0.90 ms (42 -> 3.7 us a product), eight 3.66 -> 2.01 ms by the even
+// shares alone; eight at ns = 1000, nt = 50, split (two sweeps and the residuals)
+// 20.7 -> 10.5 ms.
 // op(A) may be triangular: K tiles that lie in its other triangle are skipped.
 constexpr int THIN_KT = 32;  // K terms of one warp's tile
 template <int N>
-__global__ void __launch_bounds__(128) gemm_thin_n_kernel(GemmDesc g, int kchunk) {
+__global__ void __launch_bounds__(128) gemm_thin_n_kernel(GemmDesc g) {
   // per warp: tile of a transposed A, element (k, row) at [k][row ^ k] (no bank
   // conflicts either way, within the 48 KiB of N = 16); then the warps' sums
   __shared__ double At[4][THIN_KT][32];
   __shared__ double Bs[4][THIN_KT][N];
   pdl_wait();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int r0 = blockIdx.x * 32, r = r0 + lane;
-  int k0 = blockIdx.y * kchunk, k1 = min(g.k, k0 + kchunk);
-  if (g.triA == TRI_LOWER) k1 = min(k1, r0 + 32);               // op(A)(r, kk) = 0 for kk > r
-  if (g.triA == TRI_UPPER) k0 = max(k0, r0 / THIN_KT * THIN_KT);  // and for kk < r
+  // the row tiles with the longest K range go first
+  const int bx = g.triA == TRI_LOWER ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+  const int r0 = bx * 32, r = r0 + lane;
+  int k0 = 0, k1 = g.k;
+  if (g.triA == TRI_LOWER) k1 = min(k1, r0 + 32);  // op(A)(r, kk) = 0 for kk > r
+  if (g.triA == TRI_UPPER) k0 = min(k1, r0);       // and for kk < r
+  // even shares of that range: of the cluster's CTAs (multiples of 8), of the warps (of 4)
+  const int nk = gridDim.y, rank = blockIdx.y;  // the cluster spans blockIdx.y
+  const int share = ((k1 - k0 + nk - 1) / nk + 7) & ~7;
+  k0 = min(k1, k0 + rank * share);
+  k1 = min(k1, k0 + share);
+  const int part = ((k1 - k0 + 3) / 4 + 3) & ~3;
+  k0 = min(k1, k0 + w * part);
+  k1 = min(k1, k0 + part);
   double acc[N];
 #pragma unroll
   for (int c = 0; c < N; ++c) acc[c] = 0.0;
-  for (int kt = k0 + w * THIN_KT; kt < k1; kt += 4 * THIN_KT) {
+  for (int kt = k0; kt < k1; kt += THIN_KT) {
     const int kn = min(THIN_KT, k1 - kt);
     double ra[THIN_KT];  // op(A)(r, kt + kk), or (transposed) op(A)(r0 + kk, kt + lane)
     if (!g.transA) {
@@ -462,7 +474,6 @@ __global__ void __launch_bounds__(128) gemm_thin_n_kernel(GemmDesc g, int kchunk
     const int c = o >> 5, l = o & 31;
     red[o] = ((At[0][c][l] + At[1][c][l]) + At[2][c][l]) + At[3][c][l];
   }
-  const int nk = gridDim.y, rank = blockIdx.y;  // the cluster spans blockIdx.y
   if (nk > 1) cluster_sync();
   else __syncthreads();
   // the cluster's total in rank order; the outputs are dealt over its CTAs
@@ -524,12 +535,12 @@ dim3 thin_split(const GemmDesc& g, int least, int* kchunk) {
   *kchunk = ((g.k + kc - 1) / kc + THIN_KT - 1) / THIN_KT * THIN_KT;
   return dim3(1, kc);
 }
+// (a thin-n CTA is worth 64 FMA instructions: 16 a warp, ~0.6 us)
 template <int N>
 void launch_thin_n(const GemmDesc& g, cudaStream_t s) {
-  int kchunk;
-  const dim3 cl = thin_split(g, THIN_KT, &kchunk);
-  launch_k_cluster(gemm_thin_n_kernel<N>, dim3((g.m + 31) / 32, cl.y), dim3(128), cl, 0, s, g,
-                   kchunk);
+  int kc = 1;
+  while (kc < 8 && g.k * N > kc * 64 && g.k > kc * 8) kc *= 2;
+  launch_k_cluster(gemm_thin_n_kernel<N>, dim3((g.m + 31) / 32, kc), dim3(128), dim3(1, kc), 0, s, g);
 }
 template <int M>
 void launch_thin_m(const GemmDesc& g, cudaStream_t s) {
