@@ -23,12 +23,13 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
 }
 
-// How many neighbouring threads (1, 2, 4 or 8) share each of n elements of `terms` terms:
-// the fewest FP64 instructions of a thread, over all rounds of the CTA's threads.
+// How many neighbouring threads (a power of two up to MAX) share each of n elements of
+// `terms` terms: the fewest FP64 instructions on an SM sub-partition.
+template <int MAX>
 __device__ __forceinline__ int lanes_per_element(int n, int terms) {
   int best = 1, cost = 1 << 30;
-  for (int ks = 1, lg = 0; ks <= 8; ks *= 2, ++lg) {
-    const int c = (n * ks + CHAIN_THREADS - 1) / CHAIN_THREADS * ((terms + ks - 1) / ks + lg + 1);
+  for (int ks = 1, lg = 1; ks <= MAX; ks *= 2, ++lg) {
+    const int c = ((n * ks + 31) / 32 + 3) / 4 * ((terms + ks - 1) / ks + lg);
     if (c < cost) {
       cost = c;
       best = ks;
@@ -122,7 +123,7 @@ __global__ void __launch_bounds__(CHAIN_THREADS) selinv_chain_kernel(const Selin
     __syncthreads();
     if (i > 0) fetch(i - 1);
     {  // G, own columns
-      const int n = ncol * mm, ks = lanes_per_element(n, mm), t = tid & (ks - 1);
+      const int n = ncol * mm, ks = lanes_per_element<8>(n, mm), t = tid & (ks - 1);
       for (int e0 = 0; e0 < n; e0 += CHAIN_THREADS / ks) {
         const int e = e0 + tid / ks;
         const bool live = e < n;
@@ -151,7 +152,7 @@ __global__ void __launch_bounds__(CHAIN_THREADS) selinv_chain_kernel(const Selin
     {  // Sigma_ii, own columns, lower part
       int n = 0;
       for (int j = 0; j < ncol; ++j) n += ns - rank - nc * j;
-      const int ks = lanes_per_element(n, mm), t = tid & (ks - 1);
+      const int ks = lanes_per_element<8>(n, mm), t = tid & (ks - 1);
       for (int e0 = 0; e0 < n; e0 += CHAIN_THREADS / ks) {
         int e = e0 + tid / ks, j = 0, c = rank;
         const bool live = e < n;
@@ -185,6 +186,213 @@ __global__ void __launch_bounds__(CHAIN_THREADS) selinv_chain_kernel(const Selin
   pdl_trigger();
 }
 
+// ---- block substitution: all right-hand sides through all blocks ---------------------
+// Forward, then backward (U_i = L_ii^{-T}, F_i = L_{i+1,i}):
+//   r_i = b_i - F_{i-1} y_{i-1},  y_i = U_i^T r_i;
+//   x_d = U_d U_d^T (b_d - sum_i C_i y_i), the blocks of the sum dealt over the CTAs;
+//   v_i = y_i - [F_i; C_i]^T [x_{i+1}; x_d],  x_i = U_i v_i.
+// CTA q of the cluster owns h neighbouring rows of every block's vectors and computes
+// them; each new vector goes to every CTA's shared memory, with one cluster
+// barrier per product.  Its rows or columns of the matrices do not depend on the chain:
+// they come by asynchronous copies one product ahead.
+// A product is bound by its barrier and the latency of its reduction (~1.5-2 us), from
+// ~8 K FMAs a CTA by the FP64 units.  Solves of 40 blocks, launches per product ->
+// this, with one / eight right-hand sides: ns = 3 377 / 819 -> 153 / 167 us, ns = 64
+// 446 / 1000 -> 279 / 398, ns = 128 556 / 1100 -> 347 / 785.
+struct SolveChain {
+  int ns, nd, nrhs;
+  long long nt, n;
+  const double *MF, *U;
+  double *R, *Y;  // b, then x; y
+};
+
+// Rows of a CTA, and doubles of shared memory: two matrix slices, and the vectors.
+__host__ __device__ inline int solve_rows(int ns, int nc) { return (ns + nc - 1) / nc; }
+__host__ __device__ inline size_t solve_slice(int ns, int nd, int nc) {
+  const int h = solve_rows(ns, nc);
+  const size_t rows = (size_t)ns * odd(h), cols = (size_t)h * odd(ns + nd);
+  return rows > cols ? rows : cols;
+}
+__host__ __device__ inline size_t solve_chain_elems(int ns, int nd, int nrhs, int nc) {
+  return 2 * solve_slice(ns, nd, nc) + (size_t)nrhs * (2 * ns + nd + (nc + 2) * nd) +
+         (size_t)nd * nd;
+}
+
+__global__ void __launch_bounds__(CHAIN_THREADS) solve_chain_kernel(const SolveChain p) {
+  extern __shared__ double smem[];
+  const int ns = p.ns, nd = p.nd, m2 = ns + nd, nq = p.nrhs, nc = gridDim.x, rank = blockIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int h = solve_rows(ns, nc), hp = odd(h), cp = odd(m2);
+  const int lo = min(rank * h, ns), hi = min(lo + h, ns);  // own rows
+  const size_t slice = solve_slice(ns, nd, nc);
+  double* W = smem + 2 * slice;   // r_i, then v_i: ns a right-hand side
+  double* Z = W + nq * ns;        // y_i, then [x_i; x_d]: m2
+  double* T = Z + nq * m2;        // arrowhead: the CTAs' parts of the sum, nq x nd each
+  double* T1 = T + nc * nq * nd;  // b_d - sum, then U_d^T of it
+  double* T2 = T1 + nq * nd;
+  double* Ud = T2 + nq * nd;
+  const long long ss = (long long)ns * ns, sP = (long long)ns * (2 * ns + nd);
+  int buf = 0;                    // slice buffer of the next product
+  auto lda_of = [&](long long i) { return (long long)(i == p.nt - 1 ? ns : 2 * ns) + nd; };
+  // rows [r0, r1) of a matrix with `terms` columns from c0: term l of row r at [l hp + r - r0]
+  auto fetch_rows = [&](const double* A, long long ld, int r0, int r1, int c0, int terms) {
+    double* d = smem + buf * slice;
+    const int w = r1 - r0, g = w <= 16 ? 16 : 32;  // lanes along the rows
+    for (int l = c0 + tid / g; l < terms; l += CHAIN_THREADS / g)
+      for (int r = tid % g; r < w; r += g) cp_async8(d + l * hp + r, A + r0 + r + l * ld);
+    cp_async_commit();
+  };
+  // columns [r0, r1) of a matrix, rows [0, len(r)): term l of column r at [(r - r0) cp + l]
+  auto fetch_cols = [&](const double* A, long long ld, int r0, int r1, int terms, bool tri) {
+    double* d = smem + buf * slice;
+    for (int r = r0 + (tid >> 5); r < r1; r += CHAIN_THREADS / 32)
+      for (int l = lane; l < (tri ? r + 1 : terms); l += 32)
+        cp_async8(d + (r - r0) * cp + l, A + l + r * ld);
+    cp_async_commit();
+  };
+  auto next = [&] {  // the slice of this product has arrived; the other buffer is free
+    cp_async_wait<0>();
+    __syncthreads();
+    buf ^= 1;
+    return smem + (buf ^ 1) * slice;
+  };
+  // out(r, q, init(r, q), sum over l in [l0(r), l1(r)) of a[(r - r0) rs + l ls] v[q vs + l],
+  // t, ks) for rows [r0, r1) and every right-hand side; t is the thread's place among the
+  // ks that share the element
+  auto product = [&](const double* a, int rs, int ls, int r0, int r1, const double* v, int vs,
+                     auto l0, auto l1, int terms, auto init, auto out) {
+    const int n = (r1 - r0) * nq;
+    const int ks = lanes_per_element<32>(n, terms);
+    const int t = tid & (ks - 1);
+    for (int e0 = 0; e0 < n; e0 += CHAIN_THREADS / ks) {
+      const int e = e0 + tid / ks;
+      const bool live = e < n;
+      if (!__any_sync(0xffffffffu, live)) continue;
+      const int q = live ? e / (r1 - r0) : 0, r = live ? r0 + e - q * (r1 - r0) : r0;
+      const double* ar = a + (r - r0) * rs;
+      const double* vq = v + q * vs;
+      const double x0 = init(r, q);
+      double s0 = 0.0, s1 = 0.0;
+      int l = l0(r) + t;
+      const int end = l1(r);
+      for (; l + ks < end; l += 2 * ks) {
+        s0 = fma(ar[l * ls], vq[l], s0);
+        s1 = fma(ar[(l + ks) * ls], vq[l + ks], s1);
+      }
+      if (l < end) s0 = fma(ar[l * ls], vq[l], s0);
+      s0 += s1;
+      for (int o = 1; o < ks; o *= 2) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+      if (live) out(r, q, x0, s0, t, ks);
+    }
+    __syncwarp();
+  };
+  auto to_all = [&](double* d, double x, int t, int ks) {
+    for (int z = t; z < nc; z += ks) st_cluster(cluster_addr(d, z), x);
+  };
+  const auto zero = [](int) { return 0; };
+  const auto all_m2 = [&](int) { return m2; };
+  const auto all_ns = [&](int) { return ns; };
+  const auto none = [](int, int) { return 0.0; };
+
+  pdl_wait();
+  fetch_cols(p.U, ns, lo, hi, ns, true);
+  for (int e = tid; e < nq * ns; e += CHAIN_THREADS) W[e] = p.R[e % ns + (long long)(e / ns) * p.n];
+  for (int e = tid; e < nq * nd; e += CHAIN_THREADS)
+    T1[e] = p.R[p.nt * ns + e % nd + (long long)(e / nd) * p.n];
+  for (int e = tid; e < nd * nd; e += CHAIN_THREADS) Ud[e] = p.U[p.nt * ss + e];
+  __syncwarp();
+  cluster_sync();  // every CTA is here before the first remote store
+
+  // ---- forward ----
+  for (long long i = 0; i < p.nt; ++i) {
+    const bool last = i == p.nt - 1;
+    // y_i = U_i^T r_i
+    const double* a = next();
+    if (!last) fetch_rows(p.MF + i * sP + ns, lda_of(i), lo, hi, 0, ns);
+    product(a, cp, 1, lo, hi, W, ns, zero, [](int r) { return r + 1; }, ns, none,
+            [&](int r, int q, double, double s, int t, int ks) {
+              if (!last) to_all(Z + q * m2 + r, s, t, ks);
+              if (t == 0) p.Y[i * ns + r + q * p.n] = s;
+            });
+    cluster_sync();
+    if (last) break;
+    // r_{i+1} = b_{i+1} - F_i y_i
+    a = next();
+    fetch_cols(p.U + (i + 1) * ss, ns, lo, hi, ns, true);
+    product(a, 1, hp, lo, hi, Z, m2, zero, all_ns, ns,
+            [&](int r, int q) { return p.R[(i + 1) * ns + r + q * p.n]; },
+            [&](int r, int q, double b, double s, int t, int ks) {
+              to_all(W + q * ns + r, b - s, t, ks);
+            });
+    cluster_sync();
+  }
+  // ---- the arrowhead ----
+  fetch_cols(p.MF + (p.nt - 1) * sP + ns, ns + nd, lo, hi, nd, false);
+  if (nd > 0) {
+    for (int e = tid >> 5; e < nq * nd; e += CHAIN_THREADS / 32) {
+      const int q = e / nd, d = e % nd;
+      double s = 0.0;
+      for (long long i = rank; i < p.nt; i += nc) {
+        const long long ld = lda_of(i);
+        const double* C = p.MF + i * sP + ld - nd + d;
+        const double* y = p.Y + i * ns + q * p.n;
+#pragma unroll 4
+        for (int l = lane; l < ns; l += 32) s = fma(C[l * ld], y[l], s);
+      }
+      for (int o = 1; o < 32; o *= 2) s += __shfl_xor_sync(0xffffffffu, s, o);
+      for (int z = lane; z < nc; z += 32) st_cluster(cluster_addr(T + rank * nq * nd + e, z), s);
+    }
+    __syncwarp();
+    cluster_sync();
+    for (int e = tid; e < nq * nd; e += CHAIN_THREADS) {
+      double s = 0.0;
+      for (int z = 0; z < nc; ++z) s += T[z * nq * nd + e];
+      T1[e] -= s;
+    }
+    __syncthreads();
+    for (int e = tid; e < nq * nd; e += CHAIN_THREADS) {  // x_d = U_d (U_d^T t), in every CTA
+      const int q = e / nd, r = e % nd;
+      double s = 0.0;
+      for (int l = 0; l <= r; ++l) s = fma(Ud[r * nd + l], T1[q * nd + l], s);
+      T2[e] = s;
+    }
+    __syncthreads();
+    for (int e = tid; e < nq * nd; e += CHAIN_THREADS) {
+      const int q = e / nd, r = e % nd;
+      double s = 0.0;
+      for (int l = nd - 1; l >= r; --l) s = fma(Ud[l * nd + r], T2[q * nd + l], s);
+      Z[q * m2 + ns + r] = s;
+      if (rank == 0) p.R[p.nt * ns + r + q * p.n] = s;
+    }
+  }
+  // ---- backward ----
+  for (long long i = p.nt - 1; i >= 0; --i) {
+    const bool last = i == p.nt - 1;
+    // v_i = y_i - [F_i; C_i]^T [x_{i+1}; x_d]
+    const double* a = next();
+    fetch_rows(p.U + i * ss, ns, lo, hi, lo, ns);
+    const int s0 = last ? ns : 0;
+    product(a - s0, cp, 1, lo, hi, Z, m2, [&](int) { return s0; }, all_m2, m2 - s0,
+            [&](int r, int q) { return p.Y[i * ns + r + q * p.n]; },
+            [&](int r, int q, double y, double s, int t, int ks) {
+              to_all(W + q * ns + r, y - s, t, ks);
+            });
+    cluster_sync();
+    // x_i = U_i v_i
+    a = next();
+    if (i > 0) fetch_cols(p.MF + (i - 1) * sP + ns, lda_of(i - 1), lo, hi, m2, false);
+    product(a, 1, hp, lo, hi, W, ns, [](int r) { return r; }, all_ns, ns, none,
+            [&](int r, int q, double, double s, int t, int ks) {
+              if (i > 0) to_all(Z + q * m2 + r, s, t, ks);
+              if (t == 0) p.R[i * ns + r + q * p.n] = s;
+            });
+    if (i > 0) cluster_sync();
+  }
+  pdl_trigger();
+  __syncwarp();
+  cluster_sync();  // no CTA leaves while another may still store to it
+}
+
 }  // namespace
 
 // One CTA does blocks of up to 12 rows as fast as eight (the FP64 work of a block is
@@ -208,6 +416,29 @@ void launch_selinv_chain(const BtaShape& sh, int nc, const double* K, const doub
   allow_wide_clusters(selinv_chain_kernel, SELINV_CHAIN_SMEM);  // an attribute of the current device
   launch_k_cluster(selinv_chain_kernel, dim3(nc), dim3(CHAIN_THREADS), dim3(nc), bytes, s,
                    SelinvChain{ns, (int)sh.nd, sh.nt, K, Klast, MS});
+}
+
+// The lines, from solves of 40 to 60 blocks (chain of 16 CTAs / two launches a block and
+// direction, in us): ns = 128 347 / 556 with one right-hand side, 1319 / 1675 with 16;
+// ns = 192 499 / 574, 691 / 667 with two and about even above; ns = 256 875 / 901, then
+// behind.  One CTA beats eight while a product has up to ~600 FMAs (ns = 3: 153
+// against 195), sixteen beat eight from ~48 rows.
+int solve_chain_ctas(const BtaShape& sh, int nrhs) {
+  const long long m2 = sh.ns + sh.nd;
+  if (m2 > SOLVE_CHAIN_MAX || sh.ns > (nrhs == 1 ? 256 : 176)) return 0;
+  static const int widest = widest_cluster(solve_chain_kernel, SOLVE_CHAIN_SMEM, CHAIN_THREADS);
+  if (!widest || (widest < 16 && sh.ns > 100)) return 0;
+  const int nc = m2 * m2 * nrhs <= 600 ? 1 : m2 <= 48 ? 8 : widest;
+  if (solve_chain_elems((int)sh.ns, (int)sh.nd, nrhs, nc) * sizeof(double) > SOLVE_CHAIN_SMEM) return 0;
+  return nc;
+}
+
+void launch_solve_chain(const BtaShape& sh, int nc, const double* MF, const double* U, double* R,
+                        double* Y, int nrhs, cudaStream_t s) {
+  allow_wide_clusters(solve_chain_kernel, SOLVE_CHAIN_SMEM);  // an attribute of the current device
+  launch_k_cluster(solve_chain_kernel, dim3(nc), dim3(CHAIN_THREADS), dim3(nc),
+                   solve_chain_elems((int)sh.ns, (int)sh.nd, nrhs, nc) * sizeof(double), s,
+                   SolveChain{(int)sh.ns, (int)sh.nd, nrhs, sh.nt, sh.n, MF, U, R, Y});
 }
 
 }  // namespace rgf

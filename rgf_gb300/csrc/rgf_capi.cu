@@ -1013,6 +1013,12 @@ void issue_solve(rgf_handle* h, int nrhs) {
   double* R = h->d_rhs;
   double* Y = h->d_rhs2;
   const double* corner = h->d_MF + mf_col_offset(sh, nt);
+  if (const int chain = solve_chain_ctas(sh, nrhs)) {  // small blocks: one launch
+    launch_solve_chain(sh, chain, h->d_MF, h->d_U, R, Y, nrhs, h->stream);
+    h->kernels_issued++;
+    trace(h, "solve chain");
+    return;
+  }
   for (long long i = 0; i < nt; ++i) {
     if (i > 0) {  // b_i -= L_{i,i-1} y_{i-1}   (RGF.H:365)
       const double* Pm = h->d_MF + mf_col_offset(sh, i - 1);

@@ -213,6 +213,15 @@ int selinv_chain_ctas(const BtaShape& sh);
 void launch_selinv_chain(const BtaShape& sh, int nc, const double* K, const double* Klast,
                          double* MS, cudaStream_t s);
 
+// The block substitution of nrhs right-hand sides in one launch: R holds b on entry and x
+// on return, Y is scratch (both n x nrhs); U the inverses of all diagonal blocks and of
+// the corner.
+constexpr int SOLVE_CHAIN_MAX = 320, SOLVE_CHAIN_SMEM = 200 * 1024;
+// CTAs of that launch's cluster, 0 where separate products are the better way.
+int solve_chain_ctas(const BtaShape& sh, int nrhs);
+void launch_solve_chain(const BtaShape& sh, int nc, const double* MF, const double* U, double* R,
+                        double* Y, int nrhs, cudaStream_t s);
+
 // Every device allocation of the library goes through here (so that a test
 // can make one fail: rgf_debug_fail_alloc_after).  cudaMalloc semantics.
 // On a thread that has a device arena set (set_thread_arena), memory comes
