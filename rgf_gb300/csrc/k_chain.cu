@@ -418,14 +418,13 @@ void launch_selinv_chain(const BtaShape& sh, int nc, const double* K, const doub
                    SelinvChain{ns, (int)sh.nd, sh.nt, K, Klast, MS});
 }
 
-// The lines, from solves of 40 to 60 blocks (chain of 16 CTAs / two launches a block and
-// direction, in us): ns = 128 347 / 556 with one right-hand side, 1319 / 1675 with 16;
-// ns = 192 499 / 574, 691 / 667 with two and about even above; ns = 256 875 / 901, then
-// behind.  One CTA beats eight while a product has up to ~600 FMAs (ns = 3: 153
-// against 195), sixteen beat eight from ~48 rows.
+// The lines, from solves of 40 to 60 blocks (chain of 16 CTAs / separate products, in
+// us): ns = 128 347 / 490 with one right-hand side, 781 / 960 with eight; ns = 160 458 / 456
+// with one, 606 / 565 with two; ns = 256 875 / 812.  One CTA beats eight while a
+// product has up to ~600 FMAs (ns = 3: 153 against 195), sixteen beat eight from ~48 rows.
 int solve_chain_ctas(const BtaShape& sh, int nrhs) {
   const long long m2 = sh.ns + sh.nd;
-  if (m2 > SOLVE_CHAIN_MAX || sh.ns > (nrhs == 1 ? 256 : 176)) return 0;
+  if (m2 > SOLVE_CHAIN_MAX || sh.ns > (nrhs == 1 ? 176 : 144)) return 0;
   static const int widest = widest_cluster(solve_chain_kernel, SOLVE_CHAIN_SMEM, CHAIN_THREADS);
   if (!widest || (widest < 16 && sh.ns > 100)) return 0;
   const int nc = m2 * m2 * nrhs <= 600 ? 1 : m2 <= 48 ? 8 : widest;

@@ -354,7 +354,15 @@ __global__ void __launch_bounds__(128) gemm_thin_m_kernel(GemmDesc g, int kchunk
     const int r = o >> 5, col = c0 + (o & 31);
     double v = 0.0;
     if (nk > 1) {
-      for (int q = 0; q < nk; ++q) v += ld_cluster(red + o, q);
+      double part[8];  // all loads in flight, then the sum in rank order
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (q < nk) part[q] = ld_cluster(red + o, q);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        if (q >= nk) break;
+        v += part[q];
+      }
     } else {
       v = red[o];
     }
@@ -383,10 +391,13 @@ __global__ void __launch_bounds__(128) gemm_thin_m_kernel(GemmDesc g, int kchunk
 // per-warp 32 x 32 shared-memory tile.  Measured over whole solves (four such
 // products per block column), against 128-row tiles with 16 predicated columns
 // and a second launch for the reduction: one right-hand side at ns = 256,
-// nt = 60 10.15 -> 0.90 ms (42 -> 3.7 us a product), eight 3.66 -> 2.01 ms by the even
-// shares alone; eight at ns = 1000, nt = 50, split (two sweeps and the residuals)
-// 20.7 -> 10.5 ms.
+// nt = 60 10.15 -> 0.81 ms (42 -> 3.4 us a product), eight 3.66 -> 2.01 ms by the even
+// shares alone; eight at ns = 1000, nt = 50, split (with the residuals) 20.7 -> 7.8 ms.
 // op(A) may be triangular: K tiles that lie in its other triangle are skipped.
+// With `early` (the caller vouches that the previous kernel of the stream does not write
+// A: the block substitution, whose matrices are the factor's) the first tile of A is
+// loaded while that kernel still runs (eight right-hand sides, ns = 256, nt = 60:
+// 2.01 -> 1.65 ms; one 0.90 -> 0.81).
 constexpr int THIN_KT = 32;  // K terms of one warp's tile
 template <int N>
 __global__ void __launch_bounds__(128) gemm_thin_n_kernel(GemmDesc g) {
@@ -394,7 +405,6 @@ __global__ void __launch_bounds__(128) gemm_thin_n_kernel(GemmDesc g) {
   // conflicts either way, within the 48 KiB of N = 16); then the warps' sums
   __shared__ double At[4][THIN_KT][32];
   __shared__ double Bs[4][THIN_KT][N];
-  pdl_wait();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   // the row tiles with the longest K range go first
   const int bx = g.triA == TRI_LOWER ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
@@ -413,9 +423,9 @@ __global__ void __launch_bounds__(128) gemm_thin_n_kernel(GemmDesc g) {
   double acc[N];
 #pragma unroll
   for (int c = 0; c < N; ++c) acc[c] = 0.0;
-  for (int kt = k0; kt < k1; kt += THIN_KT) {
+  double ra[THIN_KT];  // op(A)(r, kt + kk), or (transposed) op(A)(r0 + kk, kt + lane)
+  auto load_a = [&](int kt) {
     const int kn = min(THIN_KT, k1 - kt);
-    double ra[THIN_KT];  // op(A)(r, kt + kk), or (transposed) op(A)(r0 + kk, kt + lane)
     if (!g.transA) {
       const double* a = g.A + r + (long long)kt * g.lda;
 #pragma unroll
@@ -438,6 +448,12 @@ __global__ void __launch_bounds__(128) gemm_thin_n_kernel(GemmDesc g) {
         a += g.lda;
       }
     }
+  };
+  if (g.early && k0 < k1) load_a(k0);
+  pdl_wait();
+  if (!g.early && k0 < k1) load_a(k0);
+  for (int kt = k0; kt < k1; kt += THIN_KT) {
+    const int kn = min(THIN_KT, k1 - kt);
 #pragma unroll
     for (int c = 0; c < N; ++c)
       Bs[w][lane][c] = lane < kn && c < g.n ? g.B[kt + lane + (long long)c * g.ldb] : 0.0;
@@ -461,6 +477,7 @@ __global__ void __launch_bounds__(128) gemm_thin_n_kernel(GemmDesc g) {
       }
     }
     __syncwarp();
+    if (kt + THIN_KT < k1) load_a(kt + THIN_KT);
   }
   pdl_trigger();
   // this CTA's sums: warp partials in At[w][c][lane], summed in warp order
@@ -481,7 +498,15 @@ __global__ void __launch_bounds__(128) gemm_thin_n_kernel(GemmDesc g) {
     const int c = o >> 5, row = r0 + (o & 31);
     double v = 0.0;
     if (nk > 1) {
-      for (int q = 0; q < nk; ++q) v += ld_cluster(red + o, q);
+      double part[8];  // all loads in flight, then the sum in rank order
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (q < nk) part[q] = ld_cluster(red + o, q);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        if (q >= nk) break;
+        v += part[q];
+      }
     } else {
       v = red[o];
     }

@@ -1019,17 +1019,23 @@ void issue_solve(rgf_handle* h, int nrhs) {
     trace(h, "solve chain");
     return;
   }
+  // the factor and its inverses are complete before the stage: their loads need not wait
+  // for the product before
+  auto product = [&](GemmDesc g) {
+    g.early = true;
+    gemm(h, g, SMALL);
+  };
   for (long long i = 0; i < nt; ++i) {
     if (i > 0) {  // b_i -= L_{i,i-1} y_{i-1}   (RGF.H:365)
       const double* Pm = h->d_MF + mf_col_offset(sh, i - 1);
-      gemm(h, mk(ins, nrhs, ins, Pm + ns, mf_lda(sh, i - 1), 0, Y + (i - 1) * ns, n, 0,
-                 R + i * ns, n, R + i * ns, n, -1.0, 1.0), SMALL);
+      product(mk(ins, nrhs, ins, Pm + ns, mf_lda(sh, i - 1), 0, Y + (i - 1) * ns, n, 0,
+                 R + i * ns, n, R + i * ns, n, -1.0, 1.0));
     }
     // y_i = L_ii^{-1} b_i = U_i^T b_i   (RGF.H:356, 367)
     GemmDesc g = mk(ins, nrhs, ins, h->d_U + i * ss, ns, 1, R + i * ns, n, 0, nullptr, 0,
                     Y + i * ns, n, 1.0, 0.0);
     g.triA = TRI_LOWER;
-    gemm(h, g, SMALL);
+    product(g);
   }
   if (nd > 0) {
     // b_d -= sum_i C_i y_i; y_d, then x_d, by the corner factor   (RGF.H:377-393)
@@ -1052,14 +1058,14 @@ void issue_solve(rgf_handle* h, int nrhs) {
   for (long long i = nt - 1; i >= 0; --i) {
     if (i < nt - 1) {  // y_i -= L_{i+1,i}^T x_{i+1}   (RGF.H:410)
       const double* P = h->d_MF + mf_col_offset(sh, i);
-      gemm(h, mk(ins, nrhs, ins, P + ns, mf_lda(sh, i), 1, R + (i + 1) * ns, n, 0, Y + i * ns, n,
-                 Y + i * ns, n, -1.0, 1.0), SMALL);
+      product(mk(ins, nrhs, ins, P + ns, mf_lda(sh, i), 1, R + (i + 1) * ns, n, 0, Y + i * ns, n,
+                 Y + i * ns, n, -1.0, 1.0));
     }
     // x_i = L_ii^{-T} y_i = U_i y_i   (RGF.H:408, 417)
     GemmDesc g = mk(ins, nrhs, ins, h->d_U + i * ss, ns, 0, Y + i * ns, n, 0, nullptr, 0,
                     R + i * ns, n, 1.0, 0.0);
     g.triA = TRI_UPPER;
-    gemm(h, g, SMALL);
+    product(g);
   }
 }
 

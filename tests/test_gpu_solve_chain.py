@@ -1,5 +1,5 @@
 """Block substitution in one launch and its lines: block sizes around the cluster sizes'
-lines and the last ones it takes (176; 256 with one right-hand side), no and wide
+lines and the last ones it takes (144; 176 with one right-hand side), no and wide
 arrowheads, one block, one to many right-hand sides (more than fit its shared memory,
 too), FP64 and refined split solves.
 
@@ -20,7 +20,7 @@ EPS = np.finfo(np.float64).eps
 
 @pytest.mark.parametrize("precision", ["fp64", "split"])
 @pytest.mark.parametrize("ns,nt,nd", [(1, 1, 0), (1, 5, 1), (7, 1, 3), (3, 40, 2), (20, 4, 0), (20, 3, 60),
-                                      (46, 3, 2), (47, 3, 2), (64, 3, 0), (100, 2, 1), (175, 3, 3),
+                                      (46, 3, 2), (47, 3, 2), (64, 3, 0), (100, 2, 1), (144, 3, 3), (145, 3, 3), (175, 3, 3),
                                       (176, 3, 1), (177, 3, 1), (256, 3, 4), (257, 3, 0), (250, 2, 80)])
 def test_solve(rgf, precision, ns, nt, nd):
     ia, ja, a = gen.generate_bta(ns, nt, nd, seed=ns + nd)
