@@ -49,9 +49,11 @@ __global__ void __launch_bounds__(128) gemm_fp64_kernel(GemmDesc g) {
   constexpr int LPT = TM * TK / 128;     // elements per thread per operand and stage
   constexpr int PAD = TM + 4;
   pdl_wait();
-  const int m0 = blockIdx.x * TM;
-  const int n0 = blockIdx.y * TM;
-  if (!tile_written(g.outLower, g.outUpper, m0, n0, TM)) return;
+  // blockIdx.x counts the written tiles only, column by column.  (With a CTA for every
+  // tile the skipped ones' places were dealt out too, and SMs got two of the others while
+  // some got none: the lower half of 333 x 333 x 338 in 132 CTAs 110 us, now 65.)
+  const TilePos tile = tile_at(g.outLower, (g.m + TM - 1) / TM, blockIdx.x);
+  const int m0 = tile.x * TM, n0 = tile.y * TM;
   // blockIdx.z = batch item * ksplit + K slice; the slices of a tile are a cluster
   const bool splitk = g.ksplit > 1;
   const long long bz = blockIdx.z / g.ksplit;
@@ -192,8 +194,7 @@ __global__ void __launch_bounds__(128) gemm_fp64_kernel(GemmDesc g) {
       for (int u = 0; u < U; ++u) {
         const int idx = (kz * share + q0 + u) * 128 + tid;
         const int r = m0 + idx % TM, c = n0 + idx / TM;
-        if (q0 + u >= share || idx >= TM * TM || r >= g.m || c >= g.n || (g.outLower && r < c) ||
-            (g.outUpper && r > c))
+        if (q0 + u >= share || idx >= TM * TM || r >= g.m || c >= g.n || (g.outLower && r < c))
           continue;
         double x = g.alpha * v[u];
         if (g.beta != 0.0) x += g.beta * (r < mD1 ? C : C2)[(long long)r + (long long)c * g.ldc];
@@ -215,7 +216,7 @@ __global__ void __launch_bounds__(128) gemm_fp64_kernel(GemmDesc g) {
       for (int e = 0; e < 2; ++e) {
         const int c = n0 + wn + j * 8 + (lane & 3) * 2 + e;
         if (c >= g.n) continue;
-        if ((g.outLower && r < c) || (g.outUpper && r > c)) continue;
+        if (g.outLower && r < c) continue;
         double v = g.alpha * acc[i][j][e];
         if (g.beta != 0.0) v += g.beta * Cr[(long long)r + (long long)c * g.ldc];
         Dr[(long long)r + (long long)c * g.ldd] = v;
@@ -602,7 +603,6 @@ double gemm_flops(const GemmDesc& g) {
   double f = 2.0 * m * n * k;
   if (g.triA != TRI_NONE) f = m * (m + 1.0) * n;
   if (g.triB != TRI_NONE) f = m * n * (n + 1.0);
-  if (g.outUpper && g.m == g.n) f = k * m * (m + 1.0);
   if (g.outLower && g.m >= g.n && g.n > 0) f = 2.0 * k * (n * (n + 1.0) / 2.0 + (m - n) * n);
   return f * g.batch;
 }
@@ -610,12 +610,12 @@ double gemm_flops(const GemmDesc& g) {
 int launch_gemm_fp64(const GemmDesc& g0, cudaStream_t s) {
   if (g0.m <= 0 || g0.n <= 0 || g0.batch <= 0) return 0;
   GemmDesc g = g0;
-  if (g.m <= 16 && g.transB && g.triA == TRI_NONE && g.batch == 1 && !g.outLower && !g.outUpper &&
+  if (g.m <= 16 && g.transB && g.triA == TRI_NONE && g.batch == 1 && !g.outLower &&
       !g.A2) {
     launch_gemm_thin_m(g, s);
     return 1;
   }
-  if (g.n <= 16 && !g.transB && g.triB == TRI_NONE && g.batch == 1 && !g.outLower && !g.outUpper &&
+  if (g.n <= 16 && !g.transB && g.triB == TRI_NONE && g.batch == 1 && !g.outLower &&
       !g.A2 && !g.D2) {
     launch_gemm_thin_n(g, s);
     return 1;
@@ -653,8 +653,7 @@ int launch_gemm_fp64(const GemmDesc& g0, cudaStream_t s) {
     }
   }
   g.ksplit = ksplit;
-  const int tx = (g.m + tm - 1) / tm, ty = (g.n + tm - 1) / tm;
-  const dim3 grid(tx, ty, ksplit * g.batch), cluster(1, 1, ksplit);
+  const dim3 grid((unsigned)tiles_written(g, tm), 1, ksplit * g.batch), cluster(1, 1, ksplit);
   if (tm == 32) launch_k_cluster(gemm_fp64_kernel<32, 8>, grid, dim3(128), cluster, 0, s, g);
   else launch_k_cluster(gemm_fp64_kernel<64, 16>, grid, dim3(128), cluster, 0, s, g);
   return 1;

@@ -77,7 +77,7 @@ struct SplitParams {
   // at a time; level of the first half gl1, of the second gl2 (NO_SLICE: none)
   int ngroups;
   unsigned char g0[MAXGROUPS], gs[MAXGROUPS], gl1[MAXGROUPS], gl2[MAXGROUPS], gchunk[MAXGROUPS];
-  int triA, triB, outLower, outUpper;
+  int triA, triB, outLower;
   const int* exA;
   const int* exB;
   int exA_stride, exB_stride;   // per batch item (padded rows)
@@ -328,8 +328,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-  if (!tile_written(p.outLower, p.outUpper, m0, n0, BM)) return;  // nothing to write (uniform exit)
+  const TilePos tile = tile_at(p.outLower, (p.m + BM - 1) / BM, blockIdx.x);  // written ones only
+  const int m0 = tile.x * BM, n0 = tile.y * BN;
   const int zb = blockIdx.z / p.ksplit;     // batch item: slice planes zb*S .. zb*S+S-1
   const int kz = blockIdx.z - zb * p.ksplit;
   const int zS = zb * p.S;
@@ -543,27 +543,25 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
           live ? p.exA[(long long)zb * p.exA_stride + r] + p.cs - p.beta * (p.S + 1) + 2 : 0;
       const double alpha = p.alpha, betac = p.betac;
       const long long ldc = p.ldc * cstep, ldd = p.ldd * cstep;
-      // columns c with c < n, c <= r (outLower), c >= r (outUpper): i in [c_lo, nlive)
+      // columns c with c < n, c <= r (outLower): i < nlive
       int climit = min(n0 + cend, p.n);  // first column not written
       if (p.outLower) climit = min(climit, r + 1);
       const int nlive = live && climit > cbase ? (climit - cbase + cstep - 1) / cstep : 0;
-      const int c_lo = p.outUpper && r > cbase ? (r - cbase + cstep - 1) / cstep : 0;
-      // the warp's columns: from the first any lane writes to the last
+      // the warp's columns: to the last that any lane writes
       const int i_end = __reduce_max_sync(0xffffffffu, nlive);
-      const int i_beg = __reduce_min_sync(0xffffffffu, c_lo) & ~7;
       auto convert = [&](auto with_c) {
         constexpr bool WITH_C = decltype(with_c)::value;
         // column pointers advance by ldc / ldd (no 64-bit multiply per output)
         const double* Cp =
-            WITH_C && live ? C + r + (cbase + (long long)cstep * i_beg) * p.ldc : nullptr;
-        double* Dp = live ? D + r + (cbase + (long long)cstep * i_beg) * p.ldd : nullptr;
+            WITH_C && live ? C + r + (long long)cbase * p.ldc : nullptr;
+        double* Dp = live ? D + r + (long long)cbase * p.ldd : nullptr;
 #pragma unroll 1
-        for (int i0 = i_beg; i0 < i_end; i0 += 8) {
+        for (int i0 = 0; i0 < i_end; i0 += 8) {
           double cv[8];
           if (WITH_C) {
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
-              cv[q] = i0 + q < nlive && i0 + q >= c_lo ? *Cp : 0.0;
+              cv[q] = i0 + q < nlive ? *Cp : 0.0;
               Cp += ldc;
             }
           }
@@ -594,7 +592,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
               v *= alpha;
             }
             if (WITH_C) v = fma(betac, cv[q], v);
-            if (i < nlive && i >= c_lo) *Dp = v;
+            if (i < nlive) *Dp = v;
             Dp += ldd;
           }
         }
@@ -1273,7 +1271,7 @@ long long SplitEngine::gemm(const GemmDesc& g, cudaStream_t s, DevStatus* st,
     p.gchunk[gi] = (unsigned char)std::max(1, EXACT_TERMS / (SBK * gr.count));
   }
   const int np = S * (S + 1) / 2;  // digit-pair products per output tile and K term
-  p.triA = g.triA; p.triB = g.triB; p.outLower = g.outLower; p.outUpper = g.outUpper;
+  p.triA = g.triA; p.triB = g.triB; p.outLower = g.outLower;
   p.ldc = g.ldc; p.ldd = g.ldd; p.sC = g.sC; p.sD = g.sD;
   p.alpha = g.alpha; p.betac = g.beta;
   p.st = st;
@@ -1372,7 +1370,7 @@ long long SplitEngine::gemm(const GemmDesc& g, cudaStream_t s, DevStatus* st,
     int jobs = 0;  // jobs of a tile with the full K range
     for (int gi = 0; gi < p.ngroups; ++gi) jobs += (Kp / SBK + p.gchunk[gi] - 1) / p.gchunk[gi];
     p.ksplit = split_k((long long)ntiles * nbat, jobs);
-    dim3 grid(RpA / BM, RpB / BN, nbat * p.ksplit);
+    dim3 grid(ntiles, 1, nbat * p.ksplit);
     if (tensor_flops) {
       const double tiles = ntiles;  // tiles with nothing to write are skipped
       *tensor_flops += tiles * nbat * 2.0 * BM * BN * (double)round_up(Kp, SBK) * np;

@@ -464,7 +464,7 @@ int class_slices(const rgf_handle* h, const SplitEngine* eng, const GemmDesc& g,
   if (eng->may_slice(g, h->split_bias)) return own;
   GemmDesc full = g;
   full.triA = full.triB = TRI_NONE;
-  full.outLower = full.outUpper = 0;
+  full.outLower = 0;
   return fd == 1 && S <= EXACT && eng->may_slice(full, h->split_bias) ? EXACT : 0;
 }
 

@@ -118,8 +118,8 @@ enum Tri { TRI_NONE = 0, TRI_LOWER = 1, TRI_UPPER = 2 };
 
 // D = alpha * op(A) * op(B) + beta * C, column-major, op(A) m x k, op(B) k x n.
 // triA/triB declare a triangular operand (of op(X)); its other triangle is
-// treated as zero whatever memory holds.  outLower writes only r >= c,
-// outUpper only r <= c; output tiles with nothing to write are not computed.
+// treated as zero whatever memory holds.  outLower writes only r >= c; output
+// tiles with nothing to write are not computed.
 // batch > 1 runs independent problems offset by sA/sB/sC/sD elements.
 struct GemmDesc {
   int m = 0, n = 0, k = 0;
@@ -135,7 +135,7 @@ struct GemmDesc {
   const double* C = nullptr; long long ldc = 0;
   double* D = nullptr; long long ldd = 0;
   double alpha = 1.0, beta = 0.0;
-  int triA = TRI_NONE, triB = TRI_NONE, outLower = 0, outUpper = 0;
+  int triA = TRI_NONE, triB = TRI_NONE, outLower = 0;
   int batch = 1;
   long long sA = 0, sB = 0, sC = 0, sD = 0;
   int ksplit = 1;       // FP64 kernel: set by the launcher
@@ -145,14 +145,22 @@ struct GemmDesc {
 };
 
 // Whether the t x t output tile at (m0, n0) has anything to write.
-__host__ __device__ inline bool tile_written(int outLower, int outUpper, int m0, int n0, int t) {
-  return !(outLower && m0 + t <= n0) && !(outUpper && n0 + t <= m0);
+inline bool tile_written(int outLower, int m0, int n0, int t) { return !(outLower && m0 + t <= n0); }
+// The i-th of the written tiles, column by column (nx tiles to a full column).
+struct TilePos {
+  int x, y;
+};
+__device__ inline TilePos tile_at(int outLower, int nx, int i) {
+  if (!outLower) return {i % nx, i / nx};
+  int y = 0;
+  while (i >= nx - y) i -= nx - y++;
+  return {i + y, y};
 }
 // Number of t x t tiles of the m x n output that are written (one batch item).
 inline long long tiles_written(const GemmDesc& g, int t) {
   long long tiles = 0;
   for (int m0 = 0; m0 < g.m; m0 += t)
-    for (int n0 = 0; n0 < g.n; n0 += t) tiles += tile_written(g.outLower, g.outUpper, m0, n0, t);
+    for (int n0 = 0; n0 < g.n; n0 += t) tiles += tile_written(g.outLower, m0, n0, t);
   return tiles;
 }
 
