@@ -294,7 +294,7 @@ int rgf_batch_kernels(rgf_batch* b, long long* kernels);
  * algorithm or the operation count; each changes how it is cut into kernels:
  *   leaf_nb     how wide a diagonal tile of the panel factorization one launch
  *               factors (32-column FP64 leaves inside): 16 = 64 columns,
- *               32 or 64 = 128 columns;
+ *               32 or 64 = 128 columns, the last up to 160;
  *   lookahead   1 = the rows below each diagonal block are solved and updated
  *               on a second, lower-priority stream; 0 = one stream;
  *   split_bias  split precision: a product runs on the tensor cores when its

@@ -1,5 +1,5 @@
 // FP64 kernels of the panel factorization: the Cholesky of a diagonal tile of
-// up to 128 columns in one launch (a cluster of eight CTAs), and the triangular
+// up to 160 columns in one launch (a cluster of sixteen CTAs), and the triangular
 // solve of the rows below it.
 //
 // On GB300 an FP64 warp instruction holds its SM sub-partition's FP64 unit ~76
@@ -17,7 +17,6 @@ namespace rgf {
 namespace {
 
 constexpr int LB = PANEL_LEAF;                 // leaf width: 32
-constexpr int TW = PANEL_TILE;                 // tile width: 128
 constexpr int XPITCH = LB + 1;
 constexpr int LEAF_WARPS = 8;                  // of the leaf CTA's warps; one more sends
 constexpr int TILE_THREADS = (LEAF_WARPS + 1) * 32;
@@ -326,7 +325,7 @@ __device__ __forceinline__ void leaf_row_solve(double (&u)[LB / G], const double
   }
 }
 
-// ---- the tile: Cholesky of the w x w (w <= 128) lower tile at P ----------------
+// ---- the tile: Cholesky of the w x w (w <= 160) lower tile at P ----------------
 // Rank 0 (the leaf CTA) factors the 32-wide leaves one after another; NW
 // workers hold the tile's other rows (row 32 + rank - 1 + NW i each) in shared
 // memory.  Step k:
@@ -347,7 +346,7 @@ __device__ __forceinline__ void leaf_row_solve(double (&u)[LB / G], const double
 // with their row solves (15 us) and three small products took ~215 us;
 // factorization of ns = 128, nt = 10 in split precision 1.86 -> 0.88 ms, of
 // ns = 2000, nt = 4 17.1 -> 13.2 ms (11.7 ms launched directly).
-template <int NW>
+template <int NW, int TW>  // workers; widest tile
 __global__ void __launch_bounds__(TILE_THREADS, 5)
     panel_tile_kernel(double* P, long long lda, int w, double* ws, int col0, DevStatus* st,
                       int wait_polls) {
@@ -876,7 +875,8 @@ void launch_rows_g(double* X, int rows, const double* P, long long lda, int w, c
     case 1: launch_k(panel_rows_kernel<G, 1, NT>, grid, block, 0, s, X, rows, P, lda, w, ws); break;
     case 2: launch_k(panel_rows_kernel<G, 2, NT>, grid, block, 0, s, X, rows, P, lda, w, ws); break;
     case 3: launch_k(panel_rows_kernel<G, 3, NT>, grid, block, 0, s, X, rows, P, lda, w, ws); break;
-    default: launch_k(panel_rows_kernel<G, 4, NT>, grid, block, 0, s, X, rows, P, lda, w, ws); break;
+    case 4: launch_k(panel_rows_kernel<G, 4, NT>, grid, block, 0, s, X, rows, P, lda, w, ws); break;
+    default: launch_k(panel_rows_kernel<G, 5, NT>, grid, block, 0, s, X, rows, P, lda, w, ws); break;
   }
 }
 
@@ -885,28 +885,7 @@ void launch_rows_g(double* X, int rows, const double* P, long long lda, int w, c
 namespace {
 // Whether clusters of 16 CTAs of panel_tile_kernel can be resident on this device.
 bool wide_clusters() {
-  static const bool ok = [] {
-    auto* k = panel_tile_kernel<15>;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(16);
-    cfg.blockDim = dim3(TILE_THREADS);
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 16;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    return n >= 4;  // one per four GPCs or more: not only a corner of the chip
-  }();
+  static const bool ok = widest_cluster(panel_tile_kernel<15, PANEL_TILE>, 0, TILE_THREADS) == 16;
   return ok;
 }
 }  // namespace
@@ -919,8 +898,12 @@ void launch_panel_tile(double* P, long long lda, int w, double* ws, int col0, De
   const int polls = wait_polls > 0 ? wait_polls : LEAF_WAIT_POLLS;
   const bool wide = w > LB && wide_clusters();
   const dim3 n(w <= LB ? 1 : wide ? 16 : 8);
-  launch_k_cluster(wide ? panel_tile_kernel<15> : panel_tile_kernel<7>, n, dim3(TILE_THREADS), n, 0, s, P,
-                   lda, w, ws, col0, st, polls);
+  auto* kern = w <= PANEL_TILE - PANEL_LEAF
+                   ? (wide ? panel_tile_kernel<15, PANEL_TILE - PANEL_LEAF>
+                           : panel_tile_kernel<7, PANEL_TILE - PANEL_LEAF>)
+                   : (wide ? panel_tile_kernel<15, PANEL_TILE> : panel_tile_kernel<7, PANEL_TILE>);
+  if (wide) allow_wide_clusters(kern, 0);  // an attribute of the current device
+  launch_k_cluster(kern, n, dim3(TILE_THREADS), n, 0, s, P, lda, w, ws, col0, st, polls);
 }
 
 // G lanes a row and four or eight warps: 4 / 8 / 16 rows a CTA, the fewest that

@@ -531,8 +531,12 @@ void gemm(rgf_handle* h, const GemmDesc& g, int cls) {
   }
 }
 
-// Widest diagonal tile factored by one launch.
-int panel_width(const rgf_handle* h) { return h->nb == 16 ? PANEL_TILE / 2 : PANEL_TILE; }
+// Columns of a diagonal tile (one launch).  A last tile of up to 160 is not divided: a
+// narrow one costs its own launches (tile, rows, update: ~50 us at ns = 515 for three
+// columns; factorization at ns = 515, nt = 20 split 8.9 -> 8.3 ms).  160 throughout is
+// slower (ns = 2000, nt = 10 25.9 against 24.6: the rows' FP64 work grows with the width).
+int panel_width(const rgf_handle* h) { return h->nb == 16 ? 64 : 128; }
+int panel_last(const rgf_handle* h) { return h->nb == 16 ? 64 : PANEL_TILE; }
 
 double* panel_ws(rgf_handle* h, int off) {
   return h->d_panel_ws + (long long)(off / panel_width(h)) * PANEL_WS;
@@ -578,7 +582,7 @@ void trsm_rows(rgf_handle* h, double* X, long long xrs, long long xcs, int rows,
 // TRSM of the rows below folded in (RGF.H:254-260, 284-287, 312-317, 335 as
 // one pass).  Halving the column range makes every trailing update one GEMM
 // with an inner dimension of half the range, so most of the work runs in a
-// few large products; 128-column tiles are factored in FP64 by one launch
+// few large products; tiles of 128 (the last one up to 160) columns are factored in FP64 by one launch
 // (panel_tile_kernel) and the rows below them solved by another.
 // off: first column of P within the diagonal block.
 //
@@ -591,9 +595,9 @@ void trsm_rows(rgf_handle* h, double* X, long long xrs, long long xcs, int rows,
 void panel_potrf(rgf_handle* h, double* P, long long lda, int rows, int cols, int dr, int off,
                  int col0) {
   const int nb = panel_width(h);
-  const bool la = h->lookahead && h->side && !(off == 0 && dr <= nb);
+  const bool la = h->lookahead && h->side && !(off == 0 && dr <= panel_last(h));
   const int split_row = la ? dr : rows;  // rows at or past this go to the side stream
-  if (cols <= nb) {
+  if (cols <= panel_last(h)) {
     panel_tile(h, P, lda, cols, off, col0);
     panel_rows(h, P + cols, split_row - cols, P, lda, cols, off);
     if (rows > split_row) {
@@ -1458,8 +1462,7 @@ int rgf_create(const size_t* ia, const size_t* ja, const double* a, size_t ns, s
     if ((st = dalloc(h, &h->d_scalars, 8))) break;
     if ((st = dalloc(h, &h->d_diag, n))) break;
     if ((st = dalloc(h, &h->d_status, 1))) break;
-    if ((st = dalloc(h, &h->d_panel_ws, (std::max(ns, nd) + PANEL_TILE / 2 - 1) / (PANEL_TILE / 2) *
-                                            PANEL_WS))) break;
+    if ((st = dalloc(h, &h->d_panel_ws, (std::max(ns, nd) + 63) / 64 * PANEL_WS))) break;
     if (nd > 0 && nd <= ARROW_SYRK_MAX_ND &&
         (st = dalloc(h, &h->d_arrow, arrow_syrk_elems(h->sh))))
       break;

@@ -189,7 +189,7 @@ int launch_gemm_fp64(const GemmDesc& g, cudaStream_t s);
 // (0 = LEAF_WAIT_POLLS); a wait that runs out records a timeout in st and the
 // tile's leaves stop updating.  ws (PANEL_WS doubles) receives what
 // launch_panel_rows reads: per 32-column leaf its unit columns, then d^{-1/2}.
-constexpr int PANEL_LEAF = 32, PANEL_TILE = 128;
+constexpr int PANEL_LEAF = 32, PANEL_TILE = 160;
 constexpr int PANEL_LEAF_WS = PANEL_LEAF * PANEL_LEAF + PANEL_LEAF;
 constexpr int PANEL_WS = PANEL_TILE / PANEL_LEAF * PANEL_LEAF_WS;
 constexpr int LEAF_WAIT_POLLS = 1 << 26;

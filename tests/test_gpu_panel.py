@@ -76,3 +76,9 @@ def test_column_of_a_non_positive_pivot(rgf, col):
             s.factorize()
         assert e.value.status == 3
         assert s.info()["not_spd_column"] == col
+
+
+@pytest.mark.parametrize("ns", [130, 159, 161, 255, 287, 288, 289, 416, 417])
+@pytest.mark.parametrize("nd", [0, 3, 150, 161])
+def test_last_tiles_past_128(rgf, ns, nd):
+    _check(rgf, ns, 2, nd)
