@@ -18,6 +18,12 @@ struct DevStatus {
   int pad;
 };
 
+// What the host reads after a stage, in one copy.
+struct DevResults {
+  DevStatus status;
+  double scalars[8];  // [0] logdet, [1] ||r||, [2] ||b||
+};
+
 // ---- programmatic dependent launch -------------------------------------------
 // Kernels are launched with programmatic stream serialization (launch_k): the
 // next kernel in a stream may be scheduled once every CTA of the running one
