@@ -66,6 +66,7 @@ struct rgf_handle {
   double* d_U = nullptr;     // Linv^T of every diagonal block (ns x ns each), then the corner
   double* d_T1 = nullptr;    // ns x ns (compat recursion)
   double* d_T2 = nullptr;    // ns x ns (compat recursion)
+  double* d_far = nullptr;   // inverse of a column group and its scratch (far_product)
   double* d_K = nullptr;     // k_chunk blocks of (ns + nd) x ns
   double* d_S = nullptr;     // (ns + nd) x (ns + nd)
   long long k_chunk = 0;     // blocks whose K_i is formed at once
@@ -406,6 +407,9 @@ void dfree(void* p) { device_free(p); }
 // BULK1: as BULK, one slice more (U U^T, whose operands' truncations are the same and
 // so add up instead of averaging out: 1.4 times the error of a product of two
 // different operands at equal slices).
+// Column groups of the diagonal block (see far_by_inverse): most columns, and fewest rows
+// below the diagonal block.
+constexpr int FAR_GROUP = 512, FAR_MIN_ROWS = 1450;
 enum GemmClass { SMALL = 0, BULK = 1, DIAG = 2, BULK1 = 3 };
 
 cudaStream_t cur_stream(const rgf_handle* h) { return h->on_side ? h->side : h->stream; }
@@ -579,6 +583,40 @@ void trsm_rows(rgf_handle* h, double* X, long long xrs, long long xcs, int rows,
   }
 }
 
+void issue_trtri(rgf_handle* h, double* U, long long ldu, long long n, const double* L,
+                 long long ldl, double* Tmp, long long ldt, int batch, long long sU, long long sL,
+                 long long sT, bool leaves = true);
+
+// The block rows below the diagonal block, X L^T = B for a group of `cols` columns of it,
+// as one product with the group's inverse: X := X U, U = L_gg^{-T}, in place (the split
+// engine has cut X into digits before it writes).
+GemmDesc far_product(rgf_handle* h, double* X, long long lda, int m, int cols) {
+  GemmDesc g;
+  g.m = m; g.n = g.k = cols;
+  g.A = X; g.lda = lda;
+  g.B = h->d_far; g.ldb = cols; g.triB = TRI_UPPER;
+  g.D = X; g.ldd = lda;
+  g.alpha = 1.0; g.beta = 0.0;
+  return g;
+}
+
+// Whether a group of columns takes that way: with 7-slice products (FP64-accurate
+// emulation) where the split engine is the faster one for them, and never for the last
+// columns of a diagonal block, whose inverse would stand between them and the next
+// block.  The row solves of a group are FP64 work (m cols^2 / 2 FMAs) that the diagonal
+// block's own row solves wait for: factorization at ns = 2000, nt = 10 24.6 -> 22.1 ms,
+// ns = 1750, nt = 8 15.9 -> 14.8, ns = 1500 12.6 -> 12.3; at ns = 1250 12.1 -> 12.5, so the
+// line lies between.
+bool far_by_inverse(rgf_handle* h, int m, int cols, int dr) {
+  if (!h->d_far || cols > FAR_GROUP || cols <= panel_last(h) || dr <= cols || m < FAR_MIN_ROWS ||
+      h->opts.fp64_diag != 1)
+    return false;
+  h->on_side = true;
+  const bool ok = routed_slices(h, far_product(h, h->d_MF, 1, m, cols), DIAG) > 0;
+  h->on_side = false;
+  return ok;
+}
+
 // ---- panel Cholesky: [D; B; C] (rows x cols, lda) -> [L; B L^-T; C L^-T] ----
 // Recursive (left half first) Cholesky of the top cols x cols block with the
 // TRSM of the rows below folded in (RGF.H:254-260, 284-287, 312-317, 335 as
@@ -599,6 +637,15 @@ void panel_potrf(rgf_handle* h, double* P, long long lda, int rows, int cols, in
   const int nb = panel_width(h);
   const bool la = h->lookahead && h->side && !(off == 0 && dr <= panel_last(h));
   const int split_row = la ? dr : rows;  // rows at or past this go to the side stream
+  if (rows > split_row && far_by_inverse(h, rows - dr, cols, dr)) {
+    panel_potrf(h, P, lda, dr, cols, dr, off, col0);
+    fork_side(h);
+    h->on_side = true;
+    issue_trtri(h, h->d_far, cols, cols, P, lda, h->d_far + (long long)cols * cols, cols, 1, 0, 0, 0);
+    gemm(h, far_product(h, P + dr, lda, rows - dr, cols), DIAG);
+    h->on_side = false;
+    return;
+  }
   if (cols <= panel_last(h)) {
     panel_tile(h, P, lda, cols, off, col0);
     panel_rows(h, P + cols, split_row - cols, P, lda, cols, off);
@@ -734,43 +781,62 @@ void issue_factor(rgf_handle* h) {
   h->kernels_issued += 2;
 }
 
+// One step of the inverse below: U12 = -U11 (L21^T U22) for `batch` pairs of diagonal
+// sub-blocks of n1 and n2 columns, the first of them at U, L and T.
+void trtri_pairs(rgf_handle* h, double* U, long long ldu, long long n1, long long n2,
+                 const double* L, long long ldl, double* T, long long ldt, int batch, long long sU,
+                 long long sL, long long sT) {
+  GemmDesc a;  // T12 = L21^T U22
+  a.m = (int)n1; a.n = (int)n2; a.k = (int)n2;
+  a.A = L + n1; a.lda = ldl; a.transA = 1;
+  a.B = U + n1 + n1 * ldu; a.ldb = ldu; a.triB = TRI_UPPER;
+  a.D = T + n1 * ldt; a.ldd = ldt; a.alpha = 1.0; a.beta = 0.0;
+  a.batch = batch; a.sA = sL; a.sB = sU; a.sD = sT;
+  gemm(h, a, DIAG);
+  GemmDesc b;  // U12 = -U11 T12
+  b.m = (int)n1; b.n = (int)n2; b.k = (int)n1;
+  b.A = U; b.lda = ldu; b.triA = TRI_UPPER;
+  b.B = T + n1 * ldt; b.ldb = ldt;
+  b.D = U + n1 * ldu; b.ldd = ldu; b.alpha = -1.0; b.beta = 0.0;
+  b.batch = batch; b.sA = sU; b.sB = sT; b.sD = sU;
+  gemm(h, b, DIAG);
+}
+
 // For `batch` diagonal blocks at once: U = L^{-T} (upper triangular).
-// Recursive halving: with L = [L11 0; L21 L22], U = [U11 U12; 0 U22] where
-// U11 = L11^{-T}, U22 = L22^{-T} and U12 = -U11 (L21^T U22).  The two halves
-// are independent; each level adds two GEMMs with an inner dimension of half
-// the range, batched over all blocks, so the inverse runs as a few large
-// products (DIAG class: FP64 or FP64-accurate split).  Leaves (<= 64) solve
-// X L^T = I row-parallel, all of them at once.  T (the product L21^T U22) lives in Tmp at the
-// position of U12.
+// With L = [L11 0; L21 L22], U = [U11 U12; 0 U22] where U11 = L11^{-T}, U22 = L22^{-T} and
+// U12 = -U11 (L21^T U22).  Leaves (<= 64) solve X L^T = I row-parallel, all of them at
+// once; then two GEMMs a level (DIAG class: FP64 or FP64-accurate split), batched over
+// all blocks, by recursive halving.  A single block's levels double instead (64, 128,
+// ...) and each takes its pairs as one batch: 6 products for 512 columns instead of
+// 14 (265 -> ~135 us beside a factorization).  T (the product L21^T U22) lives in Tmp
+// at the position of U12.
 void issue_trtri(rgf_handle* h, double* U, long long ldu, long long n, const double* L,
                  long long ldl, double* Tmp, long long ldt, int batch, long long sU, long long sL,
-                 long long sT, bool leaves = true) {
+                 long long sT, bool leaves) {
   if (batch <= 0 || n <= 0) return;
   if (leaves) {  // all <= 64-column leaves in one launch
     launch_leaf_inverses(U, ldu, (int)n, L, ldl, batch, sU, sL, cur_stream(h));
     h->kernels_issued++;
     trace(h, "leaf inverses");
   }
+  if (batch == 1) {
+    for (long long w = NB; w < n; w *= 2) {
+      const long long full = n / (2 * w), o = full * 2 * w, rest = n - o - w;
+      if (full > 0)
+        trtri_pairs(h, U, ldu, w, w, L, ldl, Tmp, ldt, (int)full, 2 * w * (ldu + 1),
+                    2 * w * (ldl + 1), 2 * w * (ldt + 1));
+      if (rest > 0)
+        trtri_pairs(h, U + o * (ldu + 1), ldu, w, rest, L + o * (ldl + 1), ldl, Tmp + o * (ldt + 1),
+                    ldt, 1, 0, 0, 0);
+    }
+    return;
+  }
   if (n <= NB) return;
   const long long n1 = ((n / 2 + NB - 1) / NB) * NB, n2 = n - n1;
   issue_trtri(h, U, ldu, n1, L, ldl, Tmp, ldt, batch, sU, sL, sT, false);
-  issue_trtri(h, U + n1 + n1 * ldu, ldu, n2, L + n1 + n1 * ldl, ldl, Tmp + n1 + n1 * ldt, ldt,
+  issue_trtri(h, U + n1 * (ldu + 1), ldu, n2, L + n1 * (ldl + 1), ldl, Tmp + n1 * (ldt + 1), ldt,
               batch, sU, sL, sT, false);
-  double* T = Tmp + n1 * ldt;
-  GemmDesc a;  // T = L21^T U22
-  a.m = (int)n1; a.n = (int)n2; a.k = (int)n2;
-  a.A = L + n1; a.lda = ldl; a.transA = 1;
-  a.B = U + n1 + n1 * ldu; a.ldb = ldu; a.triB = TRI_UPPER;
-  a.D = T; a.ldd = ldt; a.alpha = 1.0; a.beta = 0.0;
-  a.batch = batch; a.sA = sL; a.sB = sU; a.sD = sT;
-  gemm(h, a, DIAG);
-  GemmDesc b;  // U12 = -U11 T
-  b.m = (int)n1; b.n = (int)n2; b.k = (int)n1;
-  b.A = U; b.lda = ldu; b.triA = TRI_UPPER;
-  b.B = T; b.ldb = ldt;
-  b.D = U + n1 * ldu; b.ldd = ldu; b.alpha = -1.0; b.beta = 0.0;
-  b.batch = batch; b.sA = sU; b.sB = sT; b.sD = sU;
-  gemm(h, b, DIAG);
+  trtri_pairs(h, U, ldu, n1, n2, L, ldl, Tmp, ldt, batch, sU, sL, sT);
 }
 
 GemmDesc mk(int m, int n, int k, const double* A, long long lda, int tA, const double* B,
@@ -1335,7 +1401,7 @@ void release(rgf_handle* h) {
   if (h->trace_t0) cudaEventDestroy(h->trace_t0);
   delete h->split;
   delete h->split_side;
-  void* bufs[] = {h->d_ia, h->d_ja, h->d_a, h->d_MF, h->d_MS, h->d_U, h->d_T1, h->d_T2, h->d_T3, h->d_K, h->d_S,
+  void* bufs[] = {h->d_ia, h->d_ja, h->d_a, h->d_MF, h->d_MS, h->d_U, h->d_T1, h->d_T2, h->d_T3, h->d_K, h->d_S, h->d_far,
                   h->d_logpart, h->d_diag, h->d_results, h->d_rhs, h->d_partial,
                   h->d_res, h->d_ref, h->d_rhs2,
                   h->d_norms, h->d_panel_ws, h->d_arrow};
@@ -1501,6 +1567,9 @@ int rgf_create(const size_t* ia, const size_t* ja, const double* a, size_t ns, s
       if (st) break;
       st = h->split_side->prepare((int)(ns + nd), (int)ns, 1);
       if (st) break;
+      if ((long long)(ns + nd) >= FAR_MIN_ROWS && nt > 1 &&
+          (st = dalloc(h, &h->d_far, 2 * FAR_GROUP * FAR_GROUP)))
+        break;
     }
     if (async) {  // copies and ingests overlap the first factorization
       st = start_upload(h, ia, ja, a);

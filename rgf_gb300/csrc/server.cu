@@ -56,6 +56,7 @@ size_t estimate_bytes(const rgf_opts& o, size_t ns, size_t nt, size_t nd, size_t
     b += std::max(one, std::min<size_t>((size_t)1 << 30, nt * one / 4)) + (1 << 20);
     const size_t r2 = (ns + nd + 127) / 128 * 128;
     b += 2 * 8 * r2 * k * 2 + (1 << 20);
+    b += 4 << 20;  // inverses of column groups (large blocks)
   }
   return b + (8u << 20);
 }

@@ -52,3 +52,29 @@ def test_split_lines(rgf, ns, nd):
 
 def test_batches_of_k(rgf):
     _check(rgf, 1500, 10, 3)
+
+
+@pytest.mark.parametrize("ns,nt,nd", [(1450, 2, 0), (1460, 3, 2), (1664, 2, 6)])
+def test_column_groups(rgf, ns, nt, nd):
+    """Blocks large enough that the rows below them are solved by group inverses: the
+    factor's entries too (bulk products at 5 slices, as above)."""
+    ia, ja, a = gen.generate_bta(ns, nt, nd, seed=ns + nd)
+    layout = O.Layout(ns, nt, nd)
+    MF = O.ingest(layout, ia, ja, a)
+    O.factorize(layout, MF)
+    _, want = O.selinv_exact(layout, MF, blocks=True)
+    tol = 16 * (ns + nd) * EPS + 4 * 2.0 ** (3 - 8 * 5) * (ns + nd)
+    with rgf.RGF(ia, ja, a, ns, nt, nd, precision="split") as s:
+        for _ in range(3):
+            s.factorize()
+            got = s.export_factor()
+            pos = 0
+            for i in range(nt):
+                lda = (2 * ns if i < nt - 1 else ns) + nd
+                keep = np.arange(lda)[None, :] >= np.arange(ns)[:, None]
+                g = got[pos:pos + lda * ns].reshape(ns, lda)[keep]
+                w = MF[pos:pos + lda * ns].reshape(ns, lda)[keep]
+                assert np.max(np.abs(g - w)) <= tol * np.max(np.abs(w))
+                pos += lda * ns
+            sig = s.export_selinv()
+            assert np.max(np.abs(sig - want)) <= tol * np.max(np.abs(want))
