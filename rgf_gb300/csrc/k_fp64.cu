@@ -44,7 +44,7 @@ __device__ __forceinline__ GemmTileRange k_range(const GemmDesc& g, int m0, int 
 // SM retires only ~3.5 FP64 flops per cycle, so a small product on few SMs
 // is slow however short it is).
 template <int TM, int TK>
-__global__ void __launch_bounds__(128) gemm_fp64_kernel(GemmDesc g) {
+__global__ void __launch_bounds__(128, TM == 64 ? 3 : 8) gemm_fp64_kernel(GemmDesc g) {
   constexpr int F = TM / 16;             // 8 x 8 fragments per warp side
   constexpr int LPT = TM * TK / 128;     // elements per thread per operand and stage
   constexpr int PAD = TM + 4;
@@ -175,12 +175,28 @@ __global__ void __launch_bounds__(128) gemm_fp64_kernel(GemmDesc g) {
 #pragma unroll
         for (int e = 0; e < 2; ++e)
           smem[(wn + j * 8 + (lane & 3) * 2 + e) * TM + wm + i * 8 + (lane >> 2)] = acc[i][j][e];
-    cluster_sync();
     const int share = (TM * TM / 128 + g.ksplit - 1) / g.ksplit;  // passes of 128 elements
     constexpr int U = 4;                                          // passes in flight
+    // only the passes there are issue FP64 instructions, alpha = +-1 takes none, and C is
+    // on its way before the exchange (selected inversion at ns = 128, nt = 40 1.75 -> 1.69
+    // ms, ns = 333, nt = 17 4.69 -> 4.64)
+    bool met = false;
 #pragma unroll 1
     for (int q0 = 0; q0 < share; q0 += U) {
-      double v[U] = {};
+      const int nu = min(U, share - q0);
+      double v[U] = {}, cv[U];
+      double* out[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int idx = (kz * share + q0 + u) * 128 + tid;
+        const int r = m0 + idx % TM, c = n0 + idx / TM;
+        const bool ok = u < nu && idx < TM * TM && r < g.m && c < g.n && !(g.outLower && r < c);
+        out[u] = ok ? (r < mD1 ? D : D2) + (long long)r + (long long)c * g.ldd : nullptr;
+        cv[u] = 0.0;
+        if (ok && g.beta != 0.0) cv[u] = (r < mD1 ? C : C2)[(long long)r + (long long)c * g.ldc];
+      }
+      if (!met) cluster_sync();
+      met = true;
 #pragma unroll 4
       for (int z = 0; z < g.ksplit; ++z) {
         double w[U];
@@ -188,19 +204,30 @@ __global__ void __launch_bounds__(128) gemm_fp64_kernel(GemmDesc g) {
         for (int u = 0; u < U; ++u)
           w[u] = ld_cluster(smem + min((kz * share + q0 + u) * 128 + tid, TM * TM - 1), z);
 #pragma unroll
-        for (int u = 0; u < U; ++u) v[u] += w[u];
+        for (int u = 0; u < U; ++u) {
+          if (u >= nu) break;
+          v[u] += w[u];
+          __syncwarp();
+        }
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int idx = (kz * share + q0 + u) * 128 + tid;
-        const int r = m0 + idx % TM, c = n0 + idx / TM;
-        if (q0 + u >= share || idx >= TM * TM || r >= g.m || c >= g.n || (g.outLower && r < c))
-          continue;
-        double x = g.alpha * v[u];
-        if (g.beta != 0.0) x += g.beta * (r < mD1 ? C : C2)[(long long)r + (long long)c * g.ldc];
-        (r < mD1 ? D : D2)[(long long)r + (long long)c * g.ldd] = x;
+        if (u >= nu) break;
+        double x = v[u];
+        if (g.alpha == -1.0) {
+          x = -x;
+        } else if (g.alpha != 1.0) {
+          x *= g.alpha;
+          __syncwarp();
+        }
+        if (g.beta != 0.0) {
+          x = fma(g.beta, cv[u], x);
+          __syncwarp();
+        }
+        if (out[u]) *out[u] = x;
       }
     }
+    __syncwarp();
     cluster_sync();  // a CTA's sums are read until every CTA is here
     return;
   }
