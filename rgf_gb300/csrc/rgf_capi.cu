@@ -853,8 +853,8 @@ GemmDesc mk(int m, int n, int k, const double* A, long long lda, int tA, const d
 
 // U_i = L_ii^{-T} of every diagonal block and of the corner, as one batched
 // recursive TRTRI (the blocks are independent once the factor exists); MS is
-// the recursion's scratch.  Only the upper triangles are written: every product
-// declares U triangular.
+// the recursion's scratch.  Only the upper triangles and the 64 x 64 diagonal tiles
+// are written: a product with a larger U declares it triangular.
 void issue_inverses(rgf_handle* h) {
   const BtaShape& sh = h->sh;
   const long long ns = sh.ns, nt = sh.nt, nd = sh.nd;
@@ -892,7 +892,12 @@ void issue_selinv(rgf_handle* h) {
   issue_inverses(h);
   if (nd > 0) {
     // Sigma_dd = L_dd^{-T} L_dd^{-1} = U_d U_d^T   (RGF.H:439-442)
-    gemm(h, mk(ind, ind, ind, Ud, nd, 0, Ud, nd, 1, nullptr, 0, Sdd, nd, 1.0, 0.0), SMALL);
+    GemmDesc d = mk(ind, ind, ind, Ud, nd, 0, Ud, nd, 1, nullptr, 0, Sdd, nd, 1.0, 0.0);
+    if (ind > NB) {  // past one leaf tile U_d's lower triangle is not written (nor zeroed)
+      d.triA = TRI_UPPER;
+      d.triB = TRI_LOWER;
+    }
+    gemm(h, d, SMALL);
   }
   const bool compat = h->opts.selinv_mode == RGF_SELINV_COMPAT;
   const int m2 = ins + ind;
