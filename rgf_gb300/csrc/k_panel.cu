@@ -73,7 +73,11 @@ __device__ __forceinline__ double recip_pos(double d) {
 // by its high word; a value with that high word (a NaN) is stored as the
 // canonical NaN.  Polls are bounded by `polls` (the bound is the only thing a poll loop
 // counts: it has to turn around in a few cycles); one that runs out records a
-// timeout and sets abort_, after which the CTA's later leaves are skipped.
+// timeout and sets abort_, after which the CTA's later leaves are skipped and a
+// thread's later polls in the same leaf end at once.  abort_ may be set at any
+// time by a warp whose own wait ran out, so whatever stands before a barrier
+// is decided from one reduction over all the barrier's threads (bar_any_leaf within
+// a leaf, __syncthreads_or after it), never from a warp's own read.
 constexpr int UNSET_HI = 0x7ff85e5e;
 constexpr unsigned long long CANON_NAN = 0x7ff8000000000000ull;
 
@@ -104,7 +108,7 @@ __device__ __forceinline__ void sts_slot(unsigned addr, double v) {
 }
 __device__ __forceinline__ double lds_wait(unsigned addr, const Wait& w, bool& over) {
   double v = lds_peek(addr);
-  int left = w.polls;
+  int left = over ? 0 : w.polls;
 #pragma unroll 1
   while (slot_empty(v)) {
     if (--left <= 0) {
@@ -154,7 +158,7 @@ __device__ __forceinline__ void leaf_half(const double (*S)[LB], double (*V)[LB]
   // a -= column j times column c's multiplier l_cj
   auto step = [&](double a, int j, int c) {
     double l, v;
-    int left = w.polls;
+    int left = over ? 0 : w.polls;
 #pragma unroll 1
     for (;;) {
       l = lds_peek(sl + j * ROW + c * 8);
@@ -198,6 +202,15 @@ __device__ __forceinline__ void leaf_half(const double (*S)[LB], double (*V)[LB]
 __device__ __forceinline__ void bar_sync_leaf() {
   asm volatile("bar.sync 1, %0;" ::"n"(LEAF_WARPS * 32) : "memory");
 }
+// the same; whether any of their threads brought `stop`: all of them get one answer
+__device__ __forceinline__ bool bar_any_leaf(bool stop) {
+  int any;
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.s32 p, %1, 0;\n bar.red.or.pred q, 1, %2, p;\n"
+      " selp.s32 %0, 1, 0, q;\n}"
+      : "=r"(any) : "r"((int)stop), "n"(LEAF_WARPS * 32) : "memory");
+  return any != 0;
+}
 
 // S(r, c) -= sum_{j < 16} V_rj l_cj over the lower elements 16 <= c <= r < 32 of the
 // second half (136 of them; the terms are summed before they meet S, here and in
@@ -238,8 +251,7 @@ __device__ __forceinline__ void leaf_ldl(double (*S)[LB], double (*V)[LB], doubl
 #pragma unroll 1
   for (int b0 = 0; b0 < nbk; b0 += LB / 2) {
     if (b0 > 0) {
-      bar_sync_leaf();
-      if (*w.abort_) return;
+      if (bar_any_leaf(*w.abort_ != 0)) return;
       leaf_trailing(S, V, Lc);
       bar_sync_leaf();
     }
@@ -383,13 +395,14 @@ __global__ void __launch_bounds__(TILE_THREADS, 5)
     for (int e = tid; e < LB * LB; e += TILE_THREADS) bufB[e] = unset;
     __syncthreads();
     if (nl > 1) { cluster_arrive(); cluster_wait(); }
+    bool stop = false;
     for (int k = 0; k < nl; ++k) {
       const int nbk = min(LB, w - k * LB);
-      if (!*wait.abort_) {
+      if (!stop) {
         if (warp < LEAF_WARPS) leaf_ldl(S, V, Lc, nbk, &sh, wait);
         else leaf_send<NW>(V, Lc, ys, nbk, wait, k + 1 < nl);
       }
-      __syncthreads();
+      stop = __syncthreads_or(*wait.abort_);
       if (k + 1 < nl) cluster_arrive();  // (workers: rows solved)
       else pdl_trigger();                // the next kernel's CTAs may come in
       // results: L = V d^{-1/2} to P, the unit columns and d^{-1/2} to ws
@@ -429,6 +442,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 5)
   __syncthreads();
   cluster_arrive();
   cluster_wait();
+  bool stop = false;
   for (int k = 0; k + 1 < nl; ++k) {
     const int kc = k * LB, kn = kc + LB;          // this leaf's and the next one's first column
     {  // solve: WG lanes a row, 32 / WG rows a warp
@@ -436,7 +450,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 5)
       const int q = lane & (WG - 1), i = warp * (32 / WG) + lane / WG;
       const int r = row0 + NW * i;
       const bool live = i < nown && r >= kn;
-      if (warp < LEAF_WARPS && !*wait.abort_ && __any_sync(0xffffffffu, live)) {
+      if (warp < LEAF_WARPS && !stop && __any_sync(0xffffffffu, live)) {
         bool over = false;
         double u[SL];
 #pragma unroll
@@ -459,7 +473,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 5)
         if (over) wait_gave_up(wait);
       }
     }
-    __syncthreads();
+    stop = __syncthreads_or(*wait.abort_);
     clear_slots();
     __syncthreads();
     cluster_arrive();
@@ -715,6 +729,7 @@ __global__ void __launch_bounds__(CHAIN_THREADS)
   __syncthreads();
   cluster_sync();  // every CTA is here before the first remote store
 
+  bool stop = false;
   for (long long i = 0; i < nt; ++i) {
     const bool last = i == nt - 1;
     double* P = MF + i * sP;
@@ -736,7 +751,7 @@ __global__ void __launch_bounds__(CHAIN_THREADS)
 #pragma unroll 1
     for (int k = 0; k < nl; ++k) {
       const int kc = k * LB, nbk = min(LB, ns - kc);
-      if (!*wait.abort_) {
+      if (!stop) {
         if (warp < LEAF_WARPS) {
           leaf_ldl(S, V, Lc, nbk, &sh, wait);
         } else if (warp == LEAF_WARPS) {
@@ -779,7 +794,7 @@ __global__ void __launch_bounds__(CHAIN_THREADS)
           }
         }
       }
-      __syncthreads();
+      stop = __syncthreads_or(*wait.abort_);
       cluster_arrive();
       // L = V d^{-1/2}: each CTA writes its share of the leaf's columns
       for (int c = rank + nc * warp; c < nbk; c += nc * (CHAIN_THREADS / 32))
