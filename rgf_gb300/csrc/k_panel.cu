@@ -27,20 +27,15 @@ __device__ __forceinline__ bool positive_bits(double d) {
   return b > 0 && b <= 0x7ff0000000000000ll;
 }
 
-// 1 / d of a positive double (within 2^-62 relative before the final rounding)
-// in integer arithmetic: no FP64 instruction on the pivot chain.  d = m 2^e with m
-// in [1, 2); y0 is an FP32 reciprocal of m's leading 24 bits (|1 - m y0| < 2^-22);
-// with e = 1 - m y0 exact to 2^-62, one cubic step 1/m = y0 + y0 e + y0 e^2 leaves an
-// error of e^3 < 2^-66.  Its dependent steps are single 32-bit operations and
+// 2 / m of a normal positive double d = m 2^e, m in [1, 2) (within 2^-62 relative before
+// the final rounding) in integer arithmetic: no FP64 instruction on the pivot chain.
+// y0 is an FP32 reciprocal of m's leading 24 bits (|1 - m y0| < 2^-22);
+// with t = 1 - m y0 exact to 2^-62, one cubic step 1/m = y0 + y0 t + y0 t^2 leaves an
+// error of t^3 < 2^-66.  Its dependent steps are single 32-bit operations and
 // 32 x 32 -> 64 multiplications: ~150 cycles, where FP32 double-float refinement and
-// two FP64 operations took ~230 and a reciprocal square root 454.  A d that is not
-// positive gives NaN.
-__device__ __noinline__ double recip_slow(double d) {  // not positive: NaN
-  return positive_bits(d) ? 1.0 / d : __longlong_as_double(0x7ff8000000000000ll);
-}
-__device__ __forceinline__ double recip_pos(double d) {
+// two FP64 operations took ~230 and a reciprocal square root 454.
+__device__ __forceinline__ double recip_significand(double d) {
   const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
-  const unsigned ex = hi >> 20;
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;"
       : "=f"(y)
@@ -50,20 +45,51 @@ __device__ __forceinline__ double recip_pos(double d) {
   const unsigned Y0 = (min(__float_as_uint(y), 0x3f7fffffu) << 8) | 0x80000000u;
   const int Y31 = (int)(Y0 >> 1);
   const unsigned long long P = (unsigned long long)Mh * Y0 + __umulhi(Ml, Y0);  // m y0 2^63
-  const long long E = (long long)(0x8000000000000000ull - P);                  // e 2^63
-  const int Eh = (int)(E >> 20);                                               // e 2^43
+  const long long E = (long long)(0x8000000000000000ull - P);                  // t 2^63
+  const int Eh = (int)(E >> 20);                                               // t 2^43
   const int El = (int)(((unsigned)E & 0xfffffu) << 1);                         // rest, 2^64
-  const int E2 = __mulhi((int)(E >> 10), Eh);                                  // e^2 2^64
+  const int E2 = __mulhi((int)(E >> 10), Eh);                                  // t^2 2^64
   const long long A = (long long)Y31 * Eh;                                     // 2^74
   const long long D = (long long)Y31 * El + (long long)Y31 * E2;               // 2^95
   // 1/m 2^63 plus half a unit of the 53 bits kept
   const unsigned long long Y1 = (((unsigned long long)Y0 << 31) + 512) +
                                 (unsigned long long)(A >> 11) +
                                 (unsigned long long)(long long)(int)(D >> 32);
-  const double r = __longlong_as_double(
-      (long long)(((unsigned long long)(2044u - ex) << 52) + (Y1 >> 10)));
-  // subnormal d or result, infinity, not positive
-  return hi - 0x100000u < 0x7f800000u ? r : recip_slow(d);
+  return __longlong_as_double((long long)((1022ull << 52) + (Y1 >> 10)));
+}
+// the high word of 2^-(e + 1) less that of 1: added to another high word, it scales by it
+__device__ __forceinline__ unsigned half_recip_power(double d) {
+  return 0x3fe00000u - ((unsigned)__double2hiint(d) & 0x7ff00000u);
+}
+
+// x / d; NaN for a d that is not positive
+__device__ __noinline__ double over_pivot_slow(double x, double d) {
+  return positive_bits(d) ? x / d : __longlong_as_double(0x7ff8000000000000ll);
+}
+__device__ __forceinline__ double over_pivot(double x, double d) {
+  const double r = recip_significand(d);
+  // 1 / d has to be normal: 2^-1022 <= d < 2^1017
+  if ((unsigned)__double2hiint(d) - 0x100000u >= 0x7f800000u) return over_pivot_slow(x, d);
+  return x * __hiloint2double(__double2hiint(r) + (int)half_recip_power(d), __double2loint(r));
+}
+// a - v w / d.  The product of two entries of unscaled columns has the square of the
+// matrix's magnitude, so w first gives up d's power of two (in its exponent field,
+// beside the reciprocal): |v w / d| is at most that of a's row and column.  d and |w|
+// between 2^-503 and 2^517 take that way (two range tests: every instruction of the
+// leaf's loops counts); of the others a zero w has no term, the rest divide.
+__device__ __forceinline__ double minus_term(double a, double v, double w, double d) {
+  constexpr unsigned LO = 520u << 20, RANGE = 1020u << 20;
+  const unsigned dh = (unsigned)__double2hiint(d), wh = (unsigned)__double2hiint(w);
+  const double p = v * __hiloint2double((int)(wh + half_recip_power(d)), __double2loint(w));
+  double x = fma(-p, recip_significand(d), a);
+  asm volatile("" : "+d"(x));  // the rare branch stands behind the chain, not in it
+  if (max(dh - LO, (wh & 0x7fffffffu) - LO) >= RANGE) {
+    const bool no_term = dh - LO < RANGE && ((wh << 1) | (unsigned)__double2loint(w)) == 0 &&
+                         ((unsigned)__double2hiint(v) & 0x7fffffffu) < 0x7ff00000u;
+    x = a;
+    if (!no_term) x = fma(-v, over_pivot_slow(w, d), a);
+  }
+  return x;
 }
 
 // ---- hand-off of doubles through shared memory -----------------------------------
@@ -124,7 +150,9 @@ __device__ __forceinline__ double lds_wait(unsigned addr, const Wait& w, bool& o
 // Square-root free: column j is published unscaled (V_rj, with V_jj = d_j the
 // pivot), later its unit form l_rj = V_rj / d_j.  Columns take a_rc -= V_rj l_cj;
 // the column that comes next takes a_rc - (V_rj V_cj) (1 / d_j) instead, from V
-// alone: its warp forms the product and the reciprocal side by side.  So the
+// alone: its warp forms the product and the reciprocal side by side (d_j's power of
+// two is taken out of V_cj before the product, by its exponent field: the product
+// itself would leave FP64's range for entries past 1e+-154).  So the
 // chain per column is one hand-off, the reciprocal and one FMA (~400 cycles, 500
 // with the warps that come late; a second hand-off, of the reciprocal, made it
 // 560-650).  The columns become
@@ -181,13 +209,12 @@ __device__ __forceinline__ void leaf_half(const double (*S)[LB], double (*V)[LB]
     if (c > b0) {  // the last step, from column j alone
       const double v = lds_wait(sv + j * ROW, w, over);
       __syncwarp();
-      const double p = v * __shfl_sync(0xffffffffu, v, c);
-      a = fma(-p, recip_pos(__shfl_sync(0xffffffffu, v, j)), a);
+      a = minus_term(a, v, __shfl_sync(0xffffffffu, v, c), __shfl_sync(0xffffffffu, v, j));
     }
     a = slot_clean(a);
     sts_slot(sv + c * ROW, a);
     const double d = __shfl_sync(0xffffffffu, a, c);
-    const double l = a * recip_pos(d);
+    const double l = over_pivot(a, d);
     sts_slot(sl + c * ROW + lane * 8, lane > c ? slot_clean(l) : 0.0);
     if (lane == 0 && !positive_bits(d)) atomicMin(&sh->fail, c);
     if (__any_sync(0xffffffffu, over)) {
@@ -666,7 +693,7 @@ struct ChainShape {  // of one CTA's shared memory
   }
 };
 
-__global__ void __launch_bounds__(CHAIN_THREADS)
+__global__ void __launch_bounds__(CHAIN_THREADS, 1)
     chain_factor_kernel(double* MF, int ns, int nd, long long nt, DevStatus* st, int wait_polls) {
   extern __shared__ double dyn[];
   __shared__ __align__(16) double Lc[LB][LB];
