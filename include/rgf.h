@@ -225,6 +225,13 @@ int rgf_device_cache_bytes(size_t* held);
  * succeed again.  after < 0 switches it off. */
 int rgf_debug_fail_alloc_after(long long after);
 
+/* One diagonal tile of the panel factorization by itself, for tests: the lower Cholesky
+ * factor of the w x w (1 <= w <= 160) matrix in host memory (column-major, leading dimension
+ * w), in place.  ctas is the number of thread blocks that share it: 16, or 8 as on a device
+ * that has too few places for clusters of 16 (RGF_ENOTSUP where 16 do not fit).
+ * RGF_ENOTSPD as rgf_factorize; no handle, and nothing is kept. */
+int rgf_debug_panel_tile(double* tile, int w, int ctas);
+
 /* Measured FP64 (DMMA m8n8k4) throughput of the current device in TFLOP/s:
  * the denominator of the FP64 roofline.  Runs about 100 ms of GPU work. */
 int rgf_measure_fp64_peak(double* tflops);

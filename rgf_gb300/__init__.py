@@ -144,6 +144,7 @@ _SIGS = {
     "rgf_batch_autotune": (C.c_int, [C.c_void_p, C.c_int, C.POINTER(C.c_size_t)]),
     "rgf_set_wait_limit": (C.c_int, [C.c_void_p, C.c_int]),
     "rgf_debug_fail_alloc_after": (C.c_int, [C.c_longlong]),
+    "rgf_debug_panel_tile": (C.c_int, [C.c_void_p, C.c_int, C.c_int]),
     "rgf_set_device_cache": (C.c_int, [C.c_size_t]),
     "rgf_device_cache_bytes": (C.c_int, [C.POINTER(C.c_size_t)]),
     "rgf_residual_norm_noalloc": (C.c_int, [C.c_size_t] + [C.c_void_p] * 7),
@@ -194,6 +195,14 @@ def debug_fail_alloc_after(after: int) -> None:
     """Failure injection for tests: the next ``after`` device allocations of
     the library succeed and the one after fails (RGF_ENOMEM); -1 turns it off."""
     _check(load_library().rgf_debug_fail_alloc_after(int(after)), "rgf_debug_fail_alloc_after")
+
+
+def debug_panel_tile(tile: np.ndarray, ctas: int) -> np.ndarray:
+    """The lower Cholesky factor of one tile of up to 160 columns by the kernel for
+    diagonal tiles, shared by ``ctas`` (8 or 16) thread blocks; for tests."""
+    t = np.array(tile, dtype=np.float64, order="F")
+    _check(load_library().rgf_debug_panel_tile(_ptr(t), t.shape[0], int(ctas)), "rgf_debug_panel_tile")
+    return np.tril(t)
 
 
 def set_device_cache(max_bytes: int) -> None:

@@ -472,13 +472,16 @@ __global__ void __launch_bounds__(TILE_THREADS, 5)
   bool stop = false;
   for (int k = 0; k + 1 < nl; ++k) {
     const int kc = k * LB, kn = kc + LB;          // this leaf's and the next one's first column
-    {  // solve: WG lanes a row, 32 / WG rows a warp
-      constexpr int SL = LB / WG;
-      const int q = lane & (WG - 1), i = warp * (32 / WG) + lane / WG;
-      const int r = row0 + NW * i;
-      const bool live = i < nown && r >= kn;
-      if (warp < LEAF_WARPS && !stop && __any_sync(0xffffffffu, live)) {
-        bool over = false;
+    {  // solve: WG lanes a row, ROUND rows at a time
+      constexpr int SL = LB / WG, ROUND = LEAF_WARPS * (32 / WG);
+      const int q = lane & (WG - 1);
+      bool over = false;
+#pragma unroll 1
+      for (int i0 = 0; i0 < WROWS && warp < LEAF_WARPS && !stop; i0 += ROUND) {
+        const int i = i0 + warp * (32 / WG) + lane / WG;
+        const int r = row0 + NW * i;
+        const bool live = i < nown && r >= kn;
+        if (!__any_sync(0xffffffffu, live)) continue;
         double u[SL];
 #pragma unroll
         for (int t = 0; t < SL; ++t) u[t] = live ? own(i)[kc + t * WG + q] : 0.0;
@@ -497,7 +500,10 @@ __global__ void __launch_bounds__(TILE_THREADS, 5)
             P[r + (long long)(kc + c) * lda] = x;
           }
         }
-        if (over) wait_gave_up(wait);
+        if (__any_sync(0xffffffffu, over)) {
+          if (lane == 0) wait_gave_up(wait);
+          break;
+        }
       }
     }
     stop = __syncthreads_or(*wait.abort_);
@@ -925,20 +931,20 @@ void launch_rows_g(double* X, int rows, const double* P, long long lda, int w, c
 }  // namespace
 
 namespace {
-// Whether clusters of 16 CTAs of panel_tile_kernel can be resident on this device.
-bool wide_clusters() {
+}  // namespace
+
+bool panel_wide_clusters() {
   static const bool ok = widest_cluster(panel_tile_kernel<15, PANEL_TILE>, 0, TILE_THREADS) == 16;
   return ok;
 }
-}  // namespace
 
 // One CTA for a single leaf; else a cluster of 16, or of 8 where the device
 // has too few places for 16.
 void launch_panel_tile(double* P, long long lda, int w, double* ws, int col0, DevStatus* st,
-                       cudaStream_t s, int wait_polls) {
+                       cudaStream_t s, int wait_polls, bool narrow) {
   if (w <= 0) return;
   const int polls = wait_polls > 0 ? wait_polls : LEAF_WAIT_POLLS;
-  const bool wide = w > LB && wide_clusters();
+  const bool wide = w > LB && !narrow && panel_wide_clusters();
   const dim3 n(w <= LB ? 1 : wide ? 16 : 8);
   auto* kern = w <= PANEL_TILE - PANEL_LEAF
                    ? (wide ? panel_tile_kernel<15, PANEL_TILE - PANEL_LEAF>

@@ -1965,6 +1965,27 @@ int rgf_debug_fail_alloc_after(long long after) {
   return RGF_OK;
 }
 
+int rgf_debug_panel_tile(double* tile, int w, int ctas) {
+  if (!tile || w < 1 || w > PANEL_TILE || (ctas != 8 && ctas != 16)) return RGF_EINVAL;
+  if (ctas == 16 && !panel_wide_clusters()) return RGF_ENOTSUP;
+  const size_t elems = (size_t)w * w;
+  double* d = nullptr;  // the tile, its workspace, the status
+  RGF_CK(device_malloc((void**)&d, sizeof(double) * (elems + PANEL_WS) + sizeof(DevStatus)));
+  DevStatus* st = reinterpret_cast<DevStatus*>(d + elems + PANEL_WS);
+  DevStatus host{INT_MAX, 0, 0, 0};
+  cudaError_t e = cudaMemcpy(d, tile, sizeof(double) * elems, cudaMemcpyHostToDevice);
+  if (!e) e = cudaMemcpy(st, &host, sizeof(host), cudaMemcpyHostToDevice);
+  if (!e) {
+    launch_panel_tile(d, w, w, d + elems, 0, st, nullptr, 0, ctas == 8);
+    e = cudaGetLastError();
+  }
+  if (!e) e = cudaMemcpy(&host, st, sizeof(host), cudaMemcpyDeviceToHost);
+  if (!e) e = cudaMemcpy(tile, d, sizeof(double) * elems, cudaMemcpyDeviceToHost);
+  device_free(d);
+  if (e) return cuda_status(e);
+  return host.timeout ? RGF_ETIMEOUT : host.not_spd_col != INT_MAX ? RGF_ENOTSPD : RGF_OK;
+}
+
 int rgf_set_wait_limit(rgf_handle* h, int polls) {
   if (!h || polls < 0) return RGF_EINVAL;
   if (polls == h->leaf_wait_polls) return RGF_OK;

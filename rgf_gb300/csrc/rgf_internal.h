@@ -199,8 +199,11 @@ constexpr int PANEL_LEAF = 32, PANEL_TILE = 160;
 constexpr int PANEL_LEAF_WS = PANEL_LEAF * PANEL_LEAF + PANEL_LEAF;
 constexpr int PANEL_WS = PANEL_TILE / PANEL_LEAF * PANEL_LEAF_WS;
 constexpr int LEAF_WAIT_POLLS = 1 << 26;
+// narrow: a cluster of 8 CTAs even where the device has room for 16.
 void launch_panel_tile(double* P, long long lda, int w, double* ws, int col0, DevStatus* st,
-                       cudaStream_t s, int wait_polls = 0);
+                       cudaStream_t s, int wait_polls = 0, bool narrow = false);
+// Whether clusters of 16 CTAs of that launch can be resident on this device.
+bool panel_wide_clusters();
 // X := X L^{-T} for `rows` rows of w columns at X (leading dimension lda), L the
 // tile factored by launch_panel_tile at P (same lda) with its ws.
 void launch_panel_rows(double* X, int rows, const double* P, long long lda, int w,
