@@ -232,6 +232,12 @@ int rgf_debug_fail_alloc_after(long long after);
  * RGF_ENOTSPD as rgf_factorize; no handle, and nothing is kept. */
 int rgf_debug_panel_tile(double* tile, int w, int ctas);
 
+/* One in-place product X := X U of the split engine at 7 slices by itself, for tests: X is
+ * m x k and U the k x k upper triangle (k >= 64), in host memory, column-major, packed.
+ * maps = 0 runs it as if the driver could not describe the operands to the tensor cores'
+ * copies, which leaves it to the FP64 kernel. */
+int rgf_debug_product_in_place(double* X, int m, const double* U, int k, int maps);
+
 /* Measured FP64 (DMMA m8n8k4) throughput of the current device in TFLOP/s:
  * the denominator of the FP64 roofline.  Runs about 100 ms of GPU work. */
 int rgf_measure_fp64_peak(double* tflops);

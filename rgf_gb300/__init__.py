@@ -145,6 +145,7 @@ _SIGS = {
     "rgf_set_wait_limit": (C.c_int, [C.c_void_p, C.c_int]),
     "rgf_debug_fail_alloc_after": (C.c_int, [C.c_longlong]),
     "rgf_debug_panel_tile": (C.c_int, [C.c_void_p, C.c_int, C.c_int]),
+    "rgf_debug_product_in_place": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_int]),
     "rgf_set_device_cache": (C.c_int, [C.c_size_t]),
     "rgf_device_cache_bytes": (C.c_int, [C.POINTER(C.c_size_t)]),
     "rgf_residual_norm_noalloc": (C.c_int, [C.c_size_t] + [C.c_void_p] * 7),
@@ -203,6 +204,15 @@ def debug_panel_tile(tile: np.ndarray, ctas: int) -> np.ndarray:
     t = np.array(tile, dtype=np.float64, order="F")
     _check(load_library().rgf_debug_panel_tile(_ptr(t), t.shape[0], int(ctas)), "rgf_debug_panel_tile")
     return np.tril(t)
+
+
+def debug_product_in_place(X: np.ndarray, U: np.ndarray, maps: bool = True) -> np.ndarray:
+    """X U (U upper triangular) by the split engine's in-place product, or, without
+    ``maps``, by what stands in for it; for tests."""
+    x, u = (np.array(v, dtype=np.float64, order="F") for v in (X, U))
+    _check(load_library().rgf_debug_product_in_place(_ptr(x), x.shape[0], _ptr(u), u.shape[0],
+                                                     int(maps)), "rgf_debug_product_in_place")
+    return x
 
 
 def set_device_cache(max_bytes: int) -> None:

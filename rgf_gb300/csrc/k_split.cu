@@ -1188,6 +1188,7 @@ bool SplitEngine::may_slice(const GemmDesc& g, double bias) const {
 // distinct maps, and the driver call is a noticeable part of a product's host
 // cost when stages are launched directly.
 bool SplitEngine::map_for(CUtensorMap* out, void* base, int S, int Rp, int Kp) {
+  if (no_maps_) return false;
   const auto key = std::make_tuple(base, S, Rp, Kp);
   auto it = maps_.find(key);
   if (it != maps_.end()) {
@@ -1357,7 +1358,18 @@ long long SplitEngine::gemm(const GemmDesc& g, cudaStream_t s, DevStatus* st,
       if (g.D2) f.D2 = g.D2 + (long long)b0 * g.sD;
       f.C = g.C ? g.C + (long long)b0 * g.sC : nullptr;
       f.D = g.D + (long long)b0 * g.sD;
+      // In place (D is A) the FP64 kernel's CTAs would overwrite operands that others
+      // still read: its result goes through the workspace, whose slices (2 S bytes an
+      // entry of A) are of no use now.
+      const bool in_place = g.D == g.A;
+      if (in_place) {
+        f.D = reinterpret_cast<double*>(ws_);
+        f.ldd = g.m;
+      }
       launched += launch_gemm_fp64(f, s);
+      if (in_place)
+        cudaMemcpy2DAsync(g.D, sizeof(double) * g.ldd, f.D, sizeof(double) * g.m,
+                          sizeof(double) * g.m, g.n, cudaMemcpyDeviceToDevice, s);
       continue;
     }
     p.exA = exA; p.exB = exB;

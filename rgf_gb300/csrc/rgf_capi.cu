@@ -588,8 +588,8 @@ void issue_trtri(rgf_handle* h, double* U, long long ldu, long long n, const dou
                  long long sT, bool leaves = true);
 
 // The block rows below the diagonal block, X L^T = B for a group of `cols` columns of it,
-// as one product with the group's inverse: X := X U, U = L_gg^{-T}, in place (the split
-// engine has cut X into digits before it writes).
+// as one product with the group's inverse: X := X U, U = L_gg^{-T}, in place (only for
+// SplitEngine::gemm, which allows it).
 GemmDesc far_product(rgf_handle* h, double* X, long long lda, int m, int cols) {
   GemmDesc g;
   g.m = m; g.n = g.k = cols;
@@ -1984,6 +1984,39 @@ int rgf_debug_panel_tile(double* tile, int w, int ctas) {
   device_free(d);
   if (e) return cuda_status(e);
   return host.timeout ? RGF_ETIMEOUT : host.not_spd_col != INT_MAX ? RGF_ENOTSPD : RGF_OK;
+}
+
+int rgf_debug_product_in_place(double* X, int m, const double* U, int k, int maps) {
+  if (!X || !U || m < 1 || k < 64) return RGF_EINVAL;
+  int status = RGF_OK;
+  SplitEngine* eng = SplitEngine::create(0, &status);
+  if (!status) status = eng->prepare(std::max(m, k), k, 1);
+  const size_t nx = (size_t)m * k, nu = (size_t)k * k;
+  double* d = nullptr;  // X, U, the status
+  if (!status)
+    status = cuda_status(device_malloc((void**)&d, sizeof(double) * (nx + nu) + sizeof(DevStatus)));
+  if (!status) {
+    if (!maps) eng->refuse_maps();
+    DevStatus* st = reinterpret_cast<DevStatus*>(d + nx + nu);
+    DevStatus host{INT_MAX, 0, 0, 0};
+    GemmDesc g;
+    g.m = m; g.n = g.k = k;
+    g.A = g.D = d; g.lda = g.ldd = m;
+    g.B = d + nx; g.ldb = k; g.triB = TRI_UPPER;
+    cudaError_t e = cudaMemcpy(d, X, sizeof(double) * nx, cudaMemcpyHostToDevice);
+    if (!e) e = cudaMemcpy(d + nx, U, sizeof(double) * nu, cudaMemcpyHostToDevice);
+    if (!e) e = cudaMemcpy(st, &host, sizeof(host), cudaMemcpyHostToDevice);
+    if (!e) {
+      eng->gemm(g, nullptr, st, nullptr, 7);
+      e = cudaGetLastError();
+    }
+    if (!e) e = cudaMemcpy(X, d, sizeof(double) * nx, cudaMemcpyDeviceToHost);
+    if (!e) e = cudaMemcpy(&host, st, sizeof(host), cudaMemcpyDeviceToHost);
+    status = e ? cuda_status(e) : host.timeout ? RGF_ETIMEOUT : RGF_OK;
+  }
+  device_free(d);
+  delete eng;
+  return status;
 }
 
 int rgf_set_wait_limit(rgf_handle* h, int polls) {

@@ -40,9 +40,13 @@ class SplitEngine {
   // Whether g's accuracy class allows the engine's slice count (see there).
   bool may_slice(const GemmDesc& g, double bias) const;
   int min_k() const { return min_k_; }
+  // Tensor maps as if the driver could not encode them (tests).
+  void refuse_maps() { no_maps_ = true; }
   // Issue D = alpha op(A) op(B) + beta C on stream s; returns kernels launched
   // and, in *tensor_flops (if given), the bf16 slice-product flops it runs.
   // slices > 0 overrides the engine's slice count (up to 8) for this call.
+  // D may be A (A := alpha A op(B), batch 1, four slices or more): A has been cut into
+  // digits before anything is written.
   long long gemm(const GemmDesc& g, cudaStream_t s, DevStatus* st,
                  double* tensor_flops = nullptr, int slices = 0);
 
@@ -60,6 +64,7 @@ class SplitEngine {
   size_t ws_bytes_ = 0;
   int num_sms_ = 148;
   int splitk_max_ = MAX_SPLITK;
+  bool no_maps_ = false;
   std::array<int, MAX_SPLITK + 1> max_clusters_{};  // per split-K degree
 };
 
