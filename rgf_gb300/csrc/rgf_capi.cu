@@ -410,6 +410,9 @@ void dfree(void* p) { device_free(p); }
 // Column groups of the diagonal block (see far_by_inverse): most columns, and fewest rows
 // below the diagonal block.
 constexpr int FAR_GROUP = 512, FAR_MIN_ROWS = 1450;
+// Products at 7 slices (55 bits below a row's largest entry) stand in for FP64 ones outside
+// the diagonal blocks only while the caller's own products have at most this many.
+constexpr int EMULATE_MAX_SLICES = 5;
 enum GemmClass { SMALL = 0, BULK = 1, DIAG = 2, BULK1 = 3 };
 
 cudaStream_t cur_stream(const rgf_handle* h) { return h->on_side ? h->side : h->stream; }
@@ -607,6 +610,11 @@ GemmDesc far_product(rgf_handle* h, double* X, long long lda, int m, int cols) {
 // block's own row solves wait for: factorization at ns = 2000, nt = 10 24.6 -> 22.1 ms,
 // ns = 1750, nt = 8 15.9 -> 14.8, ns = 1500 12.6 -> 12.3; at ns = 1250 12.1 -> 12.5, so the
 // line lies between.
+// Only up to 5 slices: there the group's sliced updates set the error (residual of the
+// rows, relative, against substitution at ns = 1500 and conditions 1 / 1e3 / 1e6 of the
+// blocks: 2.2e-15 / 2.8e-10 / 4.6e-10, before 2.3e-15 / 3.0e-10 / 4.8e-10; the selected
+// inverse's error the same).  At 6 to 8 slices it would be 1.4 to 4.5 times the
+// substitution's (3.0e-16 against 6.8e-17 at condition 1, 3.1e-14 against 1.9e-14 at 1e3).
 bool far_by_inverse(rgf_handle* h, int m, int cols, int dr) {
   if (!h->d_far || cols > FAR_GROUP || cols <= panel_last(h) || dr <= cols || m < FAR_MIN_ROWS ||
       h->opts.fp64_diag != 1)
@@ -1573,6 +1581,7 @@ int rgf_create(const size_t* ia, const size_t* ja, const double* a, size_t ns, s
       st = h->split_side->prepare((int)(ns + nd), (int)ns, 1);
       if (st) break;
       if ((long long)(ns + nd) >= FAR_MIN_ROWS && nt > 1 &&
+          h->split->slices() <= EMULATE_MAX_SLICES &&
           (st = dalloc(h, &h->d_far, 2 * FAR_GROUP * FAR_GROUP)))
         break;
     }
