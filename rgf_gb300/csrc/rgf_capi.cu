@@ -460,8 +460,11 @@ void trace_flush(rgf_handle* h) {
 // Digit slices for g on the split engine, 0 = FP64 only.  Where the engine's own slice
 // count is not allowed for a triangular or lower-only product but would be for a full one
 // of its size (SplitEngine::may_slice), blocks of that size already carry sliced
-// products, and it may take 7: 56-bit operands, FP64-accurate emulation (ns = 256,
-// nt = 30: selected inversion 3.6 -> 2.1 ms).  Below that line everything is FP64.
+// products, and it may take 7: 55 bits below each row's largest entry (ns = 256,
+// nt = 30: selected inversion 3.6 -> 2.1 ms).  Below that line everything is FP64.  Only up
+// to 5 slices, where the full products' error is 2^16 times that (relative error of all
+// of Sigma at ns = 256, 5 slices 2.8e-13, before 2.9e-13); at 7 it would be 8.0e-16 against
+// 2.2e-16, and a small entry whose row holds a large one would lose its bits.
 // fp64_diag: 0 = diagonal blocks at the bulk slice count, 1 = at 7 slices, 2 = native
 // FP64 DMMA.
 int class_slices(const rgf_handle* h, const SplitEngine* eng, const GemmDesc& g, int cls) {
@@ -474,7 +477,7 @@ int class_slices(const rgf_handle* h, const SplitEngine* eng, const GemmDesc& g,
   GemmDesc full = g;
   full.triA = full.triB = TRI_NONE;
   full.outLower = 0;
-  return fd == 1 && S <= EXACT && eng->may_slice(full, h->split_bias) ? EXACT : 0;
+  return fd == 1 && S <= EMULATE_MAX_SLICES && eng->may_slice(full, h->split_bias) ? EXACT : 0;
 }
 
 // Whether g runs on the split engine: by estimated time, the engine's estimate (its
