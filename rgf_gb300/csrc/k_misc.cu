@@ -336,34 +336,39 @@ __global__ void __launch_bounds__(NORM_THREADS)
   cluster_sync();  // a CTA's parts are read until every CTA is here
 }
 
-// partial[(block column i, 256-column chunk)][p] = sum_j C_i(a, j) C_i(b, j)
-// for the pairs p = (a >= b); one warp per pair, fixed-order warp reduction.
-// One launch at the end of the factorization instead of a product per block
-// column beside it (nt launches of ~10 us on the look-ahead stream).
-constexpr int ARROW_CHUNK = 256;
+// partial[q][p] = sum_j C_i(a, j) C_i(b, j) for the pairs p = (a >= b), over the cells (block
+// column i, 256 of its columns) q, q + gridDim.x, ...; one warp per pair, fixed-order warp
+// reduction.  One launch at the end of the factorization instead of a product per block
+// column beside it (nt launches of ~10 us on the look-ahead stream).  At most
+// ARROW_SYRK_CTAS partial sums of a pair, eight CTAs an SM: their memory (5 MB at 32 rows)
+// does not grow with nt past that.
+constexpr int ARROW_CHUNK = 256, ARROW_SYRK_CTAS = 8 * 152;
 __global__ void __launch_bounds__(256)
     arrow_syrk_kernel(BtaShape sh, const double* MF, double* partial) {
   pdl_wait();
   pdl_trigger();
-  const long long i = blockIdx.x, ns = sh.ns, nt = sh.nt, nd = sh.nd;
-  const double* Cb = MF + col_offset_d(ns, nt, nd, i) + dense_row_d(ns, nt, i);
-  const long long lda = lda_d(ns, nt, nd, i);
+  const long long ns = sh.ns, nt = sh.nt, nd = sh.nd;
+  const long long per = (ns + ARROW_CHUNK - 1) / ARROW_CHUNK, cells = nt * per;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long j0 = (long long)blockIdx.y * ARROW_CHUNK, j1 = min(ns, j0 + ARROW_CHUNK);
   const int pairs = (int)(nd * (nd + 1) / 2);
-  double* out = partial + (i * gridDim.y + blockIdx.y) * pairs;
+  double* out = partial + (long long)blockIdx.x * pairs;
   for (int p = warp; p < pairs; p += 8) {
     int a = 0, b = p;
     while (b > a) b -= ++a;  // p = a (a + 1) / 2 + b
     double s = 0.0;
-    for (long long j = j0 + lane; j < j1; j += 32) s = fma(Cb[a + j * lda], Cb[b + j * lda], s);
+    for (long long cell = blockIdx.x; cell < cells; cell += gridDim.x) {
+      const long long i = cell / per, j0 = (cell - i * per) * ARROW_CHUNK;
+      const long long j1 = min(ns, j0 + ARROW_CHUNK), lda = lda_d(ns, nt, nd, i);
+      const double* Cb = MF + col_offset_d(ns, nt, nd, i) + dense_row_d(ns, nt, i);
+      for (long long j = j0 + lane; j < j1; j += 32) s = fma(Cb[a + j * lda], Cb[b + j * lda], s);
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) out[p] = s;
   }
 }
 
-// corner(a, b) -= the chunks' sums, one warp per pair
+// corner(a, b) -= the partial sums, one warp per pair
 __global__ void arrow_syrk_reduce_kernel(BtaShape sh, const double* partial, long long chunks,
                                          double* MF) {
   pdl_wait();
@@ -531,17 +536,18 @@ cudaError_t launch_residual(long long n, const size_t* ia, const size_t* ja, con
   return cudaGetLastError();
 }
 
-static long long arrow_chunks(const BtaShape& sh) { return (sh.ns + ARROW_CHUNK - 1) / ARROW_CHUNK; }
+static long long arrow_partials(const BtaShape& sh) {
+  return std::min<long long>(sh.nt * ((sh.ns + ARROW_CHUNK - 1) / ARROW_CHUNK), ARROW_SYRK_CTAS);
+}
 long long arrow_syrk_elems(const BtaShape& sh) {
-  return sh.nt * arrow_chunks(sh) * (sh.nd * (sh.nd + 1) / 2);
+  return arrow_partials(sh) * (sh.nd * (sh.nd + 1) / 2);
 }
 void launch_arrow_syrk(const BtaShape& sh, double* MF, double* partial, cudaStream_t s) {
-  const long long chunks = arrow_chunks(sh);
+  const long long parts = arrow_partials(sh);
   const int pairs = (int)(sh.nd * (sh.nd + 1) / 2);
-  launch_k(arrow_syrk_kernel, dim3((unsigned)sh.nt, (unsigned)chunks), dim3(256), 0, s, sh,
-           (const double*)MF, partial);
+  launch_k(arrow_syrk_kernel, dim3((unsigned)parts), dim3(256), 0, s, sh, (const double*)MF, partial);
   launch_k(arrow_syrk_reduce_kernel, dim3((pairs + 7) / 8), dim3(256), 0, s, sh,
-           (const double*)partial, sh.nt * chunks, MF);
+           (const double*)partial, parts, MF);
 }
 
 void launch_arrow_gemv(const BtaShape& sh, const double* MF, const double* rhs, long long ldr,

@@ -330,8 +330,8 @@ constexpr int SPMV_MAX_RHS = 16;
 // x += d over len entries
 void launch_add(long long len, double* x, const double* d, cudaStream_t s);
 // corner -= sum_i C_i C_i^T (lower part) over all block columns, for
-// 0 < nd <= ARROW_SYRK_MAX_ND: partial sums per 256 columns of every block
-// column into partial (arrow_syrk_elems doubles), then added in a fixed order.
+// 0 < nd <= ARROW_SYRK_MAX_ND: partial sums over 256 columns of block columns
+// into partial (arrow_syrk_elems doubles), then added in a fixed order.
 constexpr int ARROW_SYRK_MAX_ND = 32;
 long long arrow_syrk_elems(const BtaShape& sh);
 void launch_arrow_syrk(const BtaShape& sh, double* MF, double* partial, cudaStream_t s);

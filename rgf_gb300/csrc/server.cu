@@ -48,6 +48,8 @@ size_t estimate_bytes(const rgf_opts& o, size_t ns, size_t nt, size_t nd, size_t
   size_t b = 16 * nnz + 8 * (n + 1) + 8 * mf;       // CSC + factor
   b += 8 * mf + 8 * (nt * ns * ns + nd * nd) + 8 * (nd * ns + 1);  // selected inverse
   const rgf::BtaShape sh{(long long)ns, (long long)nt, (long long)nd, (long long)n};
+  b += 8 * ((std::max(ns, nd) + 63) / 64 * rgf::PANEL_WS);  // diagonal tiles
+  if (nd > 0 && nd <= rgf::ARROW_SYRK_MAX_ND) b += 8 * (size_t)rgf::arrow_syrk_elems(sh);
   if (o.selinv_mode == RGF_SELINV_COMPAT) b += 8 * 2 * ns * ns;
   else b += 8 * (ns + nd) * (ns * (size_t)rgf::selinv_chunk(sh) + ns + nd);  // its workspaces
   if (o.precision == RGF_PREC_SPLIT) {  // slice workspaces of the main and side streams
