@@ -743,6 +743,19 @@ void issue_factor(rgf_handle* h) {
     h->kernels_issued++;
     trace(h, "factor chain");
   }
+  auto corner_update = [&](long long i) {  // corner -= C_i C_i^T (RGF.H:280, 308, 332)
+    const double* Ci = h->d_MF + mf_col_offset(sh, i) + mf_dense_row(sh, i);
+    GemmDesc c;
+    c.m = c.n = (int)nd; c.k = (int)ns;
+    c.A = Ci; c.lda = mf_lda(sh, i); c.B = Ci; c.ldb = mf_lda(sh, i); c.transB = 1;
+    c.C = c.D = corner; c.ldc = c.ldd = nd;
+    c.alpha = -1.0; c.beta = 1.0; c.outLower = 1;
+    gemm(h, c, SMALL);
+  };
+  // An arrowhead too wide for the one-pass corner update has a product per block column: on
+  // the look-ahead stream, where C_i was computed, beside the next block.
+  const bool corner_beside =
+      nd > 0 && !h->d_arrow && !chain && h->lookahead && h->side && ns > panel_last(h);
   for (long long i = chain ? nt : 0; i < nt; ++i) {
     double* P = h->d_MF + mf_col_offset(sh, i);
     const long long lda = mf_lda(sh, i);
@@ -763,29 +776,26 @@ void issue_factor(rgf_handle* h) {
       }
       g.alpha = -1.0; g.beta = 1.0; g.outLower = 1;
       gemm(h, g, BULK);
+      if (corner_beside) {
+        h->on_side = h->side_used = true;
+        corner_update(i - 1);
+        h->on_side = false;
+      }
     }
     panel_potrf(h, P, lda, (int)lda, (int)ns, (int)ns, 0, (int)(i * ns));
     if (h->side_used) join_side(h);
     trace(h, "block end");
   }
   if (nd > 0) {
-    // corner -= sum_i C_i C_i^T (RGF.H:280, 308, 332): nothing reads the corner
-    // before its own factorization, so all block columns go in one pass at the end
+    // nothing reads the corner before its own factorization, so up to
+    // ARROW_SYRK_MAX_ND rows all block columns go in one pass at the end
     if (h->d_arrow) {
       launch_arrow_syrk(sh, h->d_MF, h->d_arrow, s);
       h->kernels_issued += 2;
-      trace(h, "corner");
     } else {
-      for (long long i = 0; i < nt; ++i) {
-        const double* Ci = h->d_MF + mf_col_offset(sh, i) + mf_dense_row(sh, i);
-        GemmDesc c;
-        c.m = c.n = (int)nd; c.k = (int)ns;
-        c.A = Ci; c.lda = mf_lda(sh, i); c.B = Ci; c.ldb = mf_lda(sh, i); c.transB = 1;
-        c.C = c.D = corner; c.ldc = c.ldd = nd;
-        c.alpha = -1.0; c.beta = 1.0; c.outLower = 1;
-        gemm(h, c, SMALL);
-      }
+      for (long long i = corner_beside ? nt - 1 : 0; i < nt; ++i) corner_update(i);
     }
+    trace(h, "corner");
     panel_potrf(h, corner, nd, (int)nd, (int)nd, (int)nd, 0, (int)(nt * ns));  // RGF.H:335
   }
   launch_logdet(sh, h->d_MF, h->d_logpart, h->d_scalars, s);

@@ -78,3 +78,31 @@ def test_hermitian_in_used_memory(rgf, dirty):
         want = np.diag(np.linalg.inv(H)).real
         # the embedding's blocks are twice as large
         assert np.max(np.abs(s.RGFdiag().real - want)) <= 32 * (ns + nd) * EPS * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("precision,lookahead", [("fp64", 1), ("fp64", 0), ("split", 1)])
+@pytest.mark.parametrize("ns,nt,nd", [(161, 1, 33), (161, 2, 40), (200, 5, 64), (300, 4, 100), (520, 3, 33)])
+def test_corner_of_wide_arrowheads(rgf, precision, lookahead, ns, nt, nd, tmp_path, monkeypatch):
+    """More rows than the one-pass corner update takes: with look-ahead the products of all
+    block columns but the last run on its stream.  Tolerance: test_gpu_panel.py's; at 5
+    slices test_gpu_selinv_blocks.py's."""
+    ia, ja, a = gen.generate_bta(ns, nt, nd, seed=nd)
+    layout = O.Layout(ns, nt, nd)
+    MF = O.ingest(layout, ia, ja, a)
+    O.factorize(layout, MF)
+    want = np.triu(MF[-nd * nd:].reshape(nd, nd))
+    tol = 8 * (ns + nd) * EPS + (4 * 2.0 ** (3 - 8 * 5) * (ns + nd) if precision == "split" else 0)
+    path = tmp_path / "trace.csv"
+    for traced in (False, True):
+        if traced:
+            monkeypatch.setenv("RGF_GB300_TRACE", str(path))
+        with rgf.RGF(ia, ja, a, ns, nt, nd, precision=precision) as s:
+            s.set_tuning(lookahead=lookahead, fp64_tile=32)
+            for _ in range(1 if traced else 3):  # launched directly, then captured and replayed
+                s.factorize()
+                got = np.triu(s.export_factor()[-nd * nd:].reshape(nd, nd))
+                assert np.max(np.abs(got - want)) <= tol * np.max(np.abs(want))
+    rows = [ln.split(",") for ln in path.read_text().splitlines()]
+    shape = f"fp64 cls0 m{nd} n{nd} k{ns} b1"
+    streams = [r[2] for r in rows if r[3] == shape]
+    assert streams == ["1" if lookahead else "0"] * (nt - 1) + ["0"]
