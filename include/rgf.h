@@ -309,7 +309,8 @@ int rgf_batch_kernels(rgf_batch* b, long long* kernels);
  *               factors (32-column FP64 leaves inside): 16 = 64 columns,
  *               32 or 64 = 128 columns, the last up to 160;
  *   lookahead   1 = the rows below each diagonal block are solved and updated
- *               on a second, lower-priority stream; 0 = one stream;
+ *               on a second, lower-priority stream (in the selected inversion: the
+ *               last block's inverse and the arrowhead's products); 0 = one stream;
  *   split_bias  split precision: a product runs on the tensor cores when its
  *               estimated split time times split_bias is below its estimated
  *               FP64 time (1.0 = the fitted cost model; > 1 moves products to

@@ -884,7 +884,7 @@ void issue_inverses(rgf_handle* h) {
   // stream, beside the batch of the others: their recursions are chains of small
   // launches (selected inversion at ns = 2000, nt = 10 14.3 -> 11.9 ms, half of it
   // from the leaves' row solves).
-  const bool beside = nt > 1 && h->side;
+  const bool beside = nt > 1 && h->lookahead && h->side;
   if (beside) {
     fork_side(h);
     h->on_side = true;
@@ -1009,7 +1009,7 @@ void issue_selinv(rgf_handle* h) {
           gemm(h, mk(m2, ins, m2, h->d_S, m2, 0, K, m2, 0, nullptr, 0, Q + ns, lda, -1.0, 0.0),
                BULK);
         } else {
-          if (nd > 0) join_side(h);  // -[Sigma_{d,i+1}^T; Sigma_dd] K_C is in place
+          if (h->side_used) join_side(h);  // -[Sigma_{d,i+1}^T; Sigma_dd] K_C is in place
           gemm(h, g_split(i, K, nd > 0 ? 1.0 : 0.0), BULK);
         }
       }
@@ -1029,13 +1029,15 @@ void issue_selinv(rgf_handle* h) {
       if (i > 0 && nd > 0 && !dense) {
         // the arrowhead's part of the next block's G, in FP64 (in the same sliced
         // product its larger terms would set the scale of the others); it needs
-        // nothing of Sigma_ii and runs beside it
+        // nothing of Sigma_ii and with look-ahead runs beside it
         const double* Kc = h->d_K + (i - 1 - k_lo) * ns * m2 + ns;
         double* Gn = h->d_MS + mf_col_offset(sh, i - 1) + ns;
         const double* Sd = Q + mf_dense_row(sh, i);
         const long long ldg = 2 * ns + nd;
-        fork_side(h);
-        h->on_side = true;
+        if (h->lookahead && h->side) {
+          fork_side(h);
+          h->on_side = true;
+        }
         gemm(h, mk(ins, ins, ind, Sd, lda, 1, Kc, m2, 0, nullptr, 0, Gn, ldg, -1.0, 0.0), SMALL);
         gemm(h, mk(ind, ins, ind, Sdd, nd, 0, Kc, m2, 0, nullptr, 0, Gn + ns, ldg, -1.0, 0.0), SMALL);
         h->on_side = false;
