@@ -103,3 +103,31 @@ def test_pivot_reciprocals(rgf):
     want22 = np.sqrt(lc - lv * (lv / ld))
     for got, want, k in ((P[:, 0, 0], want11, 2), (P[:, 0, 1], want21, 3), (P[:, 1, 1], want22, 4)):
         assert np.max(np.abs(got.astype(np.longdouble) / want - 1)) <= k * EPS
+
+
+@pytest.mark.parametrize("ns,nt,nd", SHAPES)
+def test_graded(rgf, ns, nt, nd):
+    """Rows and columns scaled by powers of two between 2^-220 and 2^220 each, so that magnitudes
+    from 2^-440 to 2^440 stand side by side: the factor's rows scale alike, exactly."""
+    ia, ja, a = gen.generate_bta(ns, nt, nd, seed=ns + nd)
+    n = ns * nt + nd
+    layout = O.Layout(ns, nt, nd)
+    MF = O.ingest(layout, ia, ja, a)
+    O.factorize(layout, MF)
+    want = _entries(ns, nt, nd, MF)
+    diag = O.selinv_exact(layout, MF)
+    e = 2 * np.random.default_rng(ns).integers(-110, 111, n)
+    row, col = ja.astype(np.int64), np.repeat(np.arange(n), np.diff(ia.astype(np.int64)))
+    rows = []  # the row of each entry of _entries
+    for i in range(nt):
+        r = np.arange(i * ns, min(i + 2, nt) * ns)
+        r = np.concatenate([r, np.arange(nt * ns, n)])
+        rows += [r[c:] for c in range(ns)]
+    rows += [np.arange(nt * ns + c, n) for c in range(nd)]
+    tol = 16 * (ns + nd) * EPS
+    with rgf.RGF(ia, ja, np.ldexp(a, e[row] + e[col]), ns, nt, nd) as s:
+        s.factorize()
+        got = np.ldexp(_entries(ns, nt, nd, s.export_factor()), -e[np.concatenate(rows)])
+        assert np.max(np.abs(got - want)) <= tol * np.max(np.abs(want))
+        got = np.ldexp(s.RGFdiag(), 2 * e)
+        assert np.max(np.abs(got - diag)) <= tol * np.max(np.abs(diag))
