@@ -13,16 +13,6 @@ namespace {
 
 constexpr int CHAIN_THREADS = 256;
 
-__device__ __forceinline__ void cp_async8(void* dst, const double* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;"
-               :: "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int PENDING>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
-}
-
 // How many neighbouring threads (a power of two up to MAX) share each of n elements of
 // `terms` terms: the fewest FP64 instructions on an SM sub-partition.
 template <int MAX>

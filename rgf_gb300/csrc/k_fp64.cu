@@ -555,7 +555,7 @@ struct ClusterRoom {
 const ClusterRoom& cluster_room() {
   static const ClusterRoom room = [] {
     ClusterRoom r{};
-    r.clusters[1] = 152;
+    r.clusters[1] = GB300_SMS;
     auto* k = gemm_fp64_kernel<32, 8>;
     constexpr int FILL = 160 << 10;
     const bool ok =
@@ -656,7 +656,7 @@ int launch_gemm_fp64(const GemmDesc& g0, cudaStream_t s) {
   // nt = 10 81 against 115 ms, ns = 333, nt = 17 12.2 against 16.8).  Against the
   // previous rule (up to 16 K slices of 64-wide tiles through a workspace and a
   // second launch) the selected inversion at ns = 1000, nt = 10 went from 58.8 to
-  // 49.2 ms, at ns = 333, nt = 17 from 9.0 to 6.3.
+  // 49.2 ms, at ns = 333, nt = 17 from 9.0 to 6.3.  64 is there for the fp64_tile knob.
   const int tm = g.tile == 64 ? 64 : 32, tk = tm == 64 ? 16 : 8;
   const double tiles = (double)tiles_written(g, tm) * g.batch;
   const ClusterRoom& room = cluster_room();
@@ -669,8 +669,8 @@ int launch_gemm_fp64(const GemmDesc& g0, cudaStream_t s) {
   const int ks_max = g.beside && tiles > 76 ? 2 : 8;
   for (int ks = 1; ks <= ks_max; ++ks) {
     // a K step of the kernel a slice at least; nothing to gain past a few waves
-    if (ks > 1 && (g.k < tk * ks || tiles > 8 * 152 || (long long)ks * g.batch > 65535)) break;
-    double shares = std::ceil(tiles * ks / 152.0);
+    if (ks > 1 && (g.k < tk * ks || tiles > 8 * GB300_SMS || (long long)ks * g.batch > 65535)) break;
+    double shares = std::ceil(tiles * ks / GB300_SMS);
     if (tiles > room.clusters[ks]) shares = std::max(shares, 2.0);
     const int part = ((g.k + ks - 1) / ks + tk - 1) / tk * tk;  // K terms of a slice
     const double us = shares * tm * tm * part / 3200.0 + (ks > 1 ? 2.0 : 0.0);
@@ -690,7 +690,7 @@ void launch_trsm_rows(double* X, long long xrs, long long xcs, int rows, const d
                       long long ldl, int nbk, int mode, int batch, long long sX, long long sL,
                       cudaStream_t s) {
   if (rows <= 0 || nbk <= 0 || batch <= 0) return;
-  const bool wide = (long long)rows * batch <= 4 * 152 * 4;  // up to four CTAs of four rows an SM
+  const bool wide = (long long)rows * batch <= 4 * GB300_SMS * 4;  // up to four CTAs of four rows an SM
   const dim3 grid((rows + (wide ? 3 : 15)) / (wide ? 4 : 16), batch);
   auto* kern = mode == 0 ? (wide ? trsm_rows_kernel<0, 32> : trsm_rows_kernel<0, 8>)
                          : (wide ? trsm_rows_kernel<1, 32> : trsm_rows_kernel<1, 8>);
@@ -701,7 +701,7 @@ void launch_leaf_inverses(double* U, long long ldu, int n, const double* L, long
                           int batch, long long sU, long long sL, cudaStream_t s) {
   if (n <= 0 || batch <= 0) return;
   const int leaves = (n + 63) / 64, rows = std::min(n, 64);
-  const bool wide = (long long)rows * leaves * batch <= 4 * 152 * 4;
+  const bool wide = (long long)rows * leaves * batch <= 4 * GB300_SMS * 4;
   const dim3 grid((rows + (wide ? 3 : 15)) / (wide ? 4 : 16), batch, leaves);
   launch_k(wide ? trsm_rows_kernel<0, 32, true> : trsm_rows_kernel<0, 8, true>, grid, dim3(128), 0, s,
            U, 1ll, ldu, rows, L, ldl, n, sU, sL);

@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
 // column beside it (nt launches of ~10 us on the look-ahead stream).  At most
 // ARROW_SYRK_CTAS partial sums of a pair, eight CTAs an SM: their memory (5 MB at 32 rows)
 // does not grow with nt past that.
-constexpr int ARROW_CHUNK = 256, ARROW_SYRK_CTAS = 8 * 152;
+constexpr int ARROW_CHUNK = 256, ARROW_SYRK_CTAS = 8 * GB300_SMS;
 __global__ void __launch_bounds__(256)
     arrow_syrk_kernel(BtaShape sh, const double* MF, double* partial) {
   pdl_wait();

@@ -578,16 +578,6 @@ __global__ void __launch_bounds__(TILE_THREADS, 5)
 // scaled result updates the columns after it with the tile's rows of block k.
 // The leaf and the rows of the block are copied to shared memory asynchronously,
 // the latter (and the next leaf) behind the solve.
-__device__ __forceinline__ void cp_async8(void* dst, const double* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;"
-               :: "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int PENDING>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
-}
-
 template <int G, int NB, int NT>  // NB: 32-column blocks of the tile (the last may be narrower)
 __global__ void __launch_bounds__(NT)
     panel_rows_kernel(double* X, int rows, const double* P, long long lda, int w,
@@ -955,7 +945,7 @@ void launch_panel_tile(double* P, long long lda, int w, double* ws, int col0, De
 }
 
 // G lanes a row and four or eight warps: 4 / 8 / 16 rows a CTA, the fewest that
-// still let the 152 SMs take all rows at once (a CTA's time grows with its rows;
+// still let the SMs take all rows at once (a CTA's time grows with its rows;
 // two CTAs on an SM share its FP64 units).  16 rows go as two warps a
 // sub-partition of two rows each: 6% more instructions than one warp of four, but
 // one warp's shuffles and shared-memory reads run behind the other's FMAs
@@ -963,8 +953,8 @@ void launch_panel_tile(double* P, long long lda, int w, double* ws, int col0, De
 void launch_panel_rows(double* X, int rows, const double* P, long long lda, int w,
                        const double* ws, cudaStream_t s) {
   if (rows <= 0 || w <= 0) return;
-  if (rows <= 4 * 152) launch_rows_g<32, 128>(X, rows, P, lda, w, ws, s);
-  else if (rows <= 8 * 152) launch_rows_g<16, 128>(X, rows, P, lda, w, ws, s);
+  if (rows <= 4 * GB300_SMS) launch_rows_g<32, 128>(X, rows, P, lda, w, ws, s);
+  else if (rows <= 8 * GB300_SMS) launch_rows_g<16, 128>(X, rows, P, lda, w, ws, s);
   else launch_rows_g<16, 256>(X, rows, P, lda, w, ws, s);
 }
 

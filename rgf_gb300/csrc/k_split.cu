@@ -20,9 +20,10 @@
 // MMAs: 8-bit digits need 15 pairs for 39-bit operands where 7-bit digits
 // need 21 for 42 bits.
 // The GEMM kernel is warp specialized: one warp issues TMA tile loads
-// (cp.async.bulk.tensor, 128B swizzle, 128 K terms per stage as two swizzle
-// atoms) into a 3-stage shared-memory ring, one
-// elected thread issues tcgen05.mma (M=128, N=128, K=16, bf16 -> f32) into
+// (cp.async.bulk.tensor, 128B swizzle, 64 K terms per stage: one swizzle atom of A
+// and up to two of B) into a 4-stage shared-memory ring, one
+// elected thread issues tcgen05.mma (M=128, N=256 over two of B's digits, or
+// N=128, K=16, bf16 -> f32) into
 // two TMEM accumulators, and eight warps drain the accumulators while the next
 // product accumulates.  Every wait on an mbarrier is bounded; a wait that
 // gives up records a timeout in the device status word and the CTA exits.
@@ -1136,9 +1137,7 @@ int SplitEngine::reserve(int max_rows, int max_k, int batch_hint) {
 double SplitEngine::estimate_seconds(const GemmDesc& g, int slices) const {
   const int S = slices > 0 ? std::min(slices, MAX_SLICES) : slices_;
   const int Kp = round_up(g.k, BKE);
-  const int tx = round_up(g.m, BM) / BM, ty = round_up(g.n, BN) / BN;
-  long long tiles = tiles_written(g, BM);
-  tiles *= g.batch;
+  const long long tiles = tiles_written(g, BM) * g.batch;
   const SlotPlan& plan = slot_plan(S);
   int jobs = 0;
   for (const SlotGroup& gr : plan.groups) {

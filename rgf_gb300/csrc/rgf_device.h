@@ -43,15 +43,16 @@ __device__ __forceinline__ long long ld_cluster_i64(unsigned addr) {
 __device__ __forceinline__ void st_cluster(unsigned addr, double v) {
   asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
 }
-__device__ __forceinline__ void st_release_cta(int* p, int v) {
-  asm volatile("st.release.cta.shared::cta.b32 [%0], %1;"
-               :: "r"((unsigned)__cvta_generic_to_shared(p)), "r"(v) : "memory");
+
+// ---- asynchronous copies of doubles from global to this CTA's shared memory ------
+__device__ __forceinline__ void cp_async8(void* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;"
+               :: "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
-__device__ __forceinline__ int ld_acquire_cta(const int* p) {
-  int v;
-  asm volatile("ld.acquire.cta.shared::cta.b32 %0, [%1];"
-               : "=r"(v) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
-  return v;
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
 }
 
 // ---- FP64 arithmetic off the FP64 units ----------------------------------------

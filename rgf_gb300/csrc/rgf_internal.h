@@ -24,6 +24,8 @@ struct DevResults {
   double scalars[8];  // [0] logdet, [1] ||r||, [2] ||b||
 };
 
+constexpr int GB300_SMS = 152;  // the splits of FP64 work over the chip are fitted to it
+
 // ---- programmatic dependent launch -------------------------------------------
 // Kernels are launched with programmatic stream serialization (launch_k): the
 // next kernel in a stream may be scheduled once every CTA of the running one
