@@ -287,7 +287,7 @@ def run_batch(args):
     tune = None
     if args.autotune:
         # the same batch again after the autotuner picked each (ns, nd)
-        # class's knobs (leaf width, look-ahead, routing bias)
+        # class's knobs (tile width, look-ahead, routing bias)
         ms_default = ms
         t0 = time.perf_counter()
         classes = b.autotune()

@@ -54,8 +54,11 @@ typedef struct rgf_opts {
   int use_graphs;   /* 1 = replay each stage as a captured CUDA graph         */
   int fp64_diag;    /* split precision, Cholesky and inverse of the diagonal
                        blocks: 1 (default) FP64 accuracy, their inner products
-                       emulated with 7 slices (56-bit operands); 2 native FP64
-                       units; 0 the bulk slice count                          */
+                       emulated with 7 slices (55-bit operands); 2 native FP64
+                       units; 0 the bulk slice count.  With 1 and slices <= 5,
+                       7-slice products also replace FP64 ones below large
+                       diagonal blocks and in a band of sizes under the one
+                       where bulk products are sliced                         */
   int async_upload; /* 1: rgf_create queues the CSC upload and returns; the
                        copies overlap the first factorization, which waits for
                        each block column just before using it.  Applies to
@@ -343,8 +346,8 @@ int rgf_get_tuning(rgf_handle* h, rgf_tuning* t);
 int rgf_set_tuning(rgf_handle* h, const rgf_tuning* t);
 /* Autotuner: times factorize + selected inversion (graph-replayed, best of two
  * after a direct run and a capture) for candidate knobs by coordinate
- * descent (leaf width, then look-ahead, then, in split precision, the routing
- * bias), keeps a candidate only when it is at least 2% faster, and sets the
+ * descent (tile width, then look-ahead, then, in split precision, the routing
+ * bias and split-K degree, then the FP64 tile), keeps a candidate only when it is at least 2% faster, and sets the
  * best on h.  Choices are cached per process by (device, ns, nd, options);
  * a cached class is not measured again unless flags has RGF_TUNE_FORCE.
  * Allocates the selected-inversion buffers; leaves h unfactored.  The matrix
