@@ -412,12 +412,20 @@ void launch_selinv_chain(const BtaShape& sh, int nc, const double* K, const doub
 // us): ns = 128 347 / 490 with one right-hand side, 781 / 960 with eight; ns = 160 458 / 456
 // with one, 606 / 565 with two; ns = 256 875 / 812.  One CTA beats eight while a
 // product has up to ~600 FMAs (ns = 3: 153 against 195), sixteen beat eight from ~48 rows.
+// Past 16 right-hand sides the separate products spread over the whole GPU, and the chain
+// is the better way only up to ~8 K FMAs and 256 results of a CTA a product (chain /
+// products in ms: ns = 3, nt = 60 0.85 / 0.99 with 256, 1.43 / 1.1 with 512; ns = 16, nt = 60
+// 0.86 / 1.06 with 128, 1.25 / 1.10 with 192; ns = 64, nt = 40 0.68 / 0.74 with 24, 1.24 / 0.90
+// with 64; ns = 144, nt = 30 1.16 / 0.82 with 17, 3.3 / 1.3 with 64).
 int solve_chain_ctas(const BtaShape& sh, int nrhs) {
   const long long m2 = sh.ns + sh.nd;
   if (m2 > SOLVE_CHAIN_MAX || sh.ns > (nrhs == 1 ? 176 : 144)) return 0;
   static const int widest = widest_cluster(solve_chain_kernel, SOLVE_CHAIN_SMEM, CHAIN_THREADS);
   if (!widest || (widest < 16 && sh.ns > 100)) return 0;
   const int nc = m2 * m2 * nrhs <= 600 ? 1 : m2 <= 48 ? 8 : widest;
+  if (nrhs > 16 &&
+      (sh.ns * sh.ns * nrhs > 8192LL * nc || solve_rows((int)sh.ns, nc) * (long long)nrhs > 256))
+    return 0;
   if (solve_chain_elems((int)sh.ns, (int)sh.nd, nrhs, nc) * sizeof(double) > SOLVE_CHAIN_SMEM) return 0;
   return nc;
 }

@@ -426,6 +426,7 @@ __global__ void __launch_bounds__(128) gemm_thin_m_kernel(GemmDesc g, int kchunk
 // A: the block substitution, whose matrices are the factor's) the first tile of A is
 // loaded while that kernel still runs (eight right-hand sides, ns = 256, nt = 60:
 // 2.01 -> 1.65 ms; one 0.90 -> 0.81).
+// More columns than N go as groups of N (blockIdx.z; launch_gemm_thin_groups).
 constexpr int THIN_KT = 32;  // K terms of one warp's tile
 template <int N>
 __global__ void __launch_bounds__(128) gemm_thin_n_kernel(GemmDesc g) {
@@ -434,6 +435,11 @@ __global__ void __launch_bounds__(128) gemm_thin_n_kernel(GemmDesc g) {
   __shared__ double At[4][THIN_KT][32];
   __shared__ double Bs[4][THIN_KT][N];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int first = blockIdx.z * N;  // column of this group of N
+  g.n -= first;
+  g.B += first * g.ldb;
+  g.C += first * g.ldc;
+  g.D += first * g.ldd;
   // the row tiles with the longest K range go first
   const int bx = g.triA == TRI_LOWER ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
   const int r0 = bx * 32, r = r0 + lane;
@@ -591,9 +597,26 @@ dim3 thin_split(const GemmDesc& g, int least, int* kchunk) {
 // (a thin-n CTA is worth 64 FMA instructions: 16 a warp, ~0.6 us)
 template <int N>
 void launch_thin_n(const GemmDesc& g, cudaStream_t s) {
+  const int rows = (g.m + 31) / 32, groups = (g.n + N - 1) / N;
   int kc = 1;
   while (kc < 8 && g.k * N > kc * 64 && g.k > kc * 8) kc *= 2;
-  launch_k_cluster(gemm_thin_n_kernel<N>, dim3((g.m + 31) / 32, kc), dim3(128), dim3(1, kc), 0, s, g);
+  while (groups > 1 && kc > 1 && rows * groups * kc > 4 * GB300_SMS) kc /= 2;
+  launch_k_cluster(gemm_thin_n_kernel<N>, dim3(rows, kc, groups), dim3(128), dim3(1, kc), 0, s, g);
+}
+// Block substitution with THIN_N_MAX < n <= THIN_GROUPS_MAX right-hand sides: groups of 8 columns
+// (12 from 193 on at up to 160 rows: 100, 40, 256 2.9 ms against 3.5 by eights; 200, 30, 256
+// 4.8 against 3.9), K over a cluster only while that leaves four CTAs an SM.  Against 32-wide
+// tiles, whose few K slices of 32 x 32 outputs fill little of the GPU, and 64-wide tiles
+// with up to 16 slices through a workspace before them, whole solves (ns, nt and
+// right-hand sides; this / 32-wide / before, in ms): 160, 30, 17 0.83 / 1.53 / 1.20;
+// 256, 20, 64 1.6 / 2.2 / 1.7; 144, 30, 64 1.3 / 1.7 / 1.4; 512, 10, 32 1.1 / 1.6 / 1.3;
+// 1000, 6, 128 5.5 / 5.8 / 6.8; 64, 40, 256 1.7 / 1.9 / 1.9.  Groups of 16 leave fewer CTAs
+// (256, 20, 17: 1.1 against 0.81), and past 512 the tiles read A less often
+// (nor do they pay below 8 rows).
+constexpr int THIN_N_MAX = 16, THIN_GROUPS_MAX = 512;
+void launch_gemm_thin_groups(const GemmDesc& g, cudaStream_t s) {
+  if (g.n <= 192 || g.m > 160) launch_thin_n<8>(g, s);
+  else launch_thin_n<12>(g, s);
 }
 template <int M>
 void launch_thin_m(const GemmDesc& g, cudaStream_t s) {
@@ -642,9 +665,10 @@ int launch_gemm_fp64(const GemmDesc& g0, cudaStream_t s) {
     launch_gemm_thin_m(g, s);
     return 1;
   }
-  if (g.n <= 16 && !g.transB && g.triB == TRI_NONE && g.batch == 1 && !g.outLower &&
-      !g.A2 && !g.D2) {
-    launch_gemm_thin_n(g, s);
+  if (g.n <= (g.early && g.m >= 8 ? THIN_GROUPS_MAX : THIN_N_MAX) && !g.transB && g.triB == TRI_NONE &&
+      g.batch == 1 && !g.outLower && !g.A2 && !g.D2) {
+    if (g.n <= THIN_N_MAX) launch_gemm_thin_n(g, s);
+    else launch_gemm_thin_groups(g, s);
     return 1;
   }
   // Output tile and split K (a cluster of up to 8 CTAs): the kernel is bound by

@@ -148,7 +148,8 @@ struct GemmDesc {
   long long sA = 0, sB = 0, sC = 0, sD = 0;
   int ksplit = 1;       // FP64 kernel: set by the launcher
   bool beside = false;  // FP64 kernel: other work shares the GPU
-  bool early = false;   // FP64 kernel: the stream's previous kernel does not write A
+  bool early = false;   // FP64 kernel: the stream's previous kernel does not write A (a
+                        // product of the block substitution)
   int tile = 0;  // FP64 kernel: output tile 32 or 64; 0 = chosen by the launcher
 };
 
