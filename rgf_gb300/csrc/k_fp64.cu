@@ -435,11 +435,13 @@ __global__ void __launch_bounds__(128) gemm_thin_n_kernel(GemmDesc g) {
   __shared__ double At[4][THIN_KT][32];
   __shared__ double Bs[4][THIN_KT][N];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int first = blockIdx.z * N;  // column of this group of N
-  g.n -= first;
-  g.B += first * g.ldb;
-  g.C += first * g.ldc;
-  g.D += first * g.ldd;
+  if (N >= 8) {  // (smaller ones have no groups)
+    const int first = blockIdx.z * N;  // column of this group of N
+    g.n -= first;
+    g.B += first * g.ldb;
+    g.C += first * g.ldc;
+    g.D += first * g.ldd;
+  }
   // the row tiles with the longest K range go first
   const int bx = g.triA == TRI_LOWER ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
   const int r0 = bx * 32, r = r0 + lane;
